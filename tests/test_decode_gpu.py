@@ -99,3 +99,25 @@ def test_portions_of_given_tokens(kw):
         assert np.abs(np.concatenate(got) - want).max() <= 5e-3 * max(np.abs(want).max(), 1.0), sizes
     assert np.abs(dec.step(int(t[0])).cpu().numpy() - om.forward_logits(
         params, ocfg, np.append(t, t[0])[None, :], acc=np.float64)[0, -1]).max() <= 5e-3 * max(np.abs(want).max(), 1.0)
+
+
+@pytest.mark.parametrize("case, context", [(0, 190), (0, 200), (0, 700), (1, 94), (1, 101), (1, 510)])
+def test_token_pass_over_key_ranges(case, context):
+    """The token kernel on both sides of the switch from one key range per head to several (192 positions at head
+    size 64, 96 at 128) and with many ranges: logits against the oracle over the same prefix, for a burst of
+    greedy tokens and for single chosen ones. fp32 sums over at most 700 keys behind a TF32 prompt (2^-11 per
+    operand, two layers): 5e-3 of the largest logit, as the tests above."""
+    from emberlm_b200 import engine as E
+    ocfg, ecfg, params = build(CASES[case], 51)
+    prompt = np.random.default_rng(context).integers(0, ocfg.vocab_size, size=context)
+    dec = E.Decoder(ecfg, max_seq_len=context + 8)
+    dec.load_parameters(params)
+    got = dec.generate(prompt, 6).cpu().numpy()
+    prefix = np.concatenate([prompt, got[:-1]])
+    ref = om.forward_logits(params, ocfg, prefix[None, :], acc=np.float64)[0, -1]
+    assert np.abs(dec.last_logits().cpu().numpy() - ref).max() <= 5e-3 * max(np.abs(ref).max(), 1.0)
+    dec.reset()
+    dec.extend(prompt)
+    for token in got[:-1]:
+        z = dec.step(int(token)).cpu().numpy()
+    assert np.abs(z - ref).max() <= 5e-3 * max(np.abs(ref).max(), 1.0)
