@@ -18,7 +18,7 @@
 // Why a buffer can be overwritten without an acknowledgement: every CTA owns at least one row of each
 // product (token_grid), so a complete vector implies that every CTA has finished the phase that read the
 // vector before it; between two uses of one buffer there are at least two such complete vectors.
-// Every wait is bounded: after kWaitBudgetNs the status word is set and an abort flag makes all CTAs leave.
+// Every wait is bounded (Patience).
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -51,35 +51,36 @@ __device__ __forceinline__ void get2(const Word* w, Word& x, Word& y) {   // w 1
 __device__ __forceinline__ bool is_from(Word x, unsigned epoch) { return static_cast<unsigned>(x >> 32) == epoch; }
 __device__ __forceinline__ float value_of(Word x) { return __uint_as_float(static_cast<unsigned>(x)); }
 
+// The rare part of a wait, out of line: a token runs through far more code than the instruction caches hold close, and
+// every wait has one. True when the thread gives up: another one has, or kMostPolls (some seconds) have been made
+// since the last block barrier, which sets the status word and the abort flag that makes all CTAs leave.
+constexpr unsigned kMostPolls = 1u << 23;
+__device__ __noinline__ bool wait_is_over(unsigned int* sync, int* status, unsigned polls) {
+  if (ld_acquire_u32(sync + kAbort) != 0u) return true;
+  if (polls < kMostPolls) return false;
+  if (atomicCAS(status, 0, CTDK_ETIMEOUT) == 0) {
+    status[1] = 90;
+    status[2] = static_cast<int>(blockIdx.x);
+    status[3] = static_cast<int>(threadIdx.x);
+  }
+  atomicExch(sync + kAbort, 1u);
+  return true;
+}
 // The bound of a thread's waits: more() says whether to poll on. Once it has said no it keeps to that; the
 // block agrees on leaving at the next barrier (left()).
 struct Patience {
-  const unsigned int* sync;
+  unsigned int* sync;
   int* status;
   bool gone = false;
-  unsigned spins = 0;
-  uint64_t t0 = 0;
+  unsigned polls = 0;
   __device__ __forceinline__ Patience(const TokenKernelArgs& a) : sync(a.sync), status(a.status) {}
   __device__ __forceinline__ bool more() {
-    if ((++spins & 63u) != 0u) return !gone;
-    const uint64_t now = globaltimer_ns();
-    if (spins == 64u) t0 = now;
-    if (ld_acquire_u32(sync + kAbort) != 0u) {
-      gone = true;
-    } else if (now - t0 > kWaitBudgetNs) {
-      if (atomicCAS(status, 0, CTDK_ETIMEOUT) == 0) {
-        status[1] = 90;
-        status[2] = static_cast<int>(blockIdx.x);
-        status[3] = static_cast<int>(threadIdx.x);
-      }
-      atomicExch(const_cast<unsigned int*>(sync) + kAbort, 1u);
-      gone = true;
-    }
+    if ((++polls & 63u) == 0u && wait_is_over(sync, status, polls)) gone = true;
     return !gone;
   }
-  // Block barrier; true when any thread gave up. The spin count starts anew.
+  // Block barrier; true when any thread gave up. The count starts anew.
   __device__ __forceinline__ bool left() {
-    spins = 0;
+    polls = 0;
     return __syncthreads_or(gone) != 0;
   }
 };
