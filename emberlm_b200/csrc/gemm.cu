@@ -11,6 +11,8 @@ int gemm_tcgen05(const float* A, const float* B, float* C, int64_t M, int64_t N,
 void gemm_set_kblock_limit(int k_blocks);
 int gemm_bf16_tcgen05(const void* A, const void* B, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
                       int64_t ldc, cudaStream_t stream);
+int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const float* B2, float* C, int64_t M, int64_t N, int64_t K, int64_t lda,
+                       int64_t ldb, int64_t ldc, int transa, int transb, int epilogue, const float* aux, int run, cudaStream_t stream);
 int gemm_3xtf32(const float* A, const float* B, float* C, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int transa, int transb, int epilogue,
                 const float* aux, cudaStream_t stream);
@@ -204,6 +206,10 @@ int ctdk_gemm_ws(const float* A, const float* B, float* C, int64_t M, int64_t N,
   split_tf32_kernel<<<blocks(nb / 4), 256, 0, s>>>(B, b_hi, b_lo, nb / 4);
   rc = check_launch("ctdk_gemm_ws(split B)");
   if (rc != CTDK_OK) return rc;
+  void* tok = prof_begin(CTDK_PROF_GEMM, 2.0 * static_cast<double>(M) * N * K, s);
+  rc = gemm_split_tcgen05(a_hi, a_lo, b_hi, b_lo, C, M, N, K, lda, ldb, ldc, transa, transb, epilogue, aux, 16, s);
+  prof_end(tok, s);
+  if (rc <= 0) return rc;
   // the leading product in accumulation runs of at most 16 k-blocks (512 deep); the two correction
   // products are 2^-11 of it and keep the usual schedule
   gemm_set_kblock_limit(16);

@@ -19,6 +19,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 
@@ -113,12 +114,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(final_bar + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool grouped = BF16 && args.tiles != nullptr;
-  const int m_blocks = grouped ? args.tiles[args.max_tiles] : (args.M + BM - 1) / BM;
-  const int n_blocks = (args.N + TN - 1) / TN;
-  const int num_tiles = m_blocks * n_blocks;
-  const int k_blocks = (args.K + kElems - 1) / kElems;
-  const int num_units = num_tiles * args.splits;  // unit u: tile u % num_tiles, k-range u / num_tiles
+  pdl_launch();   // the next kernel in the stream may set itself up while this one runs
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::kStages; ++s) {
@@ -142,6 +138,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();     // operands (and C, when it is accumulated into) come from earlier kernels
+  const bool grouped = BF16 && args.tiles != nullptr;
+  const int m_blocks = grouped ? args.tiles[args.max_tiles] : (args.M + BM - 1) / BM;
+  const int n_blocks = (args.N + TN - 1) / TN;
+  const int num_tiles = m_blocks * n_blocks;
+  const int k_blocks = (args.K + kElems - 1) / kElems;
+  const int num_units = num_tiles * args.splits;  // unit u: tile u % num_tiles, k-range u / num_tiles
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
@@ -378,6 +381,231 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // ----------------------------------------------------------------------------------------
+// K split over a cluster: products with too few tiles for the chip (a few hundred rows)
+// ----------------------------------------------------------------------------------------
+// A one-CTA tile of 128 x 128 takes about 0.2 us a k-block however idle the rest of the chip is: SmolLM2-135M on 127
+// rows has 5 to 24 tiles a product and spent 14 to 15 us on each, three quarters of it in the serial main loop. Here the
+// S CTAs of a cluster (2, 4 or 8) share a tile: each multiplies one range of K into its tensor memory, sends every other
+// CTA its columns of that partial tile through distributed shared memory, and after one cluster barrier adds up the S
+// parts of its own columns in the order of the ranges. Against a split over the grid there is no zeroing launch, no
+// atomics, any epilogue, and the result is the same from run to run.
+//
+// With `sweeps` == 3 the ranges run over three products, A B, A B2 and A2 B: the 3xTF32 form, one launch instead of
+// three. Ranges [0, lead) share the first product, the others the two corrections.
+template <int BN>
+struct ClusterCfg {
+  static constexpr int kBTileBytes = BN * BK * 4;
+  static constexpr int kStageBytes = kATileBytes + kBTileBytes;
+  static constexpr int kStages = BN == 128 ? 4 : 6;
+  static constexpr int kPitch = BM + 2;   // float4s between two column groups: rows of a quarter warp in different banks
+  static constexpr int kPartBytes = BN / 4 * kPitch * 16;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kPartBytes + 1024 /*align*/ + 256 /*barriers*/;
+};
+struct ClusterArgs {
+  float* C;
+  const float* aux;
+  int64_t ldc;
+  int M, N, K, epilogue, vec_ok;
+  int S, sweeps, lead;
+  int* status;
+};
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address of this CTA's shared memory `addr` in the CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+template <int BN, bool A_MN, bool B_MN, bool BF16>
+__global__ void __launch_bounds__(kThreads, 1)
+    gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
+                        const __grid_constant__ CUtensorMap tmB2, const ClusterArgs args) {
+  static_assert(!BF16 || (!A_MN && !B_MN), "bfloat16 operands are K-major");
+  using C = ClusterCfg<BN>;
+  constexpr int kElems = BF16 ? BKH : BK;
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  unsigned char* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
+  float4* parts = reinterpret_cast<float4*>(smem + C::kStages * C::kStageBytes);   // [S][columns / 4][kPitch]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kStages * C::kStageBytes + C::kPartBytes);
+  uint64_t* full = bars;
+  uint64_t* empty = bars + C::kStages;
+  uint64_t* tfull = bars + 2 * C::kStages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_launch();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::kStages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, BN);
+    tmem_relinquish();
+    tc_fence_before();
+  }
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  cluster_sync();   // every CTA of the cluster is there before its shared memory is written
+  pdl_wait();
+
+  const int S = args.S, rank = static_cast<int>(blockIdx.x) % S, clusters = static_cast<int>(gridDim.x) / S;
+  const int m_blocks = (args.M + BM - 1) / BM, n_blocks = (args.N + BN - 1) / BN, tiles = m_blocks * n_blocks;
+  const int k_blocks = (args.K + kElems - 1) / kElems;
+  // this CTA's range of the sweeps' k-blocks
+  int kb0, kb1;
+  if (args.sweeps == 1) {
+    kb0 = rank * k_blocks / S;
+    kb1 = (rank + 1) * k_blocks / S;
+  } else if (rank < args.lead) {
+    kb0 = rank * k_blocks / args.lead;
+    kb1 = (rank + 1) * k_blocks / args.lead;
+  } else {
+    const int n = S - args.lead, r = rank - args.lead;
+    kb0 = k_blocks + r * 2 * k_blocks / n;
+    kb1 = k_blocks + (r + 1) * 2 * k_blocks / n;
+  }
+  const int cols = BN / S, quads = cols / 4;   // columns of the tile that this CTA finishes
+  int s = 0;
+  uint32_t ph = 0, tile_ph = 0;
+  bool ok = true;
+  for (int tile = static_cast<int>(blockIdx.x) / S; tile < tiles; tile += clusters, tile_ph ^= 1u) {
+    int mb, nb;
+    tile_coords(tile, m_blocks, n_blocks, mb, nb);
+    if (warp == 0) {
+      if (lane == 0) {
+        const int m0 = mb * BM, n0 = nb * BN;
+        for (int kb = kb0; kb < kb1 && ok; ++kb) {
+          if (!mbar_wait_bounded(&empty[s], ph ^ 1u, args.status, 1)) {
+            ok = false;
+            break;
+          }
+          unsigned char* a_dst = smem + s * C::kStageBytes;
+          unsigned char* b_dst = a_dst + kATileBytes;
+          mbar_expect_tx(&full[s], C::kStageBytes);
+          const int sweep = kb / k_blocks, k0 = (kb - sweep * k_blocks) * kElems;
+          const CUtensorMap* ma = sweep == 2 ? &tmA2 : &tmA;
+          const CUtensorMap* mbp = sweep == 1 ? &tmB2 : &tmB;
+          if (A_MN) {
+#pragma unroll
+            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * kChunkBytes, ma, &full[s], m0 + 32 * c, k0);
+          } else {
+            tma_load_2d(a_dst, ma, &full[s], k0, m0);
+          }
+          if (B_MN) {
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) tma_load_2d(b_dst + c * kChunkBytes, mbp, &full[s], n0 + 32 * c, k0);
+          } else {
+            tma_load_2d(b_dst, mbp, &full[s], k0, n0);
+          }
+          if (++s == C::kStages) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      if (lane == 0) {
+        constexpr uint32_t idesc = make_idesc(A_MN, B_MN, BN, BF16 ? 1u : 2u);
+        for (int kb = kb0; kb < kb1 && ok; ++kb) {
+          if (!mbar_wait_bounded(&full[s], ph, args.status, 3)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes), b_addr = a_addr + kATileBytes;
+#pragma unroll
+          for (int ks = 0; ks < BK / 8; ++ks) {   // descriptors as in gemm_tf32_kernel
+            const uint64_t adesc = A_MN ? make_smem_desc(a_addr + ks * 1024, kChunkBytes, 512, kLayoutSw128Base32)
+                                        : make_smem_desc(a_addr + ks * 32, 16, 1024, kLayoutSw128);
+            const uint64_t bdesc = B_MN ? make_smem_desc(b_addr + ks * 1024, kChunkBytes, 512, kLayoutSw128Base32)
+                                        : make_smem_desc(b_addr + ks * 32, 16, 1024, kLayoutSw128);
+            if (BF16) umma_bf16(tmem_base, adesc, bdesc, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
+            else umma_tf32(tmem_base, adesc, bdesc, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
+          }
+          umma_commit(&empty[s]);
+          if (++s == C::kStages) {
+            s = 0;
+            ph ^= 1u;
+          }
+        }
+        umma_commit(tfull);   // also behind a wait that ran out: nothing of this CTA is then in flight when it goes on
+        mbar_wait_bounded(tfull, tile_ph, args.status, 4);
+      }
+      __syncwarp();
+    } else {
+      const int q = warp & 3, row = q * 32 + lane;
+      if (!mbar_wait_bounded(tfull, tile_ph, args.status, 5)) ok = false;
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll 1
+      for (int ch = 0; ch < BN / 32; ++ch) {
+        float v[32];
+        tmem_ld_32x32(t_row + static_cast<uint32_t>(ch * 32), v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int col = ch * 32 + 4 * j, dst = col / cols, quad = (col - dst * cols) >> 2;
+          store_remote(in_cta(smem_u32(parts + (rank * quads + quad) * C::kPitch + row), static_cast<uint32_t>(dst)), v[4 * j], v[4 * j + 1],
+                       v[4 * j + 2], v[4 * j + 3]);
+        }
+        __syncwarp();
+      }
+      tc_fence_before();
+    }
+    __syncwarp();
+    cluster_sync();   // all parts of this CTA's columns are there, and its tensor memory has been read
+    tc_fence_after();
+    for (int i = threadIdx.x; i < quads * BM; i += kThreads) {
+      const int quad = i % quads, row = i / quads;
+      float4 v = parts[quad * C::kPitch + row];
+      for (int r = 1; r < S; ++r) {
+        const float4 w = parts[(r * quads + quad) * C::kPitch + row];
+        v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+      }
+      const int64_t grow = static_cast<int64_t>(mb) * BM + row;
+      const int col = nb * BN + rank * cols + 4 * quad;
+      if (grow >= args.M || col >= args.N) continue;
+      float* c = args.C + grow * args.ldc + col;
+      const float* x = args.epilogue == CTDK_EPI_ACCUMULATE ? c : (args.epilogue == CTDK_EPI_RESIDUAL ? args.aux + grow * args.ldc + col : nullptr);
+      if (args.vec_ok && col + 4 <= args.N) {
+        if (x != nullptr) {
+          const float4 w = *reinterpret_cast<const float4*>(x);
+          v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+        }
+        *reinterpret_cast<float4*>(c) = v;
+      } else {
+        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (col + k < args.N) c[k] = e[k] + (x != nullptr ? x[k] : 0.0f);
+      }
+    }
+    __syncwarp();
+    cluster_sync();   // the parts may be written again, and no CTA leaves while another still writes to it
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, BN);
+  }
+}
+
+// ----------------------------------------------------------------------------------------
 // Host side
 // ----------------------------------------------------------------------------------------
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
@@ -478,7 +706,8 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args,
   const int tiles = m_blocks * n_blocks * args.splits;
   const int sms = sm_count();
   const int grid = tiles < sms ? tiles : sms;
-  kern<<<grid, kThreads, C::kSmemBytes, stream>>>(ta, tb, args);
+  const cudaError_t le = launch_pdl(kern, dim3(grid), dim3(kThreads), C::kSmemBytes, stream, ta, tb, args);
+  if (le != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: launch failed: %s", cudaGetErrorString(le));
   return check_launch("ctdk_gemm(tcgen05)");
 }
 
@@ -489,6 +718,73 @@ int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMa
   if (!a_mn && b_mn) return launch<BN, false, true>(ta, tb, args, stream);
   if (a_mn && !b_mn) return launch<BN, true, false>(ta, tb, args, stream);
   return launch<BN, true, true>(ta, tb, args, stream);
+}
+
+template <int BN, bool A_MN, bool B_MN, bool BF16 = false>
+int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ta2, const CUtensorMap& tb2, const ClusterArgs& args,
+                   int clusters, cudaStream_t stream) {
+  using C = ClusterCfg<BN>;
+  auto* kern = gemm_cluster_kernel<BN, A_MN, B_MN, BF16>;
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm(cluster): shared memory opt-in failed: %s", cudaGetErrorString(e));
+    attr_set[dev] = true;
+  }
+  const int tiles = ((args.M + BM - 1) / BM) * ((args.N + BN - 1) / BN);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((tiles < clusters ? tiles : clusters) * args.S);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = args.S;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, ta2, tb2, args);
+  if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm(cluster): launch failed: %s", cudaGetErrorString(e));
+  return check_launch("ctdk_gemm(tcgen05, cluster)");
+}
+template <int BN>
+int launch_cluster_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ta2, const CUtensorMap& tb2,
+                         const ClusterArgs& args, int clusters, cudaStream_t stream) {
+  if (!a_mn && !b_mn) return launch_cluster<BN, false, false>(ta, tb, ta2, tb2, args, clusters, stream);
+  if (!a_mn && b_mn) return launch_cluster<BN, false, true>(ta, tb, ta2, tb2, args, clusters, stream);
+  if (a_mn && !b_mn) return launch_cluster<BN, true, false>(ta, tb, ta2, tb2, args, clusters, stream);
+  return launch_cluster<BN, true, true>(ta, tb, ta2, tb2, args, clusters, stream);
+}
+
+// Clusters of S CTAs (one per SM) that run at a time; a GPC's SMs that do not fill a cluster stay idle.
+int clusters_of(int S) {
+  const int sms = sm_budget();
+  return S == 8 ? sms / 9 : (S == 4 ? sms / 4 - 1 : sms / S);
+}
+
+// Estimated time of a product on the cluster kernel in the unit of choose_tile (a k-block of a 256-wide tile), and its
+// tile width and cluster size.
+double choose_cluster(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* s_out) {
+  double best = 1e300;
+  const int widths[2] = {128, 64};
+  for (int w : widths) {
+    const int64_t tiles = ((M + BM - 1) / BM) * ((N + w - 1) / w);
+    for (int S = 8; S >= 2; S /= 2) {
+      if (k_blocks < 2 * S) continue;   // every CTA has a range worth its share of the exchange
+      if (tiles > clusters_of(S)) continue;   // one tile a cluster: the exchange does not overlap the next tile's loop
+      const double t = static_cast<double>((k_blocks + S - 1) / S) * (w == 128 ? 0.6 : 0.45) + (w == 128 ? 6.0 : 5.0);
+      if (t < best * 0.97) {
+        best = t;
+        *bn_out = w;
+        *s_out = S;
+      }
+    }
+  }
+  return best;
 }
 
 }  // namespace
@@ -586,7 +882,7 @@ void gemm_set_kblock_limit(int k_blocks) { t_kblock_limit = k_blocks; }
 namespace {
 
 // Tile width, K split and one-CTA / paired-CTA kernel for an M x N product of k_blocks stage rows.
-void choose_tile(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* splits_out, bool* pair_out) {
+double choose_tile(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* splits_out, bool* pair_out) {
   // Tile width and K split: estimated time = rounds of the persistent grid x k-blocks per
   // unit x relative cost of a k-block (a 128-wide tile does half the work of a 256-wide one
   // but moves 2/3 of the operand bytes, hence the 0.6). Splitting K only pays when the output
@@ -594,8 +890,9 @@ void choose_tile(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* split
   const int sms = sm_budget();
   const int64_t m_blocks = (M + BM - 1) / BM;
   int bn = 64, splits = 1;
+  double best = static_cast<double>((m_blocks + sms - 1) / sms) * (static_cast<double>(k_blocks) + 6.0) * 0.45;
   if (N > 64) {
-    double best = 1e300;
+    best = 1e300;
     const int widths[2] = {256, 128};
     for (int wi = 0; wi < 2; ++wi) {
       const int w = widths[wi];
@@ -657,6 +954,8 @@ void choose_tile(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* split
   *bn_out = bn;
   *splits_out = splits;
   *pair_out = use_pair;
+  // splitting K over the grid needs a launch that zeroes the output, about 3 us
+  return best + (splits > 1 ? 8.0 : 0.0);
 }
 
 }  // namespace
@@ -676,7 +975,24 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
   const int64_t k_blocks = (K + BK - 1) / BK;
   int bn, splits;
   bool use_pair;
-  choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
+  const double plain = choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
+  // From 256 rows on the order of additions stays as it is: the forms with a fused epilogue, which begin there, give the
+  // same bits as the product and the kernel behind it. (Weight gradients that are split over the grid were tried on
+  // clusters: SmolLM2-135M on 4 x 511 positions 10.9 -> 11.4 ms, the clusters hold SMs that the main stream needs.)
+  if (!use_pair && t_kblock_limit == 0 && M < 256) {
+    int cbn = 0, S = 0;
+    if (choose_cluster(M, N, k_blocks, &cbn, &S) < plain) {
+      CUtensorMap ta, tb;
+      int rc = a_mn ? make_map(&ta, A, M, K, lda, BK, true, false) : make_map(&ta, A, K, M, lda, BM, false, false);
+      if (rc == CTDK_OK) rc = b_mn ? make_map(&tb, B, N, K, ldb, BK, true, false) : make_map(&tb, B, K, N, ldb, cbn, false, false);
+      if (rc != CTDK_OK) return rc;
+      ClusterArgs c{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, S, 1, 0, device_status_word()};
+      c.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
+      if (c.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
+      return cbn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta, tb, c, clusters_of(S), stream)
+                        : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta, tb, c, clusters_of(S), stream);
+    }
+  }
 
   if (t_kblock_limit > 0) {
     int64_t need = (k_blocks + t_kblock_limit - 1) / t_kblock_limit;
@@ -787,8 +1103,11 @@ int gemm_bf16_tcgen05(const void* A, const void* B, float* Cp, int64_t M, int64_
   const int64_t k_blocks = (K + BKH - 1) / BKH;
   int bn, splits;
   bool use_pair;
-  choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
-  if (bn == 64 && splits == 1)   // one narrow column of tiles (low-rank factors): split K while SMs are idle
+  const double plain = choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
+  int cbn = 0, S = 0;
+  const bool cluster = !use_pair && choose_cluster(M, N, k_blocks, &cbn, &S) < plain;
+  if (cluster) bn = cbn;
+  if (!cluster && bn == 64 && splits == 1)   // one narrow column of tiles (low-rank factors): split K while SMs are idle
     while ((M + BM - 1) / BM * splits * 2 <= sm_budget() && k_blocks / (splits * 2) >= 8) splits *= 2;
   auto map_bf16 = [](CUtensorMap* map, const void* base, int64_t inner, int64_t outer, int64_t ld, int box_rows) {
     const uint64_t dims[2] = {static_cast<uint64_t>(inner), static_cast<uint64_t>(outer)}, strides[1] = {static_cast<uint64_t>(ld) * 2};
@@ -802,6 +1121,11 @@ int gemm_bf16_tcgen05(const void* A, const void* B, float* Cp, int64_t M, int64_
   int* st = device_status_word();
   if (st == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
   const int vec = (a16(Cp) && (ldc & 3) == 0) ? 1 : 0;
+  if (cluster) {
+    const ClusterArgs c{Cp, nullptr, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), CTDK_EPI_STORE, vec, S, 1, 0, st};
+    return bn == 128 ? launch_cluster<128, false, false, true>(ta, tb, ta, tb, c, clusters_of(S), stream)
+                     : launch_cluster<64, false, false, true>(ta, tb, ta, tb, c, clusters_of(S), stream);
+  }
   if (splits > 1) {
     const cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float),
                                             static_cast<size_t>(M), stream);
@@ -871,11 +1195,58 @@ int gemm_bf16_out16(const void* A, int64_t lda, const void* B, int64_t ldb, __nv
   return up_row > 0 ? launch_out16<kOutGlu>(bn, ta, tb, args, stream) : launch_out16<kOutBf16>(bn, ta, tb, args, stream);
 }
 
-// Near-fp32 GEMM (3xTF32 split). Returns 1 (not eligible) until the split kernel is built,
-// so the caller computes the exact fp32 result with the SIMT kernel.
+// Near-fp32 GEMM (3xTF32 split) is ctdk_gemm_ws; without its workspace the caller takes the exact SIMT kernel.
 int gemm_3xtf32(const float*, const float*, float*, int64_t, int64_t, int64_t, int64_t, int64_t,
                 int64_t, int, int, int, const float*, cudaStream_t) {
   return 1;
+}
+
+// C = A B + A B2 + A2 B (operands split into high and low parts: the 3xTF32 product) in one launch of the cluster kernel.
+// The first product is accumulated in runs of at most `run` k-blocks. Returns 1 when the shape does not suit it: more
+// tiles than clusters (903 rows of SmolLM2-135M in several rounds a product: 38.4 -> 40.2 ms a step), or a K whose runs
+// do not fit a cluster.
+int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const float* B2, float* Cp, int64_t M, int64_t N, int64_t K, int64_t lda,
+                       int64_t ldb, int64_t ldc, int transa, int transb, int epilogue, const float* aux, int run, cudaStream_t stream) {
+  auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (!a16(A) || !a16(B) || !a16(A2) || !a16(B2) || (lda & 3) || (ldb & 3)) return 1;
+  if (M < 1 || N < 8 || K < 1 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX / 4) return 1;
+  const bool a_mn = transa != 0, b_mn = transb == 0;
+  const int64_t k_blocks = (K + BK - 1) / BK;
+  const int64_t m_blocks = (M + BM - 1) / BM;
+  // the first product's CTAs: as many as its runs need, or its share of the work
+  int best_bn = 0, best_s = 0, best_lead = 0;
+  double best = 1e300;
+  const int widths[2] = {128, 64};
+  for (int w : widths)
+    for (int S = 2; S <= 8; S *= 2) {
+      const int64_t runs = (k_blocks + run - 1) / run;
+      const int64_t lead = runs > (S + 2) / 3 ? runs : (S + 2) / 3;
+      if (lead >= S || m_blocks * ((N + w - 1) / w) > clusters_of(S) || k_blocks < lead || 2 * k_blocks < S - lead) continue;   // every CTA has a range
+      const int64_t longest = std::max((k_blocks + lead - 1) / lead, (2 * k_blocks + S - lead - 1) / (S - lead));
+      const double t = static_cast<double>(longest) * (w == 128 ? 0.6 : 0.45) + (w == 128 ? 6.0 : 5.0);
+      if (t < best * 0.97) {
+        best = t;
+        best_bn = w;
+        best_s = S;
+        best_lead = static_cast<int>(lead);
+      }
+    }
+  if (best_s == 0) return 1;
+  auto map_a = [&](CUtensorMap* m, const float* p) { return a_mn ? make_map(m, p, M, K, lda, BK, true, false) : make_map(m, p, K, M, lda, BM, false, false); };
+  auto map_b = [&](CUtensorMap* m, const float* p) {
+    return b_mn ? make_map(m, p, N, K, ldb, BK, true, false) : make_map(m, p, K, N, ldb, best_bn, false, false);
+  };
+  CUtensorMap ta, tb, ta2, tb2;
+  int rc = map_a(&ta, A);
+  if (rc == CTDK_OK) rc = map_a(&ta2, A2);
+  if (rc == CTDK_OK) rc = map_b(&tb, B);
+  if (rc == CTDK_OK) rc = map_b(&tb2, B2);
+  if (rc != CTDK_OK) return rc;
+  ClusterArgs c{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, best_s, 3, best_lead, device_status_word()};
+  c.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
+  if (c.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
+  return best_bn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream)
+                        : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream);
 }
 
 }  // namespace ctdk

@@ -1,0 +1,58 @@
+"""Products with few tiles: K split over the CTAs of a cluster. Small integers are exact in TF32, so a wrong tile, range
+or column exchange shows as a wrong integer; the parts are added in a fixed order, so two runs agree bit for bit."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _ints(shape, seed):
+    import torch
+
+    return torch.randint(-3, 4, shape, generator=torch.Generator("cuda").manual_seed(seed), device="cuda").float()
+
+
+# one and several rows of tiles, ragged edges (N = 130: rows that cannot be stored in fours), the shortest K of each cluster
+# size (2, 4 and 8 CTAs: 128, 256 and 512), a K that leaves ranges of different lengths, more tiles than clusters
+SHAPES = [(1, 576, 576), (127, 960, 576), (37, 576, 1536), (129, 130, 1000), (300, 3072, 576), (5, 64, 512), (64, 192, 256), (128, 8, 128),
+          (200, 2048, 2052)]
+
+
+@pytest.mark.parametrize("epilogue", ["store", "accumulate", "residual"])
+@pytest.mark.parametrize("ta,tb", [(0, 1), (0, 0), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("precision", ["tf32", "3xtf32"])
+def test_exact_and_repeatable(precision, M, N, K, ta, tb, epilogue):
+    import torch
+
+    from emberlm_b200 import lib, ops
+
+    if (ta and M % 4) or (not tb and N % 4):
+        pytest.skip("rows of the operand are not 16-byte aligned: another kernel's")
+    a, b, c = _ints((K, M) if ta else (M, K), 1), _ints((N, K) if tb else (K, N), 2), _ints((M, N), 3)
+    want = ((a.T if ta else a).double() @ (b.T if tb else b).double() + (0 if epilogue == "store" else c.double())).float()
+    p = lib.GEMM_TF32 if precision == "tf32" else lib.GEMM_3XTF32
+    got = []
+    for _ in range(2):
+        if epilogue == "accumulate":
+            got.append(ops.matmul(a, b, bool(ta), bool(tb), p, out=c.clone(), epilogue=lib.EPI_ACCUMULATE))
+        elif epilogue == "residual":
+            got.append(ops.matmul(a, b, bool(ta), bool(tb), p, epilogue=lib.EPI_RESIDUAL, aux=c))
+        else:
+            got.append(ops.matmul(a, b, bool(ta), bool(tb), p))
+    assert torch.equal(got[0], want) and torch.equal(got[1], want)
+
+
+@pytest.mark.parametrize("M,N,K", [(127, 960, 576), (903, 3072, 576), (576, 1536, 903)])
+def test_random_products(M, N, K):
+    """TF32 rounds each operand by at most 2^-11: a product of independent values errs by about 2^-11 sqrt(2 / 3) of its
+    size, well under 1e-3 in the 2-norm. 3xTF32 leaves 2^-21 an operand and fp32 sums: 2e-6."""
+    import torch
+
+    from emberlm_b200 import lib, ops
+
+    gen = torch.Generator("cuda").manual_seed(4)
+    a, b = (torch.randn(s, generator=gen, device="cuda") for s in ((M, K), (N, K)))
+    want = a.double() @ b.double().T
+    for p, limit in ((lib.GEMM_TF32, 1e-3), (lib.GEMM_3XTF32, 2e-6)):
+        err = (ops.matmul(a, b, False, True, p).double() - want).norm() / want.norm()
+        assert err < limit, (p, float(err))
