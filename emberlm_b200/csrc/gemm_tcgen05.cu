@@ -61,7 +61,26 @@ struct GemmArgs {
   // bfloat16 outputs (kOutBf16, kOutGlu)
   __nv_bfloat16* out16 = nullptr;
   int up_row = 0;   // kOutGlu: rows of B between a gate row and its up row; N counts pairs
+  // lead > 0: the 3xTF32 form A B + A B2 + A2 B. The first `lead` of the `splits` ranges share the first product, the
+  // others the two corrections one behind the other.
+  int lead = 0;
 };
+// The k-blocks of range `split`; those of the corrections count from k_blocks on.
+__device__ __forceinline__ void k_range(const GemmArgs& args, int split, int k_blocks, int& kb0, int& kb1) {
+  int first = 0, total = k_blocks, part = split, parts = args.splits;
+  if (args.lead > 0) {
+    if (split < args.lead) {
+      parts = args.lead;
+    } else {
+      first = k_blocks;
+      total = 2 * k_blocks;
+      part -= args.lead;
+      parts -= args.lead;
+    }
+  }
+  kb0 = first + static_cast<int>(static_cast<int64_t>(part) * total / parts);
+  kb1 = first + static_cast<int>(static_cast<int64_t>(part + 1) * total / parts);
+}
 
 // What the epilogue writes: fp32 sums, the same as bfloat16, or bfloat16 silu(gate) up of the two halves of
 // a tile's columns (the first half holds gate rows of B, the second their up rows).
@@ -96,7 +115,8 @@ __device__ __forceinline__ void tile_coords(int tile, int m_blocks, int n_blocks
 template <int BN, bool A_MN, bool B_MN, bool BF16, int OUT>
 __global__ void __launch_bounds__(kThreads, 1)
     gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmA,
-                     const __grid_constant__ CUtensorMap tmB, const GemmArgs args) {
+                     const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmA2,
+                     const __grid_constant__ CUtensorMap tmB2, const GemmArgs args) {
   static_assert(!BF16 || (!A_MN && !B_MN), "bfloat16 operands are K-major");
   static_assert(OUT == kOutF32 || BF16, "bfloat16 outputs go with bfloat16 operands");
   constexpr int TN = OUT == kOutGlu ? BN / 2 : BN;   // output columns of a tile
@@ -158,8 +178,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int m0 = mb * BM, n0 = nb * TN;
         const int b_row = grouped ? n0 + args.tiles[mb] * args.n_pitch : n0;
         const int split = unit / num_tiles;
-        const int kb0 = static_cast<int>(static_cast<int64_t>(split) * k_blocks / args.splits);
-        const int kb1 = static_cast<int>(static_cast<int64_t>(split + 1) * k_blocks / args.splits);
+        int kb0, kb1;
+        k_range(args, split, k_blocks, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_bounded(&empty[s], ph ^ 1u, args.status, 1)) {
             ok = false;
@@ -168,21 +188,23 @@ __global__ void __launch_bounds__(kThreads, 1)
           unsigned char* a_dst = smem + s * C::kStageBytes;
           unsigned char* b_dst = a_dst + kATileBytes;
           mbar_expect_tx(&full[s], C::kStageBytes);
-          const int k0 = kb * kElems;
+          const int sweep = kb < k_blocks ? 0 : (kb < 2 * k_blocks ? 1 : 2), k0 = (kb - sweep * k_blocks) * kElems;
+          const CUtensorMap* ma = sweep == 2 ? &tmA2 : &tmA;
+          const CUtensorMap* mbp = sweep == 1 ? &tmB2 : &tmB;
           if (A_MN) {
 #pragma unroll
             for (int c = 0; c < BM / 32; ++c)
-              tma_load_2d(a_dst + c * kChunkBytes, &tmA, &full[s], m0 + 32 * c, k0);
+              tma_load_2d(a_dst + c * kChunkBytes, ma, &full[s], m0 + 32 * c, k0);
           } else {
-            tma_load_2d(a_dst, &tmA, &full[s], k0, m0);
+            tma_load_2d(a_dst, ma, &full[s], k0, m0);
           }
           if (B_MN) {
 #pragma unroll
             for (int c = 0; c < BN / 32; ++c)
-              tma_load_2d(b_dst + c * kChunkBytes, &tmB, &full[s], n0 + 32 * c, k0);
+              tma_load_2d(b_dst + c * kChunkBytes, mbp, &full[s], n0 + 32 * c, k0);
           } else {
-            tma_load_2d(b_dst, &tmB, &full[s], k0, b_row);
-            if (OUT == kOutGlu) tma_load_2d(b_dst + C::kBTileBytes / 2, &tmB, &full[s], k0, b_row + args.up_row);
+            tma_load_2d(b_dst, mbp, &full[s], k0, b_row);
+            if (OUT == kOutGlu) tma_load_2d(b_dst + C::kBTileBytes / 2, mbp, &full[s], k0, b_row + args.up_row);
           }
           if (++s == C::kStages) {
             s = 0;
@@ -202,8 +224,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       int it = 0;
       for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x, ++it) {
         const int split = unit / num_tiles;
-        const int kb0 = static_cast<int>(static_cast<int64_t>(split) * k_blocks / args.splits);
-        const int kb1 = static_cast<int>(static_cast<int64_t>(split + 1) * k_blocks / args.splits);
+        int kb0, kb1;
+        k_range(args, split, k_blocks, kb0, kb1);
         const int acc = it & 1;
         const uint32_t acc_ph = (static_cast<uint32_t>(it) >> 1) & 1u;
         if (!mbar_wait_bounded(&tempty[acc], acc_ph ^ 1u, args.status, 2)) {
@@ -687,7 +709,7 @@ namespace {
 
 template <int BN, bool A_MN, bool B_MN, bool BF16 = false, int OUT = kOutF32>
 int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args,
-           cudaStream_t stream) {
+           cudaStream_t stream, const CUtensorMap* ta2 = nullptr, const CUtensorMap* tb2 = nullptr) {
   using C = Cfg<BN>;
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -706,18 +728,19 @@ int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& args,
   const int tiles = m_blocks * n_blocks * args.splits;
   const int sms = sm_count();
   const int grid = tiles < sms ? tiles : sms;
-  const cudaError_t le = launch_pdl(kern, dim3(grid), dim3(kThreads), C::kSmemBytes, stream, ta, tb, args);
+  const cudaError_t le = launch_pdl(kern, dim3(grid), dim3(kThreads), C::kSmemBytes, stream, ta, tb, ta2 != nullptr ? *ta2 : ta,
+                                    tb2 != nullptr ? *tb2 : tb, args);
   if (le != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: launch failed: %s", cudaGetErrorString(le));
   return check_launch("ctdk_gemm(tcgen05)");
 }
 
 template <int BN>
 int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb,
-                   const GemmArgs& args, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch<BN, false, false>(ta, tb, args, stream);
-  if (!a_mn && b_mn) return launch<BN, false, true>(ta, tb, args, stream);
-  if (a_mn && !b_mn) return launch<BN, true, false>(ta, tb, args, stream);
-  return launch<BN, true, true>(ta, tb, args, stream);
+                   const GemmArgs& args, cudaStream_t stream, const CUtensorMap* ta2 = nullptr, const CUtensorMap* tb2 = nullptr) {
+  if (!a_mn && !b_mn) return launch<BN, false, false>(ta, tb, args, stream, ta2, tb2);
+  if (!a_mn && b_mn) return launch<BN, false, true>(ta, tb, args, stream, ta2, tb2);
+  if (a_mn && !b_mn) return launch<BN, true, false>(ta, tb, args, stream, ta2, tb2);
+  return launch<BN, true, true>(ta, tb, args, stream, ta2, tb2);
 }
 
 template <int BN, bool A_MN, bool B_MN, bool BF16 = false>
@@ -1202,9 +1225,10 @@ int gemm_3xtf32(const float*, const float*, float*, int64_t, int64_t, int64_t, i
 }
 
 // C = A B + A B2 + A2 B (operands split into high and low parts: the 3xTF32 product) in one launch of the cluster kernel.
-// The first product is accumulated in runs of at most `run` k-blocks. Returns 1 when the shape does not suit it: more
-// tiles than clusters (903 rows of SmolLM2-135M in several rounds a product: 38.4 -> 40.2 ms a step), or a K whose runs
-// do not fit a cluster.
+// The first product is accumulated in runs of at most `run` k-blocks. With more tiles than clusters, or a K whose runs do
+// not fit a cluster, the ranges are units of the one-CTA kernel that add their tiles at L2 (in several rounds the
+// cluster kernel does not overlap its exchange: 903 rows of SmolLM2-135M 38.4 -> 40.2 ms a step). Returns 1 from about two
+// rounds of tiles on: the paired-CTA kernel's large tiles, three times, are then faster.
 int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const float* B2, float* Cp, int64_t M, int64_t N, int64_t K, int64_t lda,
                        int64_t ldb, int64_t ldc, int transa, int transb, int epilogue, const float* aux, int run, cudaStream_t stream) {
   auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
@@ -1231,7 +1255,26 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
         best_lead = static_cast<int>(lead);
       }
     }
-  if (best_s == 0) return 1;
+  int splits = 0;
+  if (best_s == 0) {
+    const int sms = sm_budget();
+    const int64_t lead = (k_blocks + run - 1) / run;
+    if (m_blocks * ((N + 127) / 128) > 2 * static_cast<int64_t>(sms) || lead > 24) return 1;
+    const int wide[2] = {256, 128};
+    for (int w : wide)
+      for (int64_t more = 1; more <= 2 * lead && more <= 2 * k_blocks; ++more) {
+        if (w == 256 && N <= 128) break;
+        const double rounds = static_cast<double>((m_blocks * ((N + w - 1) / w) * (lead + more) + sms - 1) / sms);
+        const int64_t longest = std::max((k_blocks + lead - 1) / lead, (2 * k_blocks + more - 1) / more);
+        const double t = rounds * (static_cast<double>(longest) + 12.0) * (w == 256 ? 1.0 : 0.6);
+        if (t < best * 0.97) {
+          best = t;
+          best_bn = w;
+          best_lead = static_cast<int>(lead);
+          splits = static_cast<int>(lead + more);
+        }
+      }
+  }
   auto map_a = [&](CUtensorMap* m, const float* p) { return a_mn ? make_map(m, p, M, K, lda, BK, true, false) : make_map(m, p, K, M, lda, BM, false, false); };
   auto map_b = [&](CUtensorMap* m, const float* p) {
     return b_mn ? make_map(m, p, N, K, ldb, BK, true, false) : make_map(m, p, K, N, ldb, best_bn, false, false);
@@ -1242,6 +1285,19 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
   if (rc == CTDK_OK) rc = map_b(&tb, B);
   if (rc == CTDK_OK) rc = map_b(&tb2, B2);
   if (rc != CTDK_OK) return rc;
+  if (splits > 0) {
+    GemmArgs g{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, splits, device_status_word()};
+    g.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
+    g.lead = best_lead;
+    if (g.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
+    if (epilogue != CTDK_EPI_ACCUMULATE) {
+      const cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float),
+                                              static_cast<size_t>(M), stream);
+      if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
+    }
+    return best_bn == 256 ? dispatch_major<256>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2)
+                          : dispatch_major<128>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2);
+  }
   ClusterArgs c{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, best_s, 3, best_lead, device_status_word()};
   c.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
   if (c.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");

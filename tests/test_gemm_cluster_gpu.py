@@ -42,6 +42,28 @@ def test_exact_and_repeatable(precision, M, N, K, ta, tb, epilogue):
     assert torch.equal(got[0], want) and torch.equal(got[1], want)
 
 
+@pytest.mark.parametrize("epilogue", ["store", "accumulate", "residual"])
+@pytest.mark.parametrize("ta,tb", [(0, 1), (0, 0), (1, 0), (1, 1)])
+@pytest.mark.parametrize("M,N,K", [(904, 576, 1536), (1000, 3000, 100), (576, 1536, 904), (260, 100, 6000), (1200, 4096, 32)])
+def test_three_products_in_one_launch(M, N, K, ta, tb, epilogue):
+    """Operands of 12 significant bits have a low part, so the ranges of all three products count; sums stay exact."""
+    import torch
+
+    from emberlm_b200 import lib, ops
+
+    gen = torch.Generator("cuda").manual_seed(5)
+    a, b = (torch.randint(-1, 2, s, generator=gen, device="cuda").float() for s in ((K, M) if ta else (M, K), (N, K) if tb else (K, N)))
+    a[::3] *= 2049.0     # TF32 holds 2048: one more bit than it has
+    c = _ints((M, N), 3)
+    want = ((a.T if ta else a).double() @ (b.T if tb else b).double() + (0 if epilogue == "store" else c.double())).float()
+    if epilogue == "accumulate":
+        got = ops.matmul(a, b, bool(ta), bool(tb), lib.GEMM_3XTF32, out=c.clone(), epilogue=lib.EPI_ACCUMULATE)
+    else:
+        got = ops.matmul(a, b, bool(ta), bool(tb), lib.GEMM_3XTF32, epilogue=lib.EPI_RESIDUAL if epilogue == "residual" else lib.EPI_STORE,
+                         aux=c if epilogue == "residual" else None)
+    assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("M,N,K", [(127, 960, 576), (903, 3072, 576), (576, 1536, 903)])
 def test_random_products(M, N, K):
     """TF32 rounds each operand by at most 2^-11: a product of independent values errs by about 2^-11 sqrt(2 / 3) of its
