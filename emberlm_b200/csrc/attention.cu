@@ -391,11 +391,14 @@ __global__ void __launch_bounds__(128)
 //   dS^T = P^T*(dP^T - delta[q])*scale, dV += P^T dO, dK += dS^T Q.
 // QT = queries per inner tile (64 for D=64, 32 for D=128 to bound registers).
 // ---------------------------------------------------------------------------------------
+// The query tiles of a key tile (times the heads of the group) are dealt to the R CTAs of a cluster, which add up their
+// dK and dV through distributed shared memory in a fixed order: 3 x 301 positions of SmolLM2-135M have 45 key tiles, the
+// first with 15 query tiles one behind the other.
 template <int D, int QT, bool X3>
 __global__ void __launch_bounds__(128)
     attn_bwd_dkv_kernel(const float* __restrict__ qkv, const float* __restrict__ dout,
                         const float* __restrict__ lse, const float* __restrict__ delta,
-                        float* __restrict__ dqkv, int T, int H, int Hk, float scale) {
+                        float* __restrict__ dqkv, int T, int H, int Hk, float scale, int R) {
   constexpr int P = D + 4;
   extern __shared__ float smem[];
   float* Ks = smem;
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(128)
   float* dOs = Qs + QT * P;
   float* s_lse = dOs + QT * P;  // [QT]
   float* s_del = s_lse + QT;    // [QT]
-  const int kj = blockIdx.x;    // key tile; low tiles have the most query tiles
+  const int kj = blockIdx.x / R, rank = blockIdx.x % R;    // key tile; low tiles have the most query tiles
   const int hk = blockIdx.y, b = blockIdx.z;
   const int G = H / Hk;
   const int64_t RS = static_cast<int64_t>(H + 2 * Hk) * D;
@@ -437,6 +440,7 @@ __global__ void __launch_bounds__(128)
     const float* dobase = dout + static_cast<int64_t>(b) * T * OS + static_cast<int64_t>(h) * D;
     const int64_t lbase = (static_cast<int64_t>(b) * H + h) * T;
     for (int qt = first_qt; qt < n_qt; ++qt) {
+      if ((hh * (n_qt - first_qt) + qt - first_qt) % R != rank) continue;
       const int q0 = qt * QT;
       __syncthreads();  // previous Q/dO tile consumed (and K/V visible on the first pass)
       load_tile<D, QT, 128>(Qs, qbase, RS, q0, T);
@@ -474,6 +478,44 @@ __global__ void __launch_bounds__(128)
     }
   }
 
+  if (R > 1) {
+    __syncthreads();   // K and V have been read: their place takes this CTA's sums
+    float* parts[2] = {Ks, Vs};
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      float(&d)[D / 8][4] = m == 0 ? dk : dv;
+      float* row = parts[m] + (warp * 16 + g) * P + 2 * t;
+#pragma unroll
+      for (int nt = 0; nt < D / 8; ++nt) {
+        *reinterpret_cast<float2*>(row + nt * 8) = make_float2(d[nt][0], d[nt][1]);
+        *reinterpret_cast<float2*>(row + 8 * P + nt * 8) = make_float2(d[nt][2], d[nt][3]);
+      }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int rows = BKV / R;   // this CTA's rows of both sums
+    for (int i = threadIdx.x; i < 2 * rows * (D / 4); i += 128) {
+      const int c = i % (D / 4), r = i / (D / 4) % rows + rank * rows, m = i / (D / 4 * rows);
+      const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(parts[m] + r * P + 4 * c));
+      float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int q = 0; q < R; ++q) {
+        uint32_t there;
+        float4 v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(q));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(there) : "memory");
+        sum = make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
+      }
+      if (k0 + r < T) {
+        float* dst = dqkv + (static_cast<int64_t>(b) * T + k0 + r) * RS + static_cast<int64_t>(H + hk + m * Hk) * D + 4 * c;
+        *reinterpret_cast<float2*>(dst) = make_float2(sum.x, sum.y);
+        *reinterpret_cast<float2*>(dst + 2) = make_float2(sum.z, sum.w);
+      }
+    }
+    __syncwarp();
+    // no CTA leaves while another still reads from it
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return;
+  }
   if (key_a < T) {
     float* pk = dqkv + (static_cast<int64_t>(b) * T + key_a) * RS +
                 static_cast<int64_t>(H + hk) * D;
@@ -546,7 +588,24 @@ int run_bwd_legacy(const float* qkv, const float* dout, const float* lse, const 
   if (do_dkv) {
     rc = set_smem(attn_bwd_dkv_kernel<D, QT, X3>, smem_k, "ctdk_attn_bwd");
     if (rc != CTDK_OK) return rc;
-    attn_bwd_dkv_kernel<D, QT, X3><<<gk, 128, smem_k, s>>>(qkv, dout, lse, delta, dqkv, Ti, H, Hk, scale);
+    // CTAs per key tile: while two a SM are not exceeded, and no more than the first key tile has query tiles
+    const int64_t tiles = static_cast<int64_t>(gk.x) * gk.y * gk.z, chain = static_cast<int64_t>(H / Hk) * ((T + QT - 1) / QT);
+    int R = 1;
+    while (R < 8 && tiles * R * 2 <= 2 * sm_count() && R * 2 <= chain) R *= 2;
+    gk.x *= R;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = gk;
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = smem_k;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = R;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = R > 1 ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_bwd_dkv_kernel<D, QT, X3>, qkv, dout, lse, delta, dqkv, Ti, H, Hk, scale, R);
+    if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "ctdk_attn_bwd(dkv): launch failed: %s", cudaGetErrorString(e));
     rc = check_launch("ctdk_attn_bwd(dkv)");
   }
   return rc;
