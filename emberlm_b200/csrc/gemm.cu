@@ -77,9 +77,11 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// hi = x rounded to TF32 (10-bit mantissa, round to nearest), lo = x - hi (exact in fp32).
-__global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, float* __restrict__ hi,
-                                                         float* __restrict__ lo, int64_t n4) {
+// hi = x rounded to TF32 (10-bit mantissa, round to nearest), lo = x - hi (exact in fp32), for two arrays in one launch.
+__global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, float* __restrict__ x_hi, float* __restrict__ x_lo, int64_t nx4,
+                                                         const float* __restrict__ y, float* __restrict__ y_hi, float* __restrict__ y_lo, int64_t ny4) {
+  pdl_launch();
+  pdl_wait();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   auto sp = [](float v, float& h, float& l) {
     uint32_t r;
@@ -87,15 +89,17 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict
     h = __uint_as_float(r);
     l = v - h;
   };
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
-    const float4 v = reinterpret_cast<const float4*>(x)[i];
+  for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < nx4 + ny4; k += stride) {
+    const bool first = k < nx4;
+    const int64_t i = first ? k : k - nx4;
+    const float4 v = reinterpret_cast<const float4*>(first ? x : y)[i];
     float4 h, l;
     sp(v.x, h.x, l.x);
     sp(v.y, h.y, l.y);
     sp(v.z, h.z, l.z);
     sp(v.w, h.w, l.w);
-    reinterpret_cast<float4*>(hi)[i] = h;
-    reinterpret_cast<float4*>(lo)[i] = l;
+    reinterpret_cast<float4*>(first ? x_hi : y_hi)[i] = h;
+    reinterpret_cast<float4*>(first ? x_lo : y_lo)[i] = l;
   }
 }
 
@@ -200,11 +204,9 @@ int ctdk_gemm_ws(const float* A, const float* B, float* C, int64_t M, int64_t N,
   float* b_lo = b_hi + up(nb);
   const int cap = sm_count() * 8;
   auto blocks = [&](int64_t n4) { return static_cast<int>(n4 / 256 + 1 < cap ? n4 / 256 + 1 : cap); };
-  split_tf32_kernel<<<blocks(na / 4), 256, 0, s>>>(A, a_hi, a_lo, na / 4);
-  int rc = check_launch("ctdk_gemm_ws(split A)");
-  if (rc != CTDK_OK) return rc;
-  split_tf32_kernel<<<blocks(nb / 4), 256, 0, s>>>(B, b_hi, b_lo, nb / 4);
-  rc = check_launch("ctdk_gemm_ws(split B)");
+  const cudaError_t e = launch_pdl(split_tf32_kernel, dim3(blocks((na + nb) / 4)), dim3(256), 0, s, A, a_hi, a_lo, na / 4, B, b_hi, b_lo, nb / 4);
+  if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "ctdk_gemm_ws: launch failed: %s", cudaGetErrorString(e));
+  int rc = check_launch("ctdk_gemm_ws(split)");
   if (rc != CTDK_OK) return rc;
   void* tok = prof_begin(CTDK_PROF_GEMM, 2.0 * static_cast<double>(M) * N * K, s);
   rc = gemm_split_tcgen05(a_hi, a_lo, b_hi, b_lo, C, M, N, K, lda, ldb, ldc, transa, transb, epilogue, aux, 16, s);
