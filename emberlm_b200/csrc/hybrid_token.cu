@@ -219,6 +219,150 @@ __device__ void stage_mixed(const TokenArgs& a, const TokenPhase& ph, float* sm,
   __syncthreads();
 }
 
+// Keys [j0, j1) of key/value head g for all query heads of the group, into the partial results of range sp: a warp per
+// key, a lane per PP pairs of dimensions (dim even, at most 64 PP), the angles of a warp's keys requested with them. The
+// form below stages tiles of keys behind four block barriers each and has one thread walk a whole score: zutalix-0.6b, 300 +
+// 64 tokens (ranges of about 31 keys of 128 dimensions), 113.1 ms with it and 110.2 with this.
+template <typename T, int PP>
+__device__ __forceinline__ void attention_warps(const TokenPhase& ph, const TokenBranch& br, int g, int sp, int j0, int j1, int slot, float* sm) {
+  constexpr int U = 4, G = 2;   // keys of a warp in flight, heads per pass
+  const int dim = br.dim, P = dim / 2, hq = br.H / br.G, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, stride = dim + kAttnStats;
+  float* qs = sm;                // [hq][dim] rotated, scaled
+  float* kn = qs + hq * dim;     // [dim] this token's key
+  float* scr = kn + dim;         // [kWarps][G][dim + 2]
+  T* cache = static_cast<T*>(br.cache) + static_cast<int64_t>(g) * br.chunk * dim;
+  const bool has_new = slot >= j0 && slot < j1;
+  float2 k[U][PP], cs[U][PP];
+  auto request = [&](int jb) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int j = jb + kWarps * u;
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int p = lane + 32 * i;
+        k[u][i] = make_float2(0.0f, 0.0f);
+        cs[u][i] = make_float2(1.0f, 0.0f);
+        if (j >= j1 || p >= P) continue;
+        if (j != slot) {
+          const T* row = cache + static_cast<int64_t>(j) * dim + 2 * p;
+          if constexpr (sizeof(T) == 2) {
+            const uint32_t w = __ldcg(reinterpret_cast<const unsigned int*>(row));
+            k[u][i] = make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+          } else {
+            k[u][i] = __ldcg(reinterpret_cast<const float2*>(row));
+          }
+        }
+        if (p < br.rot_pairs) cs[u][i] = br.table[static_cast<int64_t>(j) * br.rot_pairs + p];
+      }
+    }
+  };
+  request(j0 + wid);
+  for (int i = threadIdx.x; i < (hq + (has_new ? 1 : 0)) * P; i += kThreads) {
+    const int r = i / P, p = i - r * P, d = 2 * p;
+    const bool key = r == hq;
+    const float* src = ph.proj + (key ? br.col_k + g * dim : br.col_q + (g * hq + r) * dim) + d;
+    const float* bias = (key ? br.b_k + g * dim : br.b_q + (g * hq + r) * dim) + d;
+    float2 rot = make_float2(1.0f, 0.0f);
+    if (p < br.rot_pairs && !key) rot = br.table[static_cast<int64_t>(slot) * br.rot_pairs + p];
+    const float u = ldg_f(src) + bias[0], v = ldg_f(src + 1) + bias[1];
+    if (key) {
+      kn[d] = u;
+      kn[d + 1] = v;
+      cache[static_cast<int64_t>(slot) * dim + d] = from_f<T>(u);
+      cache[static_cast<int64_t>(slot) * dim + d + 1] = from_f<T>(v);
+    } else {
+      qs[r * dim + d] = (u * rot.x - v * rot.y) * br.scale;
+      qs[r * dim + d + 1] = (v * rot.x + u * rot.y) * br.scale;
+    }
+  }
+  __syncthreads();
+  for (int g0 = 0; g0 < hq; g0 += G) {
+    float2 q[G][PP], o[G][PP];
+    float m[G], l[G];
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      m[h] = -FLT_MAX;
+      l[h] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < PP; ++i) {
+        const int p = lane + 32 * i;
+        q[h][i] = g0 + h < hq && p < P ? *reinterpret_cast<const float2*>(qs + (g0 + h) * dim + 2 * p) : make_float2(0.0f, 0.0f);
+        o[h][i] = make_float2(0.0f, 0.0f);
+      }
+    }
+    for (int jb = j0 + wid; jb < j1; jb += kWarps * U) {
+      if (g0 > 0 || jb != j0 + wid) request(jb);
+      float s[U][G];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int h = 0; h < G; ++h) s[u][h] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < PP; ++i) {
+          const int p = lane + 32 * i;
+          if (jb + kWarps * u == slot && p < P) k[u][i] = *reinterpret_cast<const float2*>(kn + 2 * p);
+          const float2 t = k[u][i], f = cs[u][i];
+          const float2 r = make_float2(t.x * f.x - t.y * f.y, t.y * f.x + t.x * f.y);
+#pragma unroll
+          for (int h = 0; h < G; ++h) s[u][h] = fmaf(q[h][i].x, r.x, fmaf(q[h][i].y, r.y, s[u][h]));
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < G; ++h) {
+        float most = m[h];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          s[u][h] = warp_sum(s[u][h]);
+          if (jb + kWarps * u < j1) most = fmaxf(most, s[u][h]);
+        }
+        const float fix = expf(m[h] - most);
+        l[h] *= fix;
+#pragma unroll
+        for (int i = 0; i < PP; ++i) o[h][i] = make_float2(o[h][i].x * fix, o[h][i].y * fix);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (jb + kWarps * u >= j1) continue;
+          const float w = expf(s[u][h] - most);
+          l[h] += w;
+#pragma unroll
+          for (int i = 0; i < PP; ++i) o[h][i] = make_float2(fmaf(w, k[u][i].x, o[h][i].x), fmaf(w, k[u][i].y, o[h][i].y));
+        }
+        m[h] = most;
+      }
+    }
+    if (g0 > 0) __syncthreads();   // the pass before has been merged
+#pragma unroll
+    for (int h = 0; h < G; ++h) {
+      float* dst = scr + (wid * G + h) * stride;
+      if (lane == 0) *reinterpret_cast<float2*>(dst) = make_float2(m[h], l[h]);
+#pragma unroll
+      for (int i = 0; i < PP; ++i)
+        if (lane + 32 * i < P) *reinterpret_cast<float2*>(dst + kAttnStats + 2 * (lane + 32 * i)) = o[h][i];
+    }
+    __syncthreads();
+    const int heads = min(G, hq - g0);
+    for (int i = threadIdx.x; i < heads * dim; i += kThreads) {
+      const int h = i / dim, d = i - h * dim;
+      const float* src = scr + h * stride;
+      float most = -FLT_MAX, sum = 0.0f, out = 0.0f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) most = fmaxf(most, src[w * G * stride]);
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        const float f = expf(src[w * G * stride] - most);
+        sum = fmaf(f, src[w * G * stride + 1], sum);
+        out = fmaf(f, src[w * G * stride + kAttnStats + d], out);
+      }
+      float* dst = br.part + (static_cast<int64_t>(g * hq + g0 + h) * kAttnSplits + sp) * stride;
+      dst[kAttnStats + d] = out;
+      if (d == 0) {
+        dst[0] = most;
+        dst[1] = sum;
+      }
+    }
+  }
+}
+
 // Attention of the new token over one key range of key/value head g, all query heads of the group;
 // the range that arrives last merges them and applies the head gates.
 template <typename T>
@@ -232,112 +376,117 @@ __device__ void attention_item(const TokenPhase& ph, const TokenBranch& br, int 
   n_act = (L + per - 1) / per;
   if (sp >= n_act) return;
   const int j0 = sp * per, j1 = min(L, j0 + per);
-  const int KT = dim <= 128 ? 32 : (dim <= 256 ? 16 : (dim <= 512 ? 8 : 4)), ldk = dim + 1;
-  float* qs = sm;                        // [hq][dim] rotated, scaled
-  float* kr = qs + hq * dim;             // [KT][ldk] keys = values
-  float* kt = kr + KT * ldk;             // [KT][ldk] rotated keys
-  float* sc = kt + KT * ldk;             // [hq][32]
-  float* st = sc + hq * 32;              // [hq][3] maximum, sum, correction
-  float* acc = st + hq * 3;              // [hq][dim]
-  T* cache = static_cast<T*>(br.cache) + static_cast<int64_t>(g) * br.chunk * dim;
-  const int P = (dim + 1) / 2;
-  for (int i = threadIdx.x; i < hq * P; i += kThreads) {
-    const int h = i / P, p = i % P, d = 2 * p;
-    const float* src = ph.proj + br.col_q + (g * hq + h) * dim;
-    const float* bias = br.b_q + (g * hq + h) * dim;
-    const float u = ldg_f(src + d) + bias[d], v = d + 1 < dim ? ldg_f(src + d + 1) + bias[d + 1] : 0.0f;
-    float2 o = make_float2(u, v);
-    if (p < br.rot_pairs) {
-      const float2 cs = br.table[static_cast<int64_t>(slot) * br.rot_pairs + p];
-      o = make_float2(u * cs.x - v * cs.y, v * cs.x + u * cs.y);
-    }
-    qs[h * dim + d] = o.x * br.scale;
-    if (d + 1 < dim) qs[h * dim + d + 1] = o.y * br.scale;
-  }
-  for (int i = threadIdx.x; i < hq * dim; i += kThreads) acc[i] = 0.0f;
-  for (int i = threadIdx.x; i < hq; i += kThreads) {
-    st[i * 3] = -FLT_MAX;
-    st[i * 3 + 1] = 0.0f;
-  }
-  for (int jb = j0; jb < j1; jb += KT) {
-    const int nk = min(KT, j1 - jb);
-    __syncthreads();
-    for (int i = threadIdx.x; i < nk * P; i += kThreads) {
-      const int jj = i / P, p = i % P, d = 2 * p, j = jb + jj;
-      float u, v = 0.0f;
-      T* cr = cache + static_cast<int64_t>(j) * dim + d;
-      if (j == slot) {
-        const float* src = ph.proj + br.col_k + g * dim + d;
-        const float* bias = br.b_k + g * dim + d;
-        u = ldg_f(src) + bias[0];
-        cr[0] = from_f<T>(u);
-        if (d + 1 < dim) {
-          v = ldg_f(src + 1) + bias[1];
-          cr[1] = from_f<T>(v);
-        }
-      } else {
-        u = to_f(cr[0]);
-        if (d + 1 < dim) v = to_f(cr[1]);
-      }
+  const int PS = dim + kAttnStats;
+  if (dim <= 128 && (dim & 1) == 0) {
+    if (dim <= 64) attention_warps<T, 1>(ph, br, g, sp, j0, j1, slot, sm);
+    else attention_warps<T, 2>(ph, br, g, sp, j0, j1, slot, sm);
+  } else {
+    const int KT = dim <= 128 ? 32 : (dim <= 256 ? 16 : (dim <= 512 ? 8 : 4)), ldk = dim + 1;
+    float* qs = sm;                        // [hq][dim] rotated, scaled
+    float* kr = qs + hq * dim;             // [KT][ldk] keys = values
+    float* kt = kr + KT * ldk;             // [KT][ldk] rotated keys
+    float* sc = kt + KT * ldk;             // [hq][32]
+    float* st = sc + hq * 32;              // [hq][3] maximum, sum, correction
+    float* acc = st + hq * 3;              // [hq][dim]
+    T* cache = static_cast<T*>(br.cache) + static_cast<int64_t>(g) * br.chunk * dim;
+    const int P = (dim + 1) / 2;
+    for (int i = threadIdx.x; i < hq * P; i += kThreads) {
+      const int h = i / P, p = i % P, d = 2 * p;
+      const float* src = ph.proj + br.col_q + (g * hq + h) * dim;
+      const float* bias = br.b_q + (g * hq + h) * dim;
+      const float u = ldg_f(src + d) + bias[d], v = d + 1 < dim ? ldg_f(src + d + 1) + bias[d + 1] : 0.0f;
       float2 o = make_float2(u, v);
       if (p < br.rot_pairs) {
-        const float2 cs = br.table[static_cast<int64_t>(j) * br.rot_pairs + p];
+        const float2 cs = br.table[static_cast<int64_t>(slot) * br.rot_pairs + p];
         o = make_float2(u * cs.x - v * cs.y, v * cs.x + u * cs.y);
       }
-      kr[jj * ldk + d] = u;
-      kt[jj * ldk + d] = o.x;
-      if (d + 1 < dim) {
-        kr[jj * ldk + d + 1] = v;
-        kt[jj * ldk + d + 1] = o.y;
-      }
+      qs[h * dim + d] = o.x * br.scale;
+      if (d + 1 < dim) qs[h * dim + d + 1] = o.y * br.scale;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < hq * 32; i += kThreads) {
-      const int h = i >> 5, jj = i & 31;
-      float s0 = 0.0f, s1 = 0.0f;
-      if (jj < nk) {
-        const float *q = qs + h * dim, *k = kt + jj * ldk;
-        int d = 0;
-        for (; d + 1 < dim; d += 2) {
-          s0 = fmaf(q[d], k[d], s0);
-          s1 = fmaf(q[d + 1], k[d + 1], s1);
+    for (int i = threadIdx.x; i < hq * dim; i += kThreads) acc[i] = 0.0f;
+    for (int i = threadIdx.x; i < hq; i += kThreads) {
+      st[i * 3] = -FLT_MAX;
+      st[i * 3 + 1] = 0.0f;
+    }
+    for (int jb = j0; jb < j1; jb += KT) {
+      const int nk = min(KT, j1 - jb);
+      __syncthreads();
+      for (int i = threadIdx.x; i < nk * P; i += kThreads) {
+        const int jj = i / P, p = i % P, d = 2 * p, j = jb + jj;
+        float u, v = 0.0f;
+        T* cr = cache + static_cast<int64_t>(j) * dim + d;
+        if (j == slot) {
+          const float* src = ph.proj + br.col_k + g * dim + d;
+          const float* bias = br.b_k + g * dim + d;
+          u = ldg_f(src) + bias[0];
+          cr[0] = from_f<T>(u);
+          if (d + 1 < dim) {
+            v = ldg_f(src + 1) + bias[1];
+            cr[1] = from_f<T>(v);
+          }
+        } else {
+          u = to_f(cr[0]);
+          if (d + 1 < dim) v = to_f(cr[1]);
         }
-        if (d < dim) s0 = fmaf(q[d], k[d], s0);
+        float2 o = make_float2(u, v);
+        if (p < br.rot_pairs) {
+          const float2 cs = br.table[static_cast<int64_t>(j) * br.rot_pairs + p];
+          o = make_float2(u * cs.x - v * cs.y, v * cs.x + u * cs.y);
+        }
+        kr[jj * ldk + d] = u;
+        kt[jj * ldk + d] = o.x;
+        if (d + 1 < dim) {
+          kr[jj * ldk + d + 1] = v;
+          kt[jj * ldk + d + 1] = o.y;
+        }
       }
-      sc[i] = jj < nk ? s0 + s1 : -FLT_MAX;
-    }
-    __syncthreads();
-    for (int h = wid; h < hq; h += kWarps) {
-      const float s = sc[h * 32 + lane];
-      const float m = st[h * 3], mn = fmaxf(m, warp_max(s));
-      const float p = lane < nk ? expf(s - mn) : 0.0f, c = expf(m - mn);
-      const float l = st[h * 3 + 1] * c + warp_sum(p);
-      __syncwarp();
-      sc[h * 32 + lane] = p;
-      if (lane == 0) {
-        st[h * 3] = mn;
-        st[h * 3 + 1] = l;
-        st[h * 3 + 2] = c;
+      __syncthreads();
+      for (int i = threadIdx.x; i < hq * 32; i += kThreads) {
+        const int h = i >> 5, jj = i & 31;
+        float s0 = 0.0f, s1 = 0.0f;
+        if (jj < nk) {
+          const float *q = qs + h * dim, *k = kt + jj * ldk;
+          int d = 0;
+          for (; d + 1 < dim; d += 2) {
+            s0 = fmaf(q[d], k[d], s0);
+            s1 = fmaf(q[d + 1], k[d + 1], s1);
+          }
+          if (d < dim) s0 = fmaf(q[d], k[d], s0);
+        }
+        sc[i] = jj < nk ? s0 + s1 : -FLT_MAX;
+      }
+      __syncthreads();
+      for (int h = wid; h < hq; h += kWarps) {
+        const float s = sc[h * 32 + lane];
+        const float m = st[h * 3], mn = fmaxf(m, warp_max(s));
+        const float p = lane < nk ? expf(s - mn) : 0.0f, c = expf(m - mn);
+        const float l = st[h * 3 + 1] * c + warp_sum(p);
+        __syncwarp();
+        sc[h * 32 + lane] = p;
+        if (lane == 0) {
+          st[h * 3] = mn;
+          st[h * 3 + 1] = l;
+          st[h * 3 + 2] = c;
+        }
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < hq * dim; i += kThreads) {
+        const int h = i / dim, d = i % dim;
+        float t = acc[i] * st[h * 3 + 2];
+        for (int jj = 0; jj < nk; ++jj) t = fmaf(sc[h * 32 + jj], kr[jj * ldk + d], t);
+        acc[i] = t;
       }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < hq * dim; i += kThreads) {
       const int h = i / dim, d = i % dim;
-      float t = acc[i] * st[h * 3 + 2];
-      for (int jj = 0; jj < nk; ++jj) t = fmaf(sc[h * 32 + jj], kr[jj * ldk + d], t);
-      acc[i] = t;
+      br.part[(static_cast<int64_t>(g * hq + h) * kAttnSplits + sp) * PS + kAttnStats + d] = acc[i];
     }
-  }
-  __syncthreads();
-  const int PS = dim + kAttnStats;
-  for (int i = threadIdx.x; i < hq * dim; i += kThreads) {
-    const int h = i / dim, d = i % dim;
-    br.part[(static_cast<int64_t>(g * hq + h) * kAttnSplits + sp) * PS + kAttnStats + d] = acc[i];
-  }
-  for (int i = threadIdx.x; i < hq; i += kThreads) {
-    float* pp = br.part + (static_cast<int64_t>(g * hq + i) * kAttnSplits + sp) * PS;
-    pp[0] = st[i * 3];
-    pp[1] = st[i * 3 + 1];
+    for (int i = threadIdx.x; i < hq; i += kThreads) {
+      float* pp = br.part + (static_cast<int64_t>(g * hq + i) * kAttnSplits + sp) * PS;
+      pp[0] = st[i * 3];
+      pp[1] = st[i * 3 + 1];
+    }
   }
   __threadfence();
   __syncthreads();
@@ -1514,7 +1663,7 @@ size_t token_smem_bytes(int stage_floats, const TokenPhase* phases, int n) {
       if (phases[i].stage == kStageList) continue;   // counted by the caller
       if (br.kind == kTokAttention) {
         const size_t hq = br.H / br.G, kt = br.dim <= 128 ? 32 : (br.dim <= 256 ? 16 : (br.dim <= 512 ? 8 : 4));
-        f = 2 * hq * br.dim + 2 * kt * (br.dim + 1) + hq * 35;
+        f = 2 * hq * br.dim + 2 * kt * (br.dim + 1) + hq * 35;   // the warp form's (hq + 1) dim + 2 kWarps (dim + 2) is less
       } else if (br.kind == kTokLightning) {
         f = 2 * br.dim + kWarps * 32;
       } else {
