@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     kv_write_rows_kernel(const float* __restrict__ qkv, float* __restrict__ kcache, float* __restrict__ vcache,
                          int T, int H, int Hk, int D, int max_seq) {
+  pdl_launch();
+  pdl_wait();
   const int64_t n = static_cast<int64_t>(T) * 2 * Hk * (D / 4);
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int RS = (H + 2 * Hk) * D;
@@ -493,8 +495,8 @@ int prompt_pass(Decoder& d, const int64_t* ids, int64_t T, cudaStream_t s) {
       DTRY(ctdk_qk_norm_rope_fwd(d.pqkv, d.pqkv, nullptr, nullptr, nullptr, nullptr, d.rope_table, 1, T, H, Hk, D,
                                  c.rms_norm_eps, s));
     }
-    kv_write_rows_kernel<<<sm_count() * 4, 256, 0, s>>>(d.pqkv, d.kcache + l * cache_layer, d.vcache + l * cache_layer,
-                                                        static_cast<int>(T), H, Hk, D, d.max_seq);
+    launch_pdl(kv_write_rows_kernel, dim3(sm_count() * 4), dim3(256), 0, s, d.pqkv, d.kcache + l * cache_layer, d.vcache + l * cache_layer,
+               static_cast<int>(T), H, Hk, D, d.max_seq);
     DTRY(check_launch("decode kv write"));
     DTRY(ctdk_attn_fwd_p(d.pqkv, d.pattn, d.plse, 1, T, H, Hk, D, prec, s));
     DTRY(ctdk_gemm(d.pattn, P + w.wo, d.pb, T, hid, H * D, H * D, H * D, hid, 0, 1, prec, CTDK_EPI_RESIDUAL, d.pa, s));

@@ -104,6 +104,8 @@ __global__ void __launch_bounds__(256) silu_bwd_kernel(const float* __restrict__
 __global__ void __launch_bounds__(256) swiglu_fwd_kernel(const float* __restrict__ gu,
                                                          float* __restrict__ act, int64_t rows,
                                                          int I4) {
+  pdl_launch();
+  pdl_wait();
   const int64_t total = rows * I4;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const float4* gu4 = reinterpret_cast<const float4*>(gu);
@@ -129,6 +131,8 @@ __global__ void __launch_bounds__(256) swiglu_bwd_kernel(const float* __restrict
                                                          const float* __restrict__ dact,
                                                          float* __restrict__ dgu, int64_t rows,
                                                          int I4) {
+  pdl_launch();
+  pdl_wait();
   const int64_t total = rows * I4;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const float4* gu4 = reinterpret_cast<const float4*>(gu);
@@ -225,8 +229,7 @@ int ctdk_swiglu_fwd(const float* gu, float* act, int64_t rows, int I, void* stre
   CTDK_REQUIRE(gu && act, "ctdk_swiglu_fwd: null pointer");
   CTDK_REQUIRE(I % 4 == 0 && aligned16(gu) && aligned16(act),
                "ctdk_swiglu_fwd: I must be a multiple of 4 and pointers 16-byte aligned");
-  swiglu_fwd_kernel<<<grid_for(rows * (I / 4), 256, 8), 256, 0,
-                      static_cast<cudaStream_t>(stream)>>>(gu, act, rows, I / 4);
+  launch_pdl(swiglu_fwd_kernel, dim3(grid_for(rows * (I / 4), 256, 8)), dim3(256), 0, static_cast<cudaStream_t>(stream), gu, act, rows, I / 4);
   return check_launch("ctdk_swiglu_fwd");
 }
 
@@ -237,8 +240,7 @@ int ctdk_swiglu_bwd(const float* gu, const float* dact, float* dgu, int64_t rows
   CTDK_REQUIRE(gu && dact && dgu, "ctdk_swiglu_bwd: null pointer");
   CTDK_REQUIRE(I % 4 == 0 && aligned16(gu) && aligned16(dact) && aligned16(dgu),
                "ctdk_swiglu_bwd: I must be a multiple of 4 and pointers 16-byte aligned");
-  swiglu_bwd_kernel<<<grid_for(rows * (I / 4), 256, 8), 256, 0,
-                      static_cast<cudaStream_t>(stream)>>>(gu, dact, dgu, rows, I / 4);
+  launch_pdl(swiglu_bwd_kernel, dim3(grid_for(rows * (I / 4), 256, 8)), dim3(256), 0, static_cast<cudaStream_t>(stream), gu, dact, dgu, rows, I / 4);
   return check_launch("ctdk_swiglu_bwd");
 }
 
