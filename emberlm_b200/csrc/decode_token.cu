@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
     ask_rows(a.P + a.lw[0].wo, r_hid, HD);
   }
 
-  // xs = v * nw for the words of an exchange (or plain values); s_red collects the sum of squares of v. False:
-  // the block leaves.
+  // xs = v * nw for the words of an exchange, or for plain values (null: zeros); s_red collects the sum of squares of
+  // v. False: the block leaves.
   auto stage_norm = [&](const Word* words, const float* plain, unsigned epoch, const float* nw) {
     float ss = 0.0f;
     auto store = [&](int i, float u, float v) {
@@ -522,7 +522,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
     };
     if (words != nullptr) take(words, hid, epoch, p, store);
     else
-      for (int i = 2 * threadIdx.x; i < hid; i += 2 * kThreads) store(i, __ldg(plain + i), __ldg(plain + i + 1));
+      for (int i = 2 * threadIdx.x; i < hid; i += 2 * kThreads)
+        store(i, plain != nullptr ? __ldg(plain + i) : 0.0f, plain != nullptr ? __ldg(plain + i + 1) : 0.0f);
     ss = warp_sum(ss);
     if (lane == 0) s_red[wid] = ss;
     return !p.left();
@@ -539,8 +540,12 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
   };
 
   for (int t = 0; t < a.n_tokens; ++t) {
-    const float* row = a.P + a.embed + tok * hid;   // layer 0 reads the embedding row in place
-    for (int i = threadIdx.x; i < r_hid.count; i += kThreads) s_res[i] = row[r_hid.first + i];
+    // layer 0 reads the embedding row in place; a given id outside the vocabulary is a row of zeros and is counted, as
+    // in embedding_fwd_kernel
+    const bool known = tok >= 0 && tok < a.V;
+    const float* row = known ? a.P + a.embed + tok * hid : nullptr;
+    if (!known && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.status[2], 1);
+    for (int i = threadIdx.x; i < r_hid.count; i += kThreads) s_res[i] = known ? row[r_hid.first + i] : 0.0f;
     const int L = pos + 1, splits = attn_splits(L, D, a.Hk), items = a.Hk * splits;
     for (int l = 0; l < a.L; ++l) {
       const TokenLayer& w = a.lw[l];

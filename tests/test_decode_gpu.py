@@ -121,3 +121,33 @@ def test_token_pass_over_key_ranges(case, context):
     for token in got[:-1]:
         z = dec.step(int(token)).cpu().numpy()
     assert np.abs(z - ref).max() <= 5e-3 * max(np.abs(ref).max(), 1.0)
+
+
+@pytest.mark.parametrize("one_launch", [True, False])
+@pytest.mark.parametrize("kw", CASES)
+def test_ids_outside_the_vocabulary(kw, one_launch, monkeypatch):
+    """Behind a prompt too such an id is an embedding row of zeros and is counted, by the token kernel as by the kernel
+    per phase. The oracle has the row of zeros behind the vocabulary; tolerance as above."""
+    import ctypes as C
+
+    from emberlm_b200 import engine as E
+    monkeypatch.setenv("CTDK_DECODE_PERSISTENT", "1" if one_launch else "0")
+    ocfg, ecfg, params = build(kw, 53)
+    V = ocfg.vocab_size
+    wider = dict(params)
+    wider["model.embed_tokens.weight"] = np.concatenate([params["model.embed_tokens.weight"], np.zeros((1, ocfg.hidden_size), F32)])
+    t = np.random.default_rng(8).integers(0, V, size=30)
+    given = t.copy()
+    given[[20, 22, 29]] = [-1, V, 1 << 40]   # inside a portion, first of one, a lone token
+    want = om.forward_logits(wider, om.LlamaConfig(**dict(kw, vocab_size=V + 1)), np.where((given < 0) | (given >= V), V, given)[None, :],
+                             acc=np.float64)[0, :, :V]
+    dec = E.Decoder(ecfg, max_seq_len=40)
+    dec.load_parameters(params)
+    counts = []
+    for lo, hi in ((0, 17), (17, 22), (22, 29), (29, 30)):
+        words = (C.c_int * 4)()
+        z = dec.extend(given[lo:hi], want=range(hi - lo)).cpu().numpy()
+        E.lib.check(E._L.ctdk_device_status(dec.stream.cuda_stream, words))
+        counts.append(words[2])
+        assert np.abs(z - want[lo:hi]).max() <= 5e-3 * max(np.abs(want).max(), 1.0), (lo, hi)
+    assert [b - a for a, b in zip(counts, counts[1:])] == [1, 1, 1]
