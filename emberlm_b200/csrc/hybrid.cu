@@ -516,6 +516,9 @@ int HybridDecoder<T>::run_rows(const int64_t* ids, int64_t n, int64_t pos, int64
   na.ids = ids;
   na.embed = at<T>(m.embed);
   na.ld_embed = m.ldw;
+  na.vocab = vocab;
+  na.status = device_status_word();
+  CTDK_REQUIRE(na.status != nullptr, "hybrid decoder: no status word");
   na.w_embed = vec(m.embed_norm);
   na.h = h;
   na.ld_h = m.ldw;

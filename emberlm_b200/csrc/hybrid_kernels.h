@@ -11,7 +11,8 @@ namespace hybrid {
 
 // Norm, residual sum, norm in one pass over a row:
 //   y   = pending sublayer output (y2 == nullptr), or (rms(y) w_y + rms(y2) w_y2) / 2
-//   x   = x + rms(y) w_post              (or, with ids: x = rms(embed[id]) w_embed)
+//   x   = x + rms(y) w_post              (or, with ids: x = rms(embed[id]) w_embed; an id outside [0, vocab) is
+//                                         a row of zeros and is counted in status[2])
 //   h   = rms(x) w_pre, in the model's type, the input of the next projection
 // rows of x / y / y2 are gather[i] when gather is given. x_out == nullptr: x is not stored.
 template <typename T>
@@ -20,7 +21,8 @@ struct NormArgs {
   float eps = 0.0f;
   const int64_t* ids = nullptr;
   const T* embed = nullptr;
-  int64_t ld_embed = 0;
+  int64_t ld_embed = 0, vocab = 0;
+  int* status = nullptr;
   const float* w_embed = nullptr;
   const float* x = nullptr;
   const int32_t* gather = nullptr;

@@ -546,6 +546,9 @@ int HybridDecoder<T>::run_parallel_rows(const int64_t* ids, int64_t n, int64_t p
   na.ids = ids;
   na.embed = at<T>(m.embed);
   na.ld_embed = m.ldw;
+  na.vocab = vocab;
+  na.status = device_status_word();
+  CTDK_REQUIRE(na.status != nullptr, "hybrid decoder: no status word");
   na.h = h;
   na.shifted = shifted;
   na.mix = mixes;

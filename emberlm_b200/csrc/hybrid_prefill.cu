@@ -50,9 +50,12 @@ __global__ void __launch_bounds__(256) norm_rows_kernel(const NormArgs<T> a, int
     const int64_t src = a.gather != nullptr ? a.gather[r] : r;
     float ss[2] = {0.0f, 0.0f};
     if (a.ids != nullptr) {
-      const T* e = a.embed + a.ids[src] * a.ld_embed;
+      const int64_t id = a.ids[src];
+      const bool known = id >= 0 && id < a.vocab;
+      const T* e = a.embed + (known ? id * a.ld_embed : 0);
+      if (!known && threadIdx.x == 0) atomicAdd(&a.status[2], 1);
       for (int i = threadIdx.x; i < W; i += 256) {
-        const float v = to_f(e[i]);
+        const float v = known ? to_f(e[i]) : 0.0f;
         ys[i] = v;
         ss[0] += v * v;
       }

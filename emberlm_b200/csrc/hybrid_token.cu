@@ -127,6 +127,9 @@ __device__ __forceinline__ void block_sum(float (&v)[N], float* red /* [N][8] */
   }
 }
 
+// A given token may lie outside the vocabulary: its embedding row is zeros, and it is counted in the status word.
+__device__ __forceinline__ bool known_id(const TokenArgs& a, int64_t tok) { return tok >= 0 && tok < a.vocab; }
+
 // xs[0, width) = the normed input of a projection; CTA 0 stores the new residual. Zero padding to a multiple of 8.
 template <typename T>
 __device__ void stage_norm(const TokenArgs& a, const TokenPhase& ph, int64_t tok, float* xs, float* red) {
@@ -135,9 +138,10 @@ __device__ void stage_norm(const TokenArgs& a, const TokenPhase& ph, int64_t tok
   float ss[2] = {0.0f, 0.0f};
   // a thread keeps to its own columns until the last barrier
   if (ph.first_token) {
-    const T* e = static_cast<const T*>(a.embed) + tok * a.ld_embed;
+    const bool known = known_id(a, tok);
+    const T* e = static_cast<const T*>(a.embed) + (known ? tok * a.ld_embed : 0);
     for (int i = threadIdx.x; i < W; i += kThreads) {
-      const float v = to_f(e[i]);
+      const float v = known ? to_f(e[i]) : 0.0f;
       xs[i] = v;
       ss[0] += v * v;
     }
@@ -732,7 +736,8 @@ __device__ __forceinline__ void stage_shift_norm(const TokenArgs& a, const Token
   const int W = a.width, gs = W / f.groups, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int g0 = wid / f.wpg, gstep = kListWarps / f.wpg, wj = wid % f.wpg, step = 32 * V * f.wpg;
   const bool active = g0 < gstep, writer = blockIdx.x == 0, shifted = f.shift != nullptr;
-  const T* e = ph.first_token ? static_cast<const T*>(a.embed) + tok * a.ld_embed : nullptr;
+  const bool known = known_id(a, tok);
+  const T* e = ph.first_token ? static_cast<const T*>(a.embed) + (known ? tok * a.ld_embed : 0) : nullptr;
   float *xs = sm, *part = sm + f.red;
   const float* prev = shifted ? f.state + ((pos + 1) & 1) * 2 * W : nullptr;
   float* next = shifted ? f.state + (pos & 1) * 2 * W : nullptr;
@@ -766,7 +771,7 @@ __device__ __forceinline__ void stage_shift_norm(const TokenArgs& a, const Token
 #pragma unroll
         for (int k = 0; k < V; ++k) {
           if (e != nullptr) {
-            x[u].v[k] *= a.embed_scale;
+            x[u].v[k] = known ? x[u].v[k] * a.embed_scale : 0.0f;
           } else {
             float r = y1[u].v[k] * sigmoid_f(z1[u].v[k] + b1[u].v[k]);
             if (f.y2 != nullptr) r += y2[u].v[k] * sigmoid_f(z2[u].v[k] + b2[u].v[k]);
@@ -1547,6 +1552,7 @@ __global__ void __launch_bounds__(LIST ? kListThreads : kThreads, LIST ? 1 : 2) 
   unsigned int epoch = 0;
   int pos = a.counters[0];
   int64_t tok = *a.cur_token;
+  if (!known_id(a, tok) && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.status[2], 1);   // later ones are the kernel's own
   unsigned long long* words = reinterpret_cast<unsigned long long*>(a.sync + 128);
   bool alive = true;
   auto fetch = [&](int i) {   // phase descriptions are read one phase ahead

@@ -11,7 +11,8 @@ namespace ctdk {
 namespace hybrid {
 
 // One pass over the rows of a portion:
-//   x  = ids ? embed[id] * scale : x + sigmoid(z1 + b1) y1 + sigmoid(z2 + b2) y2      (y2 may be null)
+//   x  = ids ? embed[id] * scale : x + sigmoid(z1 + b1) y1 + sigmoid(z2 + b2) y2      (y2 may be null; an id outside
+//        [0, vocab) is a row of zeros and is counted in status[2])
 //   h  = w * x with every group of width / groups columns divided by its root mean square
 //   m  = h + (previous row's h - h) * shift                                          (shift may be null)
 //   mix[i] = m + (previous row's m - m) * mu[i]                                      (n_mix may be 0)
@@ -25,7 +26,8 @@ struct ShiftNormArgs {
   float eps = 0.0f, scale = 1.0f;
   const int64_t* ids = nullptr;
   const T* embed = nullptr;
-  int64_t ld_embed = 0;
+  int64_t ld_embed = 0, vocab = 0;
+  int* status = nullptr;
   const float* x = nullptr;
   const float *y1 = nullptr, *y2 = nullptr, *z1 = nullptr, *z2 = nullptr, *b1 = nullptr, *b2 = nullptr;
   int64_t ldz = 0;

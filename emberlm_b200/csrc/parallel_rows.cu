@@ -56,7 +56,10 @@ __global__ void __launch_bounds__(256, 4) shift_norm_kernel(const ShiftNormArgs<
   for (int64_t r = t0 - halo > 0 ? t0 - halo : 0; r < t1; ++r) {
     const bool own = r >= t0, have = r > 0 && r > t0 - halo;   // have: the previous row is in shared memory
     const int64_t src = a.gather != nullptr ? a.gather[r] : r;
-    const T* e = a.ids != nullptr ? a.embed + a.ids[src] * a.ld_embed : nullptr;
+    const int64_t id = a.ids != nullptr ? a.ids[src] : 0;
+    const bool known = id >= 0 && id < a.vocab;
+    const T* e = a.ids != nullptr ? a.embed + (known ? id * a.ld_embed : 0) : nullptr;
+    if (!known && own && threadIdx.x == 0) atomicAdd(&a.status[2], 1);
     float* ps = part + slot * a.groups * wpg;
     slot ^= 1;
     for (int g = g0; active && g < a.groups; g += gstep) {
@@ -66,7 +69,7 @@ __global__ void __launch_bounds__(256, 4) shift_norm_kernel(const ShiftNormArgs<
         if (e != nullptr) {
           x = vload<V>(e + c);
 #pragma unroll
-          for (int k = 0; k < V; ++k) x.v[k] *= a.scale;
+          for (int k = 0; k < V; ++k) x.v[k] = known ? x.v[k] * a.scale : 0.0f;
         } else {
           x = vload<V>(a.x + src * W + c);
           const Vec<V> y = vload<V>(a.y1 + src * W + c), z = vload<V>(a.z1 + src * a.ldz + c), b = vload<V>(a.b1 + c);

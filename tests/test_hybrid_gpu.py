@@ -324,3 +324,37 @@ def test_bf16_product(M, N, K):
     want = (A[:, :K].double() @ B[:, :K].double().T).float()
     assert torch.equal(out[:, :N], want)
     assert (out[:, N:] == -7.0).all()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("family", ["sandwich", "parallel"])
+def test_ids_outside_the_vocabulary(family, dtype):
+    """They are embedding rows of zeros in the prompt pass and in the token kernel, and are counted. The oracle has the
+    row of zeros behind the vocabulary."""
+    import ctypes as C
+
+    from emberlm_b200 import engine as E
+    from oracle import detatar as od
+    from tests import detatar_cases as dc
+    if family == "sandwich":
+        cfg = hc.model(96, 64, [hc.delta(2, 1, 32, 24, 4),
+                                hc.parallel(hc.attention(2, 1, 32, 16, 32), hc.lightning(2, 24, 32), hc.mlp(96, 2.0))])
+        w, oracle = hc.weights(cfg, 1), oh
+    else:
+        cfg, w, oracle = dc.EVEN, dc.weights(dc.EVEN, 1), od
+    V = len(w["embed"])
+    t = hc.tokens(cfg, 30, 2)
+    t[[3, 20, 22, 29]] = [1 << 40, -1, V, -(1 << 40)]
+    wider = dict(w, embed=np.concatenate([w["embed"], np.zeros_like(w["embed"][:1])]))
+    want = oracle.forward(cfg, wider, np.where((t < 0) | (t >= V), V, t))
+    dec = decoder(cfg, w, dtype)
+    counts, at = [], 0
+    words = (C.c_int * 4)()
+    lib.check(E._L.ctdk_device_status(None, words))
+    counts.append(words[2])
+    for n in (20, 1, 8, 1):
+        assert hc.error(dec.extend(t[at:at + n], range(n)).cpu().numpy(), want[at:at + n]) <= LIMIT[dtype]
+        at += n
+        lib.check(E._L.ctdk_device_status(dec.stream.cuda_stream, words))
+        counts.append(words[2])
+    assert [b - a for a, b in zip(counts, counts[1:])] == [1, 1, 1, 1]
