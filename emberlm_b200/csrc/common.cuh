@@ -23,6 +23,10 @@ int check_launch(const char* what);
 int sm_count();
 int sm_budget();   // sm_count() less the SMs set aside by ctdk_reserve_sms()
 
+// Lets launches of `kernel` on the current device use up to `bytes` of dynamic shared memory. The limit belongs to the
+// kernel, not to the caller: it is only ever raised, so decoders of different sizes can share a kernel.
+cudaError_t raise_dynamic_smem(const void* kernel, size_t bytes);
+
 // Device status word shared by all kernels that contain bounded waits. It is a
 // 4-int array in global memory: [0] = first error code, [1] = where, [2..3] = detail.
 int* device_status_word();

@@ -584,8 +584,7 @@ int ctdk_decode_create(const ctdk_model_config* cfg, const float* params, void* 
     delete d;
     return fail(CTDK_EINVAL, "ctdk_decode_create: workspace too small");
   }
-  cudaError_t e = cudaFuncSetAttribute(decode_attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(attn_smem));
+  cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(decode_attn_kernel), static_cast<size_t>(attn_smem));
   if (e != cudaSuccess) {
     delete d;
     return fail(CTDK_ELAUNCH, "ctdk_decode_create: %s", cudaGetErrorString(e));

@@ -760,7 +760,7 @@ int token_grid(const TokenKernelArgs& a) {
   if (!shape || smem > 160 * 1024) return 0;
   const void* k = reinterpret_cast<const void*>(kernel_of(D));
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || coop == 0 ||
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+      raise_dynamic_smem(k, smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return 0;

@@ -558,7 +558,7 @@ int norm_rows(const NormArgs<T>& a, int64_t rows, cudaStream_t s) {
   if (rows == 0) return CTDK_OK;
   const size_t smem = static_cast<size_t>(a.width) * 8;
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(norm_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(norm_rows_kernel<T>), smem);
     if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "hybrid norm: %s", cudaGetErrorString(e));
   }
   LAUNCH("hybrid norm", norm_rows_kernel<T>, row_grid(rows), smem, a, rows);

@@ -227,7 +227,7 @@ int moe_route(const MoeArgs& a, int64_t rows, cudaStream_t s) {
   TRY_LAUNCH("moe clear", moe_clear_kernel, (1), 256, 0, a.count, 2 * a.experts);
   const size_t smem = (static_cast<size_t>(8) * (a.outputs + route_scratch(a.outputs, a.groups)) + a.experts) * 4;
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(moe_choose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(moe_choose_kernel), smem);
     if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "moe: %s", cudaGetErrorString(e));
   }
   const int64_t ctas = (rows + 7) / 8;

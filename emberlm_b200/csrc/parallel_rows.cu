@@ -219,7 +219,7 @@ int launch_shift_norm(const ShiftNormArgs<T>& a, int64_t rows, cudaStream_t s) {
   const int64_t run64 = rows >= slots / 2 ? (rows + slots - 1) / slots : 1;
   const int run = a.gather != nullptr ? 1 : (run64 > 16 ? 16 : static_cast<int>(run64));
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(shift_norm_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const cudaError_t e = raise_dynamic_smem(reinterpret_cast<const void*>(shift_norm_kernel<T, V>), smem);
     if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "shift norm: %s", cudaGetErrorString(e));
   }
   LAUNCH("shift norm", (shift_norm_kernel<T, V>), static_cast<unsigned>((rows + run - 1) / run), smem, a, rows, run, wpg);

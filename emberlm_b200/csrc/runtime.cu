@@ -78,6 +78,15 @@ int check_launch(const char* what) {
   return CTDK_OK;
 }
 
+cudaError_t raise_dynamic_smem(const void* kernel, size_t bytes) {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  cudaFuncAttributes at;
+  const cudaError_t e = cudaFuncGetAttributes(&at, kernel);
+  if (e != cudaSuccess || static_cast<size_t>(at.maxDynamicSharedSizeBytes) >= bytes) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
 int sm_count() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 148;

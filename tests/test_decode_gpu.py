@@ -151,3 +151,24 @@ def test_ids_outside_the_vocabulary(kw, one_launch, monkeypatch):
         counts.append(words[2])
         assert np.abs(z - want[lo:hi]).max() <= 5e-3 * max(np.abs(want).max(), 1.0), (lo, hi)
     assert [b - a for a, b in zip(counts, counts[1:])] == [1, 1, 1]
+
+
+@pytest.mark.parametrize("one_launch", [True, False])
+def test_decoders_of_different_sizes_take_turns(one_launch, monkeypatch):
+    """Decoders share the kernels of their head size, and with them the limit of dynamic shared memory: a small one between
+    two passes of a large one leaves the large one's limit alone."""
+    from emberlm_b200 import engine as E
+    monkeypatch.setenv("CTDK_DECODE_PERSISTENT", "1" if one_launch else "0")
+    made = []
+    for inter, max_seq in ((8192, 8192), (256, 64)):   # 32 KB of staged vector against 18, 3 KB of scores against 1
+        ocfg, ecfg, params = build(dict(CASES[0], intermediate_size=inter), 55)
+        dec = E.Decoder(ecfg, max_seq_len=max_seq)
+        dec.load_parameters(params)
+        made.append((dec, ocfg, params))
+    t = np.random.default_rng(9).integers(0, 320, size=12)
+    for dec, _, _ in made:
+        dec.extend(t[:8])
+    for n in (8, 9, 10):
+        for dec, ocfg, params in made:
+            ref = om.forward_logits(params, ocfg, t[None, :n + 1], acc=np.float64)[0, -1]
+            assert np.abs(dec.step(int(t[n])).cpu().numpy() - ref).max() <= 5e-3 * max(np.abs(ref).max(), 1.0)
