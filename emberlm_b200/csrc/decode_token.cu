@@ -330,8 +330,6 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, int
 #pragma unroll
       for (int c = 0; c < DC; ++c) cache[lane + 32 * c] = x[c];
     }
-    // the new cache rows are read by other CTAs from the next token on: ordered before what this CTA publishes later
-    if (r >= G) __threadfence();
   }
   if (p.left()) return false;
 
@@ -679,6 +677,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_kernel(const __grid_constan
     if (threadIdx.x == 0) {
 #pragma unroll
       for (int k = 1; k < kWarps; ++k) best = s_best[k] > best ? s_best[k] : best;
+      // this CTA's new cache rows, written in front of block barriers, are read by other CTAs from the next token on:
+      // the fence stands in the thread that publishes
+      __threadfence();
       put(a.best + 2 * blockIdx.x, __uint_as_float(static_cast<unsigned>(best >> 32)), e_best);
       put(a.best + 2 * blockIdx.x + 1, __uint_as_float(static_cast<unsigned>(best)), e_best);
     }
