@@ -172,3 +172,45 @@ def test_decoders_of_different_sizes_take_turns(one_launch, monkeypatch):
         for dec, ocfg, params in made:
             ref = om.forward_logits(params, ocfg, t[None, :n + 1], acc=np.float64)[0, -1]
             assert np.abs(dec.step(int(t[n])).cpu().numpy() - ref).max() <= 5e-3 * max(np.abs(ref).max(), 1.0)
+
+
+# Shares of rows that differ from CTA to CTA (576 and 1 000 over 148), a warp with several units; two passes over the heads
+# of a key, the second full and partial; rows of several loads a warp, and (20 480) parts longer than one batch of loads.
+WIDE = [
+    dict(vocab_size=1000, hidden_size=576, intermediate_size=1536, num_hidden_layers=2, num_attention_heads=9,
+         num_key_value_heads=3, head_dim=64, rms_norm_eps=1e-5, rope_theta=10000.0),
+    dict(vocab_size=1001, hidden_size=1096, intermediate_size=4104, num_hidden_layers=2, num_attention_heads=8,
+         num_key_value_heads=1, head_dim=128, rms_norm_eps=1e-6, rope_theta=1000000.0, qk_norm=True),
+    dict(vocab_size=640, hidden_size=2048, intermediate_size=8192, num_hidden_layers=2, num_attention_heads=12,
+         num_key_value_heads=2, head_dim=64, rms_norm_eps=1e-5, rope_theta=10000.0),
+    dict(vocab_size=320, hidden_size=128, intermediate_size=20480, num_hidden_layers=2, num_attention_heads=2,
+         num_key_value_heads=1, head_dim=128, rms_norm_eps=1e-5, rope_theta=10000.0),
+]
+
+
+@pytest.mark.parametrize("one_launch", [True, False])
+@pytest.mark.parametrize("case", range(len(WIDE)))
+def test_sizes_of_either_token_path(case, one_launch, monkeypatch):
+    """Greedy and chosen tokens of the token kernel and of the kernel per phase against the oracle; tolerance as above
+    (weights are drawn so that a layer keeps the size of what passes through it)."""
+    from emberlm_b200 import engine as E
+    monkeypatch.setenv("CTDK_DECODE_PERSISTENT", "1" if one_launch else "0")
+    kw = WIDE[case]
+    ocfg, ecfg = om.LlamaConfig(**kw), E.make_config(**kw)
+    params = om.init_params(ocfg, seed=61, std=0.5 * kw["hidden_size"] ** -0.5)
+    prompt = np.random.default_rng(case).integers(0, ocfg.vocab_size, size=21)
+    dec = E.Decoder(ecfg, max_seq_len=40)
+    dec.load_parameters(params)
+    if not one_launch and kw["intermediate_size"] > 12288:   # the kernel per phase stages a vector in 48 KB
+        with pytest.raises(E.lib.CtdkError):
+            dec.generate(prompt, 6)
+        return
+    got = dec.generate(prompt, 6).cpu().numpy()
+    prefix = np.concatenate([prompt, got[:-1]])
+    ref = om.forward_logits(params, ocfg, prefix[None, :], acc=np.float64)[0, -6:]
+    limit = 5e-3 * max(np.abs(ref).max(), 1.0)
+    assert np.abs(dec.last_logits().cpu().numpy() - ref[-1]).max() <= limit
+    dec.reset()
+    dec.extend(prompt)
+    for token, want in zip(got[:-1], ref[1:]):
+        assert np.abs(dec.step(int(token)).cpu().numpy() - want).max() <= limit
