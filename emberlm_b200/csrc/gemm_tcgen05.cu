@@ -783,23 +783,52 @@ int launch_cluster_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUte
   return launch_cluster<BN, true, true>(ta, tb, ta2, tb2, args, clusters, stream);
 }
 
-// Clusters of S CTAs (one per SM) that run at a time; a GPC's SMs that do not fill a cluster stay idle.
+// Clusters of S CTAs (one per SM) that run at a time, 0 when that cannot be told. A GPC's SMs that do not fill a cluster
+// stay idle, and how many these are differs from card to card: 74, 33 and 15 clusters of 2, 4 and 8 here. One tile more than
+// that is a second wave: 16 tiles on clusters of 8 took 20.3 us where 15 would take 12.5 and the plain kernel 12.1
+// (64 x 1024 x 4096).
 int clusters_of(int S) {
-  const int sms = sm_budget();
-  return S == 8 ? sms / 9 : (S == 4 ? sms / 4 - 1 : sms / S);
+  static std::mutex mu;
+  static int most[64][9] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lk(mu);
+  if (most[dev][S] == 0) {
+    auto* kern = gemm_cluster_kernel<128, false, false, false>;
+    constexpr int smem = ClusterCfg<128>::kSmemBytes;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = S;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    most[dev][S] = n;
+  }
+  return std::min(most[dev][S], sm_budget() / S);
 }
 
-// Estimated time of a product on the cluster kernel in the unit of choose_tile (a k-block of a 256-wide tile), and its
-// tile width and cluster size.
+// Estimated time of a product on the cluster kernel in microseconds, and its tile width and cluster size. Fitted to
+// dependent launches of 84 products (16 to 255 rows, 576 to 16384 columns and terms; bfloat16 the same within 15 %): a
+// k-block of a range takes 0.31 us at 64 columns and 0.36 at 128, all else 5.6 and 8.0.
 double choose_cluster(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* s_out) {
   double best = 1e300;
-  const int widths[2] = {128, 64};
+  const int widths[2] = {128, 64}, most[9] = {0, 0, clusters_of(2), 0, clusters_of(4), 0, 0, 0, clusters_of(8)};
   for (int w : widths) {
     const int64_t tiles = ((M + BM - 1) / BM) * ((N + w - 1) / w);
     for (int S = 8; S >= 2; S /= 2) {
       if (k_blocks < 2 * S) continue;   // every CTA has a range worth its share of the exchange
-      if (tiles > clusters_of(S)) continue;   // one tile a cluster: the exchange does not overlap the next tile's loop
-      const double t = static_cast<double>((k_blocks + S - 1) / S) * (w == 128 ? 0.6 : 0.45) + (w == 128 ? 6.0 : 5.0);
+      if (tiles > most[S]) continue;   // one tile a cluster: the exchange does not overlap the next tile's loop
+      const double t = static_cast<double>((k_blocks + S - 1) / S) * (w == 128 ? 0.36 : 0.31) + (w == 128 ? 8.0 : 5.6);
       if (t < best * 0.97) {
         best = t;
         *bn_out = w;
@@ -904,7 +933,8 @@ void gemm_set_kblock_limit(int k_blocks) { t_kblock_limit = k_blocks; }
 
 namespace {
 
-// Tile width, K split and one-CTA / paired-CTA kernel for an M x N product of k_blocks stage rows.
+// Tile width, K split and one-CTA / paired-CTA kernel for an M x N product of k_blocks stage rows; returns the estimate of
+// the one-CTA kernel (k-blocks of a 256-wide tile).
 double choose_tile(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* splits_out, bool* pair_out) {
   // Tile width and K split: estimated time = rounds of the persistent grid x k-blocks per
   // unit x relative cost of a k-block (a 128-wide tile does half the work of a 256-wide one
@@ -977,9 +1007,13 @@ double choose_tile(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* spl
   *bn_out = bn;
   *splits_out = splits;
   *pair_out = use_pair;
-  // splitting K over the grid needs a launch that zeroes the output, about 3 us
-  return best + (splits > 1 ? 8.0 : 0.0);
+  return best;
 }
+
+// The same estimate in microseconds, of the same measurements as choose_cluster: 0.39 us a unit of choose_tile and 5.9 us
+// (bfloat16: 4.0) for all else. A split K also needs the launch that zeroes the output, which takes part in no dependent
+// launch, and adds every range's tile at L2: 5 us and 0.2 a range in a training step (1 us between equal products).
+double plain_us(double units, int splits, bool bf16) { return 0.39 * units + (bf16 ? 4.0 : 5.9) + (splits > 1 ? 5.0 + 0.2 * splits : 0.0); }
 
 }  // namespace
 
@@ -998,13 +1032,13 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
   const int64_t k_blocks = (K + BK - 1) / BK;
   int bn, splits;
   bool use_pair;
-  const double plain = choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
+  const double units = choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
   // From 256 rows on the order of additions stays as it is: the forms with a fused epilogue, which begin there, give the
   // same bits as the product and the kernel behind it. (Weight gradients that are split over the grid were tried on
   // clusters: SmolLM2-135M on 4 x 511 positions 10.9 -> 11.4 ms, the clusters hold SMs that the main stream needs.)
   if (!use_pair && t_kblock_limit == 0 && M < 256) {
     int cbn = 0, S = 0;
-    if (choose_cluster(M, N, k_blocks, &cbn, &S) < plain) {
+    if (choose_cluster(M, N, k_blocks, &cbn, &S) < plain_us(units, splits, false)) {
       CUtensorMap ta, tb;
       int rc = a_mn ? make_map(&ta, A, M, K, lda, BK, true, false) : make_map(&ta, A, K, M, lda, BM, false, false);
       if (rc == CTDK_OK) rc = b_mn ? make_map(&tb, B, N, K, ldb, BK, true, false) : make_map(&tb, B, K, N, ldb, cbn, false, false);
@@ -1126,9 +1160,9 @@ int gemm_bf16_tcgen05(const void* A, const void* B, float* Cp, int64_t M, int64_
   const int64_t k_blocks = (K + BKH - 1) / BKH;
   int bn, splits;
   bool use_pair;
-  const double plain = choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
+  const double units = choose_tile(M, N, k_blocks, &bn, &splits, &use_pair);
   int cbn = 0, S = 0;
-  const bool cluster = !use_pair && choose_cluster(M, N, k_blocks, &cbn, &S) < plain;
+  const bool cluster = !use_pair && choose_cluster(M, N, k_blocks, &cbn, &S) < plain_us(units, splits, true);
   if (cluster) bn = cbn;
   if (!cluster && bn == 64 && splits == 1)   // one narrow column of tiles (low-rank factors): split K while SMs are idle
     while ((M + BM - 1) / BM * splits * 2 <= sm_budget() && k_blocks / (splits * 2) >= 8) splits *= 2;

@@ -12,9 +12,10 @@ def _ints(shape, seed):
 
 
 # one and several rows of tiles, ragged edges (N = 130: rows that cannot be stored in fours), the shortest K of each cluster
-# size (2, 4 and 8 CTAs: 128, 256 and 512), a K that leaves ranges of different lengths, more tiles than clusters
+# size (2, 4 and 8 CTAs: 128, 256 and 512), a K that leaves ranges of different lengths, two rows of tiles on clusters of
+# 4 and 2, more tiles than clusters (another kernel's)
 SHAPES = [(1, 576, 576), (127, 960, 576), (37, 576, 1536), (129, 130, 1000), (300, 3072, 576), (5, 64, 512), (64, 192, 256), (128, 8, 128),
-          (200, 2048, 2052)]
+          (200, 2048, 2052), (127, 1024, 3072), (255, 960, 960), (250, 2048, 1024), (130, 1024, 64)]
 
 
 @pytest.mark.parametrize("epilogue", ["store", "accumulate", "residual"])
