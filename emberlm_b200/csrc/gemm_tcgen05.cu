@@ -64,11 +64,17 @@ struct GemmArgs {
   // lead > 0: the 3xTF32 form A B + A B2 + A2 B. The first `lead` of the `splits` ranges share the first product, the
   // others the two corrections one behind the other.
   int lead = 0;
+  // The same form with two runs a unit: range `split` of the first product in one accumulator, range `split` of the
+  // corrections in the other, one add of their sum. Up to two units a tile, the order of the adds to a zeroed C does not show.
+  int two_runs = 0;
 };
-// The k-blocks of range `split`; those of the corrections count from k_blocks on.
-__device__ __forceinline__ void k_range(const GemmArgs& args, int split, int k_blocks, int& kb0, int& kb1) {
+// The k-blocks of run `run` of range `split`; those of the corrections count from k_blocks on.
+__device__ __forceinline__ void k_range(const GemmArgs& args, int split, int run, int k_blocks, int& kb0, int& kb1) {
   int first = 0, total = k_blocks, part = split, parts = args.splits;
-  if (args.lead > 0) {
+  if (run > 0) {
+    first = k_blocks;
+    total = 2 * k_blocks;
+  } else if (args.lead > 0) {
     if (split < args.lead) {
       parts = args.lead;
     } else {
@@ -169,6 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int num_tiles = m_blocks * n_blocks;
   const int k_blocks = (args.K + kElems - 1) / kElems;
   const int num_units = num_tiles * args.splits;  // unit u: tile u % num_tiles, k-range u / num_tiles
+  const int two = !BF16 && args.two_runs != 0 ? 1 : 0;   // log2 of the runs of a unit
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
@@ -176,14 +183,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x) {
+      for (int it = 0; ok; ++it) {
+        const int unit = blockIdx.x + (it >> two) * gridDim.x;
+        if (unit >= num_units) break;
         int mb, nb;
         tile_coords(unit % num_tiles, m_blocks, n_blocks, mb, nb);
         const int m0 = mb * BM, n0 = nb * TN;
         const int b_row = grouped ? n0 + args.tiles[mb] * args.n_pitch : n0;
         const int split = unit / num_tiles;
         int kb0, kb1;
-        k_range(args, split, k_blocks, kb0, kb1);
+        k_range(args, split, it & two, k_blocks, kb0, kb1);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait_bounded(&empty[s], ph ^ 1u, args.status, 1)) {
             ok = false;
@@ -225,11 +234,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      int it = 0;
-      for (int unit = blockIdx.x; unit < num_units && ok; unit += gridDim.x, ++it) {
+      for (int it = 0; ok; ++it) {
+        const int unit = blockIdx.x + (it >> two) * gridDim.x;
+        if (unit >= num_units) break;
         const int split = unit / num_tiles;
         int kb0, kb1;
-        k_range(args, split, k_blocks, kb0, kb1);
+        k_range(args, split, it & two, k_blocks, kb0, kb1);
         const int acc = it & 1;
         const uint32_t acc_ph = (static_cast<uint32_t>(it) >> 1) & 1u;
         if (!mbar_wait_bounded(&tempty[acc], acc_ph ^ 1u, args.status, 2)) {
@@ -286,9 +296,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       tile_coords(unit % num_tiles, m_blocks, n_blocks, mb, nb);
       const bool first_split = unit < num_tiles;
       const bool atomic = args.splits > 1;
-      const int acc = it & 1;
-      const uint32_t acc_ph = (static_cast<uint32_t>(it) >> 1) & 1u;
-      if (!mbar_wait_bounded(&tfull[acc], acc_ph, args.status, 5)) {
+      const int acc = two != 0 ? 0 : it & 1;
+      const uint32_t acc_ph = (static_cast<uint32_t>(it) >> (1 - two)) & 1u;
+      if (!mbar_wait_bounded(&tfull[acc], acc_ph, args.status, 5) || (two != 0 && !mbar_wait_bounded(&tfull[1], acc_ph, args.status, 5))) {
         ok = false;
         break;
       }
@@ -334,6 +344,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (col0 >= args.N) break;  // warp-uniform
         float v[32];
         tmem_ld_32x32(t_row + static_cast<uint32_t>(ch * 32), v);
+        if (!BF16 && two != 0) {
+          float w[32];
+          tmem_ld_32x32(t_row + static_cast<uint32_t>(BN + ch * 32), w);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += w[j];
+        }
         if (!row_ok) {
           // rows past M hold zero-filled garbage: nothing to store
         } else if (atomic) {
@@ -394,7 +410,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty[acc]);
+      if (lane == 0) {
+        mbar_arrive(&tempty[acc]);
+        if (two != 0) mbar_arrive(&tempty[1]);
+      }
     }
   }
 
@@ -1263,7 +1282,8 @@ int gemm_3xtf32(const float*, const float*, float*, int64_t, int64_t, int64_t, i
 
 // C = A B + A B2 + A2 B (operands split into high and low parts: the 3xTF32 product) in one launch of the cluster kernel.
 // The first product is accumulated in runs of at most `run` k-blocks. With more tiles than clusters, or a K whose runs do
-// not fit a cluster, the ranges are units of the one-CTA kernel that add their tiles at L2 (in several rounds the
+// not fit a cluster, the ranges are units of the one-CTA kernel that add their tiles at L2, in an order that shows only
+// where it did with three products (K > 1024, or K > 512 with accumulation; in several rounds the
 // cluster kernel does not overlap its exchange: 903 rows of SmolLM2-135M 38.4 -> 40.2 ms a step). Returns 1 from about two
 // rounds of tiles on: the paired-CTA kernel's large tiles, three times, are then faster.
 int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const float* B2, float* Cp, int64_t M, int64_t N, int64_t K, int64_t lda,
@@ -1292,14 +1312,28 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
         best_lead = static_cast<int>(lead);
       }
     }
-  int splits = 0;
+  int splits = 0, two_runs = 0;
   if (best_s == 0) {
     const int sms = sm_budget();
     const int64_t lead = (k_blocks + run - 1) / run;
     if (m_blocks * ((N + 127) / 128) > 2 * static_cast<int64_t>(sms) || lead > 24) return 1;
     const int wide[2] = {256, 128};
+    // Units of two runs where they are one a tile, or two and C is zeroed: the only adds whose order does not show. They
+    // give the same bits each time, as the three products one behind the other did.
+    two_runs = lead == 1 || (lead == 2 && epilogue != CTDK_EPI_ACCUMULATE) ? 1 : 0;
+    for (int w : wide) {
+      if (two_runs == 0 || (w == 256 && N <= 128)) continue;
+      const double rounds = static_cast<double>((m_blocks * ((N + w - 1) / w) * lead + sms - 1) / sms);
+      const int64_t longest = (k_blocks + lead - 1) / lead + (2 * k_blocks + lead - 1) / lead;
+      const double t = rounds * (static_cast<double>(longest) + 12.0) * (w == 256 ? 1.0 : 0.6);
+      if (t < best * 0.97) {
+        best = t;
+        best_bn = w;
+        splits = static_cast<int>(lead);
+      }
+    }
     for (int w : wide)
-      for (int64_t more = 1; more <= 2 * lead && more <= 2 * k_blocks; ++more) {
+      for (int64_t more = 1; two_runs == 0 && more <= 2 * lead && more <= 2 * k_blocks; ++more) {
         if (w == 256 && N <= 128) break;
         const double rounds = static_cast<double>((m_blocks * ((N + w - 1) / w) * (lead + more) + sms - 1) / sms);
         const int64_t longest = std::max((k_blocks + lead - 1) / lead, (2 * k_blocks + more - 1) / more);
@@ -1326,8 +1360,9 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
     GemmArgs g{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, splits, device_status_word()};
     g.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
     g.lead = best_lead;
+    g.two_runs = two_runs;
     if (g.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
-    if (epilogue != CTDK_EPI_ACCUMULATE) {
+    if (splits > 1 && epilogue != CTDK_EPI_ACCUMULATE) {
       const cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float),
                                               static_cast<size_t>(M), stream);
       if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));

@@ -79,3 +79,31 @@ def test_random_products(M, N, K):
     for p, limit in ((lib.GEMM_TF32, 1e-3), (lib.GEMM_3XTF32, 2e-6)):
         err = (ops.matmul(a, b, False, True, p).double() - want).norm() / want.norm()
         assert err < limit, (p, float(err))
+
+
+# a cluster; units of two runs on one range (K <= 512) and two, 128 and 256 wide
+@pytest.mark.parametrize("epilogue", ["store", "residual", "accumulate"])
+@pytest.mark.parametrize("M,N,K", [(127, 960, 576), (903, 576, 576), (903, 3072, 576), (1000, 1536, 1000), (600, 2000, 500), (1100, 2048, 96)])
+def test_same_bits_each_time(M, N, K, epilogue):
+    """3xTF32 products of random values. (The ranges of K > 512 that are accumulated, and those of K > 1024, are added in
+    the order of their arrival.) Against 64 bits as test_random_products."""
+    import torch
+
+    from emberlm_b200 import lib, ops
+
+    gen = torch.Generator("cuda").manual_seed(6)
+    a, b, c = (torch.randn(s, generator=gen, device="cuda") for s in ((M, K), (N, K), (M, N)))
+    if epilogue == "accumulate" and K > 512 and M > 256:
+        pytest.skip("added in the order of arrival")
+
+    def once():
+        if epilogue == "accumulate":
+            return ops.matmul(a, b, False, True, lib.GEMM_3XTF32, out=c.clone(), epilogue=lib.EPI_ACCUMULATE)
+        return ops.matmul(a, b, False, True, lib.GEMM_3XTF32, epilogue=lib.EPI_RESIDUAL if epilogue == "residual" else lib.EPI_STORE,
+                          aux=c if epilogue == "residual" else None)
+
+    first = once()
+    want = a.double() @ b.double().T + (0 if epilogue == "store" else c.double())
+    assert (first.double() - want).norm() / want.norm() < 2e-6
+    for _ in range(5):
+        assert torch.equal(once(), first)
