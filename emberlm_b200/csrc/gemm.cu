@@ -208,9 +208,7 @@ int ctdk_gemm_ws(const float* A, const float* B, float* C, int64_t M, int64_t N,
   if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "ctdk_gemm_ws: launch failed: %s", cudaGetErrorString(e));
   int rc = check_launch("ctdk_gemm_ws(split)");
   if (rc != CTDK_OK) return rc;
-  void* tok = prof_begin(CTDK_PROF_GEMM, 2.0 * static_cast<double>(M) * N * K, s);
   rc = gemm_split_tcgen05(a_hi, a_lo, b_hi, b_lo, C, M, N, K, lda, ldb, ldc, transa, transb, epilogue, aux, 16, s);
-  prof_end(tok, s);
   if (rc <= 0) return rc;
   // the leading product in accumulation runs of at most 16 k-blocks (512 deep); the two correction
   // products are 2^-11 of it and keep the usual schedule

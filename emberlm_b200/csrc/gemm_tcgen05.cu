@@ -1356,6 +1356,8 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
   if (rc == CTDK_OK) rc = map_b(&tb, B);
   if (rc == CTDK_OK) rc = map_b(&tb2, B2);
   if (rc != CTDK_OK) return rc;
+  // the work of the three products, as where they are launched one by one
+  void* const tok = prof_begin(CTDK_PROF_GEMM, 6.0 * static_cast<double>(M) * N * K, stream);
   if (splits > 0) {
     GemmArgs g{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, splits, device_status_word()};
     g.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
@@ -1367,14 +1369,18 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
                                               static_cast<size_t>(M), stream);
       if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
     }
-    return best_bn == 256 ? dispatch_major<256>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2)
-                          : dispatch_major<128>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2);
+    rc = best_bn == 256 ? dispatch_major<256>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2)
+                        : dispatch_major<128>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2);
+    prof_end(tok, stream);
+    return rc;
   }
   ClusterArgs c{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, best_s, 3, best_lead, device_status_word()};
   c.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
   if (c.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
-  return best_bn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream)
-                        : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream);
+  rc = best_bn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream)
+                      : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream);
+  prof_end(tok, stream);
+  return rc;
 }
 
 }  // namespace ctdk

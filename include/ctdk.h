@@ -40,8 +40,8 @@ int ctdk_reserve_sms(int n);
 long long ctdk_launch_count(void);
 /* Optional live timing: while enabled, every launch of a profiled class is bracketed by CUDA
  * events on its own stream. ctdk_prof_collect synchronises the device and returns (and clears)
- * the summed duration in ms, the summed algorithmic work (FLOPs for CTDK_PROF_GEMM, bytes for
- * the others) and the number of launches of class `cls`. */
+ * the summed duration in ms, the summed algorithmic work (FLOPs for CTDK_PROF_GEMM, where a 3xTF32
+ * product counts as three; bytes for the others) and the number of launches of class `cls`. */
 #define CTDK_PROF_GEMM 0
 #define CTDK_PROF_ATTN 1
 #define CTDK_PROF_ADAMW 2

@@ -75,3 +75,22 @@ def test_engine_3xtf32_matches_oracle_to_1e4(kw):
     assert abs(ls[0] / ls[1] - float(loss)) <= 1e-5 * float(loss)
     for k, g in eng.named_grads().items():
         assert relmax(g.cpu().numpy(), ref[k]) <= 1e-4, k
+
+
+@pytest.mark.parametrize("M,N,K", [(127, 960, 576), (903, 576, 576), (4096, 3072, 2048)])
+def test_recorded_work_of_a_product(M, N, K):
+    """Three TF32 products, however many launches they take: on a cluster, as units of one launch, one by one."""
+    import ctypes as C
+
+    from emberlm_b200 import lib, ops
+    a, b = torch.ones(M, K, device="cuda"), torch.ones(N, K, device="cuda")
+    ms, work, n = C.c_double(), C.c_double(), C.c_longlong()
+    collect = lambda: lib.check(lib.raw().ctdk_prof_collect(0, C.byref(ms), C.byref(work), C.byref(n)))
+    collect()
+    lib.check(lib.raw().ctdk_prof_enable(1))
+    try:
+        ops.matmul(a, b, False, True, lib.GEMM_3XTF32)
+    finally:
+        lib.check(lib.raw().ctdk_prof_enable(0))
+    collect()
+    assert work.value == 6.0 * M * N * K and n.value in (1, 3)
