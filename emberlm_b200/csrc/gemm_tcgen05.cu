@@ -506,8 +506,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   cluster_sync();   // every CTA of the cluster is there before its shared memory is written
   pdl_wait();
 
-  const int S = args.S, rank = static_cast<int>(blockIdx.x) % S, clusters = static_cast<int>(gridDim.x) / S;
-  const int m_blocks = (args.M + BM - 1) / BM, n_blocks = (args.N + BN - 1) / BN, tiles = m_blocks * n_blocks;
+  const int S = args.S, rank = static_cast<int>(blockIdx.x) % S;
+  const int m_blocks = (args.M + BM - 1) / BM, n_blocks = (args.N + BN - 1) / BN;
   const int k_blocks = (args.K + kElems - 1) / kElems;
   // this CTA's range of the sweeps' k-blocks
   int kb0, kb1;
@@ -524,122 +524,120 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
   const int cols = BN / S, quads = cols / 4;   // columns of the tile that this CTA finishes
   int s = 0;
-  uint32_t ph = 0, tile_ph = 0;
+  uint32_t ph = 0;
   bool ok = true;
-  for (int tile = static_cast<int>(blockIdx.x) / S; tile < tiles; tile += clusters, tile_ph ^= 1u) {
-    int mb, nb;
-    tile_coords(tile, m_blocks, n_blocks, mb, nb);
-    if (warp == 0) {
-      if (lane == 0) {
-        const int m0 = mb * BM, n0 = nb * BN;
-        for (int kb = kb0; kb < kb1 && ok; ++kb) {
-          if (!mbar_wait_bounded(&empty[s], ph ^ 1u, args.status, 1)) {
-            ok = false;
-            break;
-          }
-          unsigned char* a_dst = smem + s * C::kStageBytes;
-          unsigned char* b_dst = a_dst + kATileBytes;
-          mbar_expect_tx(&full[s], C::kStageBytes);
-          const int sweep = kb / k_blocks, k0 = (kb - sweep * k_blocks) * kElems;
-          const CUtensorMap* ma = sweep == 2 ? &tmA2 : &tmA;
-          const CUtensorMap* mbp = sweep == 1 ? &tmB2 : &tmB;
-          if (A_MN) {
+  int mb, nb;
+  tile_coords(static_cast<int>(blockIdx.x) / S, m_blocks, n_blocks, mb, nb);
+  if (warp == 0) {
+    if (lane == 0) {
+      const int m0 = mb * BM, n0 = nb * BN;
+      for (int kb = kb0; kb < kb1 && ok; ++kb) {
+        if (!mbar_wait_bounded(&empty[s], ph ^ 1u, args.status, 1)) {
+          ok = false;
+          break;
+        }
+        unsigned char* a_dst = smem + s * C::kStageBytes;
+        unsigned char* b_dst = a_dst + kATileBytes;
+        mbar_expect_tx(&full[s], C::kStageBytes);
+        const int sweep = kb / k_blocks, k0 = (kb - sweep * k_blocks) * kElems;
+        const CUtensorMap* ma = sweep == 2 ? &tmA2 : &tmA;
+        const CUtensorMap* mbp = sweep == 1 ? &tmB2 : &tmB;
+        if (A_MN) {
 #pragma unroll
-            for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * kChunkBytes, ma, &full[s], m0 + 32 * c, k0);
-          } else {
-            tma_load_2d(a_dst, ma, &full[s], k0, m0);
-          }
-          if (B_MN) {
+          for (int c = 0; c < BM / 32; ++c) tma_load_2d(a_dst + c * kChunkBytes, ma, &full[s], m0 + 32 * c, k0);
+        } else {
+          tma_load_2d(a_dst, ma, &full[s], k0, m0);
+        }
+        if (B_MN) {
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c) tma_load_2d(b_dst + c * kChunkBytes, mbp, &full[s], n0 + 32 * c, k0);
-          } else {
-            tma_load_2d(b_dst, mbp, &full[s], k0, n0);
-          }
-          if (++s == C::kStages) {
-            s = 0;
-            ph ^= 1u;
-          }
+          for (int c = 0; c < BN / 32; ++c) tma_load_2d(b_dst + c * kChunkBytes, mbp, &full[s], n0 + 32 * c, k0);
+        } else {
+          tma_load_2d(b_dst, mbp, &full[s], k0, n0);
+        }
+        if (++s == C::kStages) {
+          s = 0;
+          ph ^= 1u;
         }
       }
-      __syncwarp();
-    } else if (warp == 1) {
-      if (lane == 0) {
-        constexpr uint32_t idesc = make_idesc(A_MN, B_MN, BN, BF16 ? 1u : 2u);
-        for (int kb = kb0; kb < kb1 && ok; ++kb) {
-          if (!mbar_wait_bounded(&full[s], ph, args.status, 3)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes), b_addr = a_addr + kATileBytes;
-#pragma unroll
-          for (int ks = 0; ks < BK / 8; ++ks) {   // descriptors as in gemm_tf32_kernel
-            const uint64_t adesc = A_MN ? make_smem_desc(a_addr + ks * 1024, kChunkBytes, 512, kLayoutSw128Base32)
-                                        : make_smem_desc(a_addr + ks * 32, 16, 1024, kLayoutSw128);
-            const uint64_t bdesc = B_MN ? make_smem_desc(b_addr + ks * 1024, kChunkBytes, 512, kLayoutSw128Base32)
-                                        : make_smem_desc(b_addr + ks * 32, 16, 1024, kLayoutSw128);
-            if (BF16) umma_bf16(tmem_base, adesc, bdesc, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
-            else umma_tf32(tmem_base, adesc, bdesc, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
-          }
-          umma_commit(&empty[s]);
-          if (++s == C::kStages) {
-            s = 0;
-            ph ^= 1u;
-          }
-        }
-        umma_commit(tfull);   // also behind a wait that ran out: nothing of this CTA is then in flight when it goes on
-        mbar_wait_bounded(tfull, tile_ph, args.status, 4);
-      }
-      __syncwarp();
-    } else {
-      const int q = warp & 3, row = q * 32 + lane;
-      if (!mbar_wait_bounded(tfull, tile_ph, args.status, 5)) ok = false;
-      tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-#pragma unroll 1
-      for (int ch = 0; ch < BN / 32; ++ch) {
-        float v[32];
-        tmem_ld_32x32(t_row + static_cast<uint32_t>(ch * 32), v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int col = ch * 32 + 4 * j, dst = col / cols, quad = (col - dst * cols) >> 2;
-          store_remote(in_cta(smem_u32(parts + (rank * quads + quad) * C::kPitch + row), static_cast<uint32_t>(dst)), v[4 * j], v[4 * j + 1],
-                       v[4 * j + 2], v[4 * j + 3]);
-        }
-        __syncwarp();
-      }
-      tc_fence_before();
     }
     __syncwarp();
-    cluster_sync();   // all parts of this CTA's columns are there, and its tensor memory has been read
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc(A_MN, B_MN, BN, BF16 ? 1u : 2u);
+      for (int kb = kb0; kb < kb1 && ok; ++kb) {
+        if (!mbar_wait_bounded(&full[s], ph, args.status, 3)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(smem + s * C::kStageBytes), b_addr = a_addr + kATileBytes;
+#pragma unroll
+        for (int ks = 0; ks < BK / 8; ++ks) {   // descriptors as in gemm_tf32_kernel
+          const uint64_t adesc = A_MN ? make_smem_desc(a_addr + ks * 1024, kChunkBytes, 512, kLayoutSw128Base32)
+                                      : make_smem_desc(a_addr + ks * 32, 16, 1024, kLayoutSw128);
+          const uint64_t bdesc = B_MN ? make_smem_desc(b_addr + ks * 1024, kChunkBytes, 512, kLayoutSw128Base32)
+                                      : make_smem_desc(b_addr + ks * 32, 16, 1024, kLayoutSw128);
+          if (BF16) umma_bf16(tmem_base, adesc, bdesc, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
+          else umma_tf32(tmem_base, adesc, bdesc, idesc, (kb != kb0 || ks != 0) ? 1u : 0u);
+        }
+        umma_commit(&empty[s]);
+        if (++s == C::kStages) {
+          s = 0;
+          ph ^= 1u;
+        }
+      }
+      umma_commit(tfull);   // also behind a wait that ran out: nothing of this CTA is then in flight when it goes on
+      mbar_wait_bounded(tfull, 0, args.status, 4);
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, row = q * 32 + lane;
+    if (!mbar_wait_bounded(tfull, 0, args.status, 5)) ok = false;
     tc_fence_after();
-    for (int i = threadIdx.x; i < quads * BM; i += kThreads) {
-      const int quad = i % quads, row = i / quads;
-      float4 v = parts[quad * C::kPitch + row];
-      for (int r = 1; r < S; ++r) {
-        const float4 w = parts[(r * quads + quad) * C::kPitch + row];
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+#pragma unroll 1
+    for (int ch = 0; ch < BN / 32; ++ch) {
+      float v[32];
+      tmem_ld_32x32(t_row + static_cast<uint32_t>(ch * 32), v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int col = ch * 32 + 4 * j, dst = col / cols, quad = (col - dst * cols) >> 2;
+        store_remote(in_cta(smem_u32(parts + (rank * quads + quad) * C::kPitch + row), static_cast<uint32_t>(dst)), v[4 * j], v[4 * j + 1],
+                     v[4 * j + 2], v[4 * j + 3]);
+      }
+      __syncwarp();
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  // all parts of this CTA's columns are there, and its tensor memory has been read; nothing reaches another CTA's memory
+  // from here on, so each may leave
+  cluster_sync();
+  tc_fence_after();
+  for (int i = threadIdx.x; i < quads * BM; i += kThreads) {
+    const int quad = i % quads, row = i / quads;
+    float4 v = parts[quad * C::kPitch + row];
+    for (int r = 1; r < S; ++r) {
+      const float4 w = parts[(r * quads + quad) * C::kPitch + row];
+      v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
+    }
+    const int64_t grow = static_cast<int64_t>(mb) * BM + row;
+    const int col = nb * BN + rank * cols + 4 * quad;
+    if (grow >= args.M || col >= args.N) continue;
+    float* c = args.C + grow * args.ldc + col;
+    const float* x = args.epilogue == CTDK_EPI_ACCUMULATE ? c : (args.epilogue == CTDK_EPI_RESIDUAL ? args.aux + grow * args.ldc + col : nullptr);
+    if (args.vec_ok && col + 4 <= args.N) {
+      if (x != nullptr) {
+        const float4 w = *reinterpret_cast<const float4*>(x);
         v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
       }
-      const int64_t grow = static_cast<int64_t>(mb) * BM + row;
-      const int col = nb * BN + rank * cols + 4 * quad;
-      if (grow >= args.M || col >= args.N) continue;
-      float* c = args.C + grow * args.ldc + col;
-      const float* x = args.epilogue == CTDK_EPI_ACCUMULATE ? c : (args.epilogue == CTDK_EPI_RESIDUAL ? args.aux + grow * args.ldc + col : nullptr);
-      if (args.vec_ok && col + 4 <= args.N) {
-        if (x != nullptr) {
-          const float4 w = *reinterpret_cast<const float4*>(x);
-          v = make_float4(v.x + w.x, v.y + w.y, v.z + w.z, v.w + w.w);
-        }
-        *reinterpret_cast<float4*>(c) = v;
-      } else {
-        const float e[4] = {v.x, v.y, v.z, v.w};
+      *reinterpret_cast<float4*>(c) = v;
+    } else {
+      const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (col + k < args.N) c[k] = e[k] + (x != nullptr ? x[k] : 0.0f);
-      }
+      for (int k = 0; k < 4; ++k)
+        if (col + k < args.N) c[k] = e[k] + (x != nullptr ? x[k] : 0.0f);
     }
-    __syncwarp();
-    cluster_sync();   // the parts may be written again, and no CTA leaves while another still writes to it
   }
   tc_fence_before();
   __syncthreads();
@@ -767,7 +765,7 @@ int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMa
 
 template <int BN, bool A_MN, bool B_MN, bool BF16 = false>
 int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ta2, const CUtensorMap& tb2, const ClusterArgs& args,
-                   int clusters, cudaStream_t stream) {
+                   cudaStream_t stream) {
   using C = ClusterCfg<BN>;
   auto* kern = gemm_cluster_kernel<BN, A_MN, B_MN, BF16>;
   static bool attr_set[64] = {false};
@@ -780,7 +778,7 @@ int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   }
   const int tiles = ((args.M + BM - 1) / BM) * ((args.N + BN - 1) / BN);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((tiles < clusters ? tiles : clusters) * args.S);
+  cfg.gridDim = dim3(tiles * args.S);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
@@ -798,11 +796,11 @@ int launch_cluster(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
 }
 template <int BN>
 int launch_cluster_major(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& ta2, const CUtensorMap& tb2,
-                         const ClusterArgs& args, int clusters, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch_cluster<BN, false, false>(ta, tb, ta2, tb2, args, clusters, stream);
-  if (!a_mn && b_mn) return launch_cluster<BN, false, true>(ta, tb, ta2, tb2, args, clusters, stream);
-  if (a_mn && !b_mn) return launch_cluster<BN, true, false>(ta, tb, ta2, tb2, args, clusters, stream);
-  return launch_cluster<BN, true, true>(ta, tb, ta2, tb2, args, clusters, stream);
+                         const ClusterArgs& args, cudaStream_t stream) {
+  if (!a_mn && !b_mn) return launch_cluster<BN, false, false>(ta, tb, ta2, tb2, args, stream);
+  if (!a_mn && b_mn) return launch_cluster<BN, false, true>(ta, tb, ta2, tb2, args, stream);
+  if (a_mn && !b_mn) return launch_cluster<BN, true, false>(ta, tb, ta2, tb2, args, stream);
+  return launch_cluster<BN, true, true>(ta, tb, ta2, tb2, args, stream);
 }
 
 // Clusters of S CTAs (one per SM) that run at a time, 0 when that cannot be told. A GPC's SMs that do not fill a cluster
@@ -849,7 +847,7 @@ double choose_cluster(int64_t M, int64_t N, int64_t k_blocks, int* bn_out, int* 
     const int64_t tiles = ((M + BM - 1) / BM) * ((N + w - 1) / w);
     for (int S = 8; S >= 2; S /= 2) {
       if (k_blocks < 2 * S) continue;   // every CTA has a range worth its share of the exchange
-      if (tiles > most[S]) continue;   // one tile a cluster: the exchange does not overlap the next tile's loop
+      if (tiles > most[S]) continue;   // a second wave of clusters would double the time
       const double t = static_cast<double>((k_blocks + S - 1) / S) * (w == 128 ? 0.36 : 0.31) + (w == 128 ? 8.0 : 5.6);
       if (t < best * 0.97) {
         best = t;
@@ -1068,8 +1066,8 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
       ClusterArgs c{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, S, 1, 0, device_status_word()};
       c.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
       if (c.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
-      return cbn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta, tb, c, clusters_of(S), stream)
-                        : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta, tb, c, clusters_of(S), stream);
+      return cbn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta, tb, c, stream)
+                        : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta, tb, c, stream);
     }
   }
 
@@ -1202,8 +1200,8 @@ int gemm_bf16_tcgen05(const void* A, const void* B, float* Cp, int64_t M, int64_
   const int vec = (a16(Cp) && (ldc & 3) == 0) ? 1 : 0;
   if (cluster) {
     const ClusterArgs c{Cp, nullptr, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), CTDK_EPI_STORE, vec, S, 1, 0, st};
-    return bn == 128 ? launch_cluster<128, false, false, true>(ta, tb, ta, tb, c, clusters_of(S), stream)
-                     : launch_cluster<64, false, false, true>(ta, tb, ta, tb, c, clusters_of(S), stream);
+    return bn == 128 ? launch_cluster<128, false, false, true>(ta, tb, ta, tb, c, stream)
+                     : launch_cluster<64, false, false, true>(ta, tb, ta, tb, c, stream);
   }
   if (splits > 1) {
     const cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float),
@@ -1377,8 +1375,8 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
   ClusterArgs c{Cp, aux, ldc, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), epilogue, 0, best_s, 3, best_lead, device_status_word()};
   c.vec_ok = a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux)) ? 1 : 0;
   if (c.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
-  rc = best_bn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream)
-                      : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta2, tb2, c, clusters_of(best_s), stream);
+  rc = best_bn == 128 ? launch_cluster_major<128>(a_mn, b_mn, ta, tb, ta2, tb2, c, stream)
+                      : launch_cluster_major<64>(a_mn, b_mn, ta, tb, ta2, tb2, c, stream);
   prof_end(tok, stream);
   return rc;
 }

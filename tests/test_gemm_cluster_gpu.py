@@ -1,5 +1,6 @@
 """Products with few tiles: K split over the CTAs of a cluster. Small integers are exact in TF32, so a wrong tile, range
-or column exchange shows as a wrong integer; the parts are added in a fixed order, so two runs agree bit for bit."""
+or column exchange shows as a wrong integer. The parts are added in a fixed order, so runs on random values agree bit for
+bit."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -22,7 +23,7 @@ SHAPES = [(1, 576, 576), (127, 960, 576), (37, 576, 1536), (129, 130, 1000), (30
 @pytest.mark.parametrize("ta,tb", [(0, 1), (0, 0), (1, 0), (1, 1)])
 @pytest.mark.parametrize("M,N,K", SHAPES)
 @pytest.mark.parametrize("precision", ["tf32", "3xtf32"])
-def test_exact_and_repeatable(precision, M, N, K, ta, tb, epilogue):
+def test_exact(precision, M, N, K, ta, tb, epilogue):
     import torch
 
     from emberlm_b200 import lib, ops
@@ -83,10 +84,10 @@ def test_random_products(M, N, K):
 
 # a cluster; units of two runs on one range (K <= 512) and two, 128 and 256 wide
 @pytest.mark.parametrize("epilogue", ["store", "residual", "accumulate"])
-@pytest.mark.parametrize("M,N,K", [(127, 960, 576), (903, 576, 576), (903, 3072, 576), (1000, 1536, 1000), (600, 2000, 500), (1100, 2048, 96)])
+@pytest.mark.parametrize("M,N,K", [(127, 960, 576), (200, 960, 960), (903, 576, 576), (903, 3072, 576), (1000, 1536, 1000), (600, 2000, 500), (1100, 2048, 96)])
 def test_same_bits_each_time(M, N, K, epilogue):
-    """3xTF32 products of random values. (The ranges of K > 512 that are accumulated, and those of K > 1024, are added in
-    the order of their arrival.) Against 64 bits as test_random_products."""
+    """3xTF32 products of random values, and TF32 ones on a cluster. (Off clusters the ranges of K > 512 that are
+    accumulated, and those of K > 1024, are added in the order of their arrival.) Against 64 bits as test_random_products."""
     import torch
 
     from emberlm_b200 import lib, ops
@@ -96,14 +97,17 @@ def test_same_bits_each_time(M, N, K, epilogue):
     if epilogue == "accumulate" and K > 512 and M > 256:
         pytest.skip("added in the order of arrival")
 
-    def once():
+    def once(p):
         if epilogue == "accumulate":
-            return ops.matmul(a, b, False, True, lib.GEMM_3XTF32, out=c.clone(), epilogue=lib.EPI_ACCUMULATE)
-        return ops.matmul(a, b, False, True, lib.GEMM_3XTF32, epilogue=lib.EPI_RESIDUAL if epilogue == "residual" else lib.EPI_STORE,
+            return ops.matmul(a, b, False, True, p, out=c.clone(), epilogue=lib.EPI_ACCUMULATE)
+        return ops.matmul(a, b, False, True, p, epilogue=lib.EPI_RESIDUAL if epilogue == "residual" else lib.EPI_STORE,
                           aux=c if epilogue == "residual" else None)
 
-    first = once()
     want = a.double() @ b.double().T + (0 if epilogue == "store" else c.double())
-    assert (first.double() - want).norm() / want.norm() < 2e-6
-    for _ in range(5):
-        assert torch.equal(once(), first)
+    for p, limit in ((lib.GEMM_3XTF32, 2e-6), (lib.GEMM_TF32, 1e-3)):
+        if p == lib.GEMM_TF32 and M >= 256:
+            continue
+        first = once(p)
+        assert (first.double() - want).norm() / want.norm() < limit
+        for _ in range(5):
+            assert torch.equal(once(p), first)
