@@ -64,7 +64,9 @@ def test_two_steps_match_the_engine_then_resume(tmp_path):
     eng.loss_sums.zero_()
     eng.forward_loss(ids[:3], tgt[:3], m[:3])
     ls = eng.loss_sums.tolist()
-    assert abs(val[0]["loss"] - ls[0] / ls[1]) <= 1e-5 * abs(ls[0] / ls[1])
+    # the order of the split-K adds differs between two runs, and AdamW's sign-like first steps carry it into the weights
+    # (up to 2 * lr per step where the gradient is noise): 1e-4, as for the third step below; 1.25e-5 seen in 20 runs
+    assert abs(val[0]["loss"] - ls[0] / ls[1]) <= 1e-4 * abs(ls[0] / ls[1])
 
     final = safetensors_io.load_safetensors(run_dir / "final.safetensors")
     for n, v in eng.named_parameters().items():
