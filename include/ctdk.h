@@ -525,8 +525,9 @@ int ctdk_sample(const float* logits, int64_t B, int64_t V, float temperature, in
  * ctdk_decode_workspace_bytes(cfg, max_seq) bytes holding the K/V cache [layer][kv head][max_seq][D].
  *   prefill : runs the prompt (ids int64 [T], 1 <= T < max_seq) and fills the cache;
  *   greedy  : appends n_new tokens to out_tokens (device int64), continuing where the last call
- *             stopped; token ids stay on the device, one CUDA graph launch per token when `stream`
- *             is not the legacy default stream;
+ *             stopped; token ids stay on the device, one cooperative launch for all of them. A model
+ *             that the token kernel does not take runs one CUDA graph launch per token, or kernel by
+ *             kernel when `stream` is the legacy default stream;
  *   step    : feeds ONE token chosen by the caller (a sampler, a forced token) at the next
  *             position and leaves the logits of that position behind; not to be mixed with
  *             greedy after the same prefill;
@@ -535,7 +536,8 @@ int ctdk_sample(const float* logits, int64_t B, int64_t V, float temperature, in
  *             position 0), on the cache and state that earlier calls left, wherever the portion was
  *             cut. The logits of its rows want[0, n_want) (host int32) go to want_logits
  *             [n_want, vocab] (device); n_want < 0 leaves those of the last row behind for
- *             greedy / step. Not after greedy;
+ *             greedy / step. An id outside the vocabulary is a row of zeros, counted in the device
+ *             status word. Not after greedy;
  *   reset   : an empty sequence again; what it held in the cache or state is given back.
  * ------------------------------------------------------------------------------------ */
 int64_t ctdk_decode_workspace_bytes(const ctdk_model_config* cfg, int64_t max_seq);
