@@ -492,7 +492,7 @@ def run_decode(args) -> dict:
                        "l2": "weights (2.4 GB) larger than L2"},
             "e2e": {"value": new_tokens * args.steps / e2e_s, "unit": "tokens/s", "h2d_bytes_per_step": prompt_len * 8,
                     "d2h_bytes_per_step": new_tokens * 8},
-            "roofline": {"kernel": "gemv_kernel (all weights streamed once per token)", "bound": "hbm",
+            "roofline": {"kernel": "token_kernel (all weights streamed once per token)", "bound": "hbm",
                          "achieved": bytes_per_token / (per_tok_ms / 1e3) / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": bytes_per_token / (per_tok_ms / 1e3) / 1e9 / peaks["hbm_gbs"],
                          "note": "whole-token figure incl. prefill share, attention and launch gaps", "traffic": None},
