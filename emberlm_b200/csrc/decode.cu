@@ -1,5 +1,6 @@
-// KV-cache greedy decoding (batch 1): prefill with the training-path kernels, then one token per
-// step with HBM-bound kernels, the whole step captured once in a CUDA graph and replayed.
+// KV-cache greedy decoding (batch 1): prefill with the training-path kernels, then the token kernel of
+// decode_token.cu. Models that it does not take run one token per step with the HBM-bound kernels below,
+// the whole step captured once in a CUDA graph and replayed.
 //
 // Replaces the inference path of the reference: Model::forward with a cache
 // (emberlm include/ctd/nn/model.h:155-167), Attention::forward (include/ctd/nn/attention.h:43-97),
