@@ -49,6 +49,16 @@ int encode_tensor_map(CUtensorMap* map, const float* base, int rank, const uint6
 int encode_tensor_map_bf16(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
                            const uint32_t* box);
 
+// Operands of a 3xTF32 product and their high and low parts (na and nb floats, multiples of four, 16-byte aligned).
+struct SplitOperands {
+  const float *a, *b;
+  float *a_hi, *a_lo, *b_hi, *b_lo;
+  int64_t na, nb;
+};
+// Splits both, and zeroes C[M, N] (null: nothing) in the same launch.
+int split_operands(const SplitOperands& o, float* C, int64_t M, int64_t N, int64_t ldc, cudaStream_t s);
+int zero_rows(float* C, int64_t M, int64_t N, int64_t ldc, cudaStream_t s);
+
 inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
 
 #define CTDK_REQUIRE(cond, ...)                                   \

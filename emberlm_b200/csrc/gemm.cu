@@ -11,8 +11,8 @@ int gemm_tcgen05(const float* A, const float* B, float* C, int64_t M, int64_t N,
 void gemm_set_kblock_limit(int k_blocks);
 int gemm_bf16_tcgen05(const void* A, const void* B, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
                       int64_t ldc, cudaStream_t stream);
-int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const float* B2, float* C, int64_t M, int64_t N, int64_t K, int64_t lda,
-                       int64_t ldb, int64_t ldc, int transa, int transb, int epilogue, const float* aux, int run, cudaStream_t stream);
+int gemm_split_tcgen05(const SplitOperands& ops, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int transa,
+                       int transb, int epilogue, const float* aux, int run, cudaStream_t stream);
 int gemm_3xtf32(const float* A, const float* B, float* C, int64_t M, int64_t N, int64_t K,
                 int64_t lda, int64_t ldb, int64_t ldc, int transa, int transb, int epilogue,
                 const float* aux, cudaStream_t stream);
@@ -77,9 +77,32 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// hi = x rounded to TF32 (10-bit mantissa, round to nearest), lo = x - hi (exact in fp32), for two arrays in one launch.
-__global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, float* __restrict__ x_hi, float* __restrict__ x_lo, int64_t nx4,
-                                                         const float* __restrict__ y, float* __restrict__ y_hi, float* __restrict__ y_lo, int64_t ny4) {
+// C[0 .. M, 0 .. N) = 0, a block per row.
+__device__ __forceinline__ void zero_block_rows(float* C, int64_t M, int64_t N, int64_t ldc) {
+  const bool vec = ((reinterpret_cast<uintptr_t>(C) & 15u) | (ldc & 3) | (N & 3)) == 0;
+  for (int64_t r = blockIdx.x; r < M; r += gridDim.x) {
+    float* row = C + r * ldc;
+    if (vec) {
+      for (int64_t c = threadIdx.x; c < N / 4; c += blockDim.x) reinterpret_cast<float4*>(row)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+      for (int64_t c = threadIdx.x; c < N; c += blockDim.x) row[c] = 0.0f;
+    }
+  }
+}
+
+// The zeroes in front of a product whose ranges of K add to C, a few megabytes: launch and hand-over bound it. A dependent
+// launch overlaps the kernel before it and lets the product's set-up overlap it, which a memset node does neither of
+// (SmolLM2-135M, 4 x 511 tokens, 214 of them a step: 10.93 -> 10.76 ms).
+__global__ void __launch_bounds__(256) zero_rows_kernel(float* C, int64_t M, int64_t N, int64_t ldc) {
+  pdl_launch();
+  pdl_wait();
+  zero_block_rows(C, M, N, ldc);
+}
+
+// hi = x rounded to TF32 (10-bit mantissa, round to nearest), lo = x - hi (exact in fp32), for two arrays in one launch;
+// then C = 0 (C != null) for the product behind it, whose own launch then follows directly (with a memset between the two,
+// 335 a step, SmolLM2-135M on 3 x 301 tokens took 20.40 ms, now 19.36).
+__global__ void __launch_bounds__(256) split_tf32_kernel(const SplitOperands o, int64_t nx4, int64_t ny4, float* C, int64_t M, int64_t N, int64_t ldc) {
   pdl_launch();
   pdl_wait();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -92,15 +115,16 @@ __global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict
   for (int64_t k = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < nx4 + ny4; k += stride) {
     const bool first = k < nx4;
     const int64_t i = first ? k : k - nx4;
-    const float4 v = reinterpret_cast<const float4*>(first ? x : y)[i];
+    const float4 v = reinterpret_cast<const float4*>(first ? o.a : o.b)[i];
     float4 h, l;
     sp(v.x, h.x, l.x);
     sp(v.y, h.y, l.y);
     sp(v.z, h.z, l.z);
     sp(v.w, h.w, l.w);
-    reinterpret_cast<float4*>(first ? x_hi : y_hi)[i] = h;
-    reinterpret_cast<float4*>(first ? x_lo : y_lo)[i] = l;
+    reinterpret_cast<float4*>(first ? o.a_hi : o.b_hi)[i] = h;
+    reinterpret_cast<float4*>(first ? o.a_lo : o.b_lo)[i] = l;
   }
+  if (C != nullptr) zero_block_rows(C, M, N, ldc);
 }
 
 __global__ void fill_rows_kernel(float* C, const float* aux, int64_t M, int64_t N, int64_t ldc,
@@ -113,6 +137,21 @@ __global__ void fill_rows_kernel(float* C, const float* aux, int64_t M, int64_t 
 }
 
 }  // namespace
+
+int zero_rows(float* C, int64_t M, int64_t N, int64_t ldc, cudaStream_t s) {
+  const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
+  const cudaError_t e = launch_pdl(zero_rows_kernel, dim3(static_cast<unsigned>(M < cap ? M : cap)), dim3(256), 0, s, C, M, N, ldc);
+  if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: launch failed: %s", cudaGetErrorString(e));
+  return check_launch("gemm(zero)");
+}
+
+int split_operands(const SplitOperands& o, float* C, int64_t M, int64_t N, int64_t ldc, cudaStream_t s) {
+  const int64_t cap = static_cast<int64_t>(sm_count()) * 8, want = (o.na + o.nb) / 4 / 256 + 1;
+  const cudaError_t e = launch_pdl(split_tf32_kernel, dim3(static_cast<unsigned>(want < cap ? want : cap)), dim3(256), 0, s, o, o.na / 4, o.nb / 4, C, M, N, ldc);
+  if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "ctdk_gemm_ws: launch failed: %s", cudaGetErrorString(e));
+  return check_launch("ctdk_gemm_ws(split)");
+}
+
 }  // namespace ctdk
 
 using namespace ctdk;
@@ -202,14 +241,11 @@ int ctdk_gemm_ws(const float* A, const float* B, float* C, int64_t M, int64_t N,
   float* a_lo = a_hi + up(na);
   float* b_hi = a_lo + up(na);
   float* b_lo = b_hi + up(nb);
-  const int cap = sm_count() * 8;
-  auto blocks = [&](int64_t n4) { return static_cast<int>(n4 / 256 + 1 < cap ? n4 / 256 + 1 : cap); };
-  const cudaError_t e = launch_pdl(split_tf32_kernel, dim3(blocks((na + nb) / 4)), dim3(256), 0, s, A, a_hi, a_lo, na / 4, B, b_hi, b_lo, nb / 4);
-  if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "ctdk_gemm_ws: launch failed: %s", cudaGetErrorString(e));
-  int rc = check_launch("ctdk_gemm_ws(split)");
-  if (rc != CTDK_OK) return rc;
-  rc = gemm_split_tcgen05(a_hi, a_lo, b_hi, b_lo, C, M, N, K, lda, ldb, ldc, transa, transb, epilogue, aux, 16, s);
+  const SplitOperands ops{A, B, a_hi, a_lo, b_hi, b_lo, na, nb};
+  int rc = gemm_split_tcgen05(ops, C, M, N, K, lda, ldb, ldc, transa, transb, epilogue, aux, 16, s);
   if (rc <= 0) return rc;
+  rc = split_operands(ops, nullptr, 0, 0, 0, s);
+  if (rc != CTDK_OK) return rc;
   // the leading product in accumulation runs of at most 16 k-blocks (512 deep); the two correction
   // products are 2^-11 of it and keep the usual schedule
   gemm_set_kblock_limit(16);

@@ -1104,9 +1104,8 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
     if (st == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
     const int vec = (a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux))) ? 1 : 0;
     if (splits > 1 && epilogue != CTDK_EPI_ACCUMULATE) {
-      cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0,
-                                        static_cast<size_t>(N) * sizeof(float), static_cast<size_t>(M), stream);
-      if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
+      rc = zero_rows(Cp, M, N, ldc, stream);
+      if (rc != CTDK_OK) return rc;
     }
     // Output through TMA (coalesced, off the load/store pipe): plain store, or an fp32 add at L2
     // for accumulation and for split-K partial tiles. The residual epilogue reads a second
@@ -1135,10 +1134,8 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
   args.status = device_status_word();
   if (args.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
   if (splits > 1 && epilogue != CTDK_EPI_ACCUMULATE) {
-    cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0,
-                                      static_cast<size_t>(N) * sizeof(float),
-                                      static_cast<size_t>(M), stream);
-    if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
+    rc = zero_rows(Cp, M, N, ldc, stream);
+    if (rc != CTDK_OK) return rc;
   }
 
   switch (bn) {
@@ -1204,9 +1201,8 @@ int gemm_bf16_tcgen05(const void* A, const void* B, float* Cp, int64_t M, int64_
                      : launch_cluster<64, false, false, true>(ta, tb, ta, tb, c, stream);
   }
   if (splits > 1) {
-    const cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float),
-                                            static_cast<size_t>(M), stream);
-    if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
+    rc = zero_rows(Cp, M, N, ldc, stream);
+    if (rc != CTDK_OK) return rc;
   }
   if (use_pair) {
     int tma_out = 0;
@@ -1284,8 +1280,10 @@ int gemm_3xtf32(const float*, const float*, float*, int64_t, int64_t, int64_t, i
 // where it did with three products (K > 1024, or K > 512 with accumulation; in several rounds the
 // cluster kernel does not overlap its exchange: 903 rows of SmolLM2-135M 38.4 -> 40.2 ms a step). Returns 1 from about two
 // rounds of tiles on: the paired-CTA kernel's large tiles, three times, are then faster.
-int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const float* B2, float* Cp, int64_t M, int64_t N, int64_t K, int64_t lda,
-                       int64_t ldb, int64_t ldc, int transa, int transb, int epilogue, const float* aux, int run, cudaStream_t stream) {
+// The operands are split here, in the launch that also zeroes C where the product adds to it. Nothing is enqueued when it returns 1.
+int gemm_split_tcgen05(const SplitOperands& ops, float* Cp, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int transa,
+                       int transb, int epilogue, const float* aux, int run, cudaStream_t stream) {
+  const float *A = ops.a_hi, *A2 = ops.a_lo, *B = ops.b_hi, *B2 = ops.b_lo;
   auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   if (!a16(A) || !a16(B) || !a16(A2) || !a16(B2) || (lda & 3) || (ldb & 3)) return 1;
   if (M < 1 || N < 8 || K < 1 || M > INT32_MAX || N > INT32_MAX || K > INT32_MAX / 4) return 1;
@@ -1353,6 +1351,7 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
   if (rc == CTDK_OK) rc = map_a(&ta2, A2);
   if (rc == CTDK_OK) rc = map_b(&tb, B);
   if (rc == CTDK_OK) rc = map_b(&tb2, B2);
+  if (rc == CTDK_OK) rc = split_operands(ops, splits > 1 && epilogue != CTDK_EPI_ACCUMULATE ? Cp : nullptr, M, N, ldc, stream);
   if (rc != CTDK_OK) return rc;
   // the work of the three products, as where they are launched one by one
   void* const tok = prof_begin(CTDK_PROF_GEMM, 6.0 * static_cast<double>(M) * N * K, stream);
@@ -1362,11 +1361,6 @@ int gemm_split_tcgen05(const float* A, const float* A2, const float* B, const fl
     g.lead = best_lead;
     g.two_runs = two_runs;
     if (g.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
-    if (splits > 1 && epilogue != CTDK_EPI_ACCUMULATE) {
-      const cudaError_t e = cudaMemset2DAsync(Cp, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float),
-                                              static_cast<size_t>(M), stream);
-      if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
-    }
     rc = best_bn == 256 ? dispatch_major<256>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2)
                         : dispatch_major<128>(a_mn, b_mn, ta, tb, g, stream, &ta2, &tb2);
     prof_end(tok, stream);
