@@ -155,6 +155,15 @@ __device__ __forceinline__ bool mbar_wait_bounded_w(uint64_t* bar, uint32_t pari
   return __all_sync(0xffffffffu, ok);
 }
 
+// Contiguous bytes into this CTA's shared memory (both 16-byte aligned, a multiple of 16 bytes), counted on `bar`; policy:
+// of createpolicy.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+                   smem_u32(smem_dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+               : "memory");
+}
+
 // ---- TMA (no multicast anywhere: every load targets this CTA's shared memory) ----
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -2,7 +2,7 @@
 // more tokens through all layers.
 #pragma once
 
-#include "decode_core.h"
+#include "token_ring.cuh"
 
 namespace ctdk {
 
@@ -22,14 +22,15 @@ struct TokenKernelArgs {
   const float* P;
   TokenLayer lw[kTokenMaxLayers];
   int64_t embed, norm;
-  int L, hid, I, D, H, Hk, V, QKVN, max_seq;
+  int L, hid, I, D, H, Hk, group, V, QKVN, max_seq;   // group: H / Hk
   int qk_norm;
   float eps, scale;
   const float2* table;      // [max_seq][D/2] (cos, sin)
   float *kcache, *vcache;   // [L][Hk][max_seq][D]
   float* logits;
   Word *x, *hm, *qkv, *part, *attn, *act, *best;
-  int s_qkv, s_o, s_gu, s_d;   // log2 of the warps that share a weight row, per product
+  RingRows product[5];         // QKV, O, gate|up, down, head
+  int vector_floats, stage_floats, residual_floats, stages, stage_bytes;   // shared memory: a place of the vector (0: there is one only), ...
   int64_t* cur_token;
   int* counters;
   unsigned int* sync;          // [2]: abort flag

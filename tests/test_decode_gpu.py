@@ -214,3 +214,22 @@ def test_sizes_of_either_token_path(case, one_launch, monkeypatch):
     dec.extend(prompt)
     for token, want in zip(got[:-1], ref[1:]):
         assert np.abs(dec.step(int(token)).cpu().numpy() - want).max() <= limit
+
+
+@pytest.mark.parametrize("case, context, inter", [(0, 9, 256), (1, 12, 256), (0, 30, 256), (1, 21, 26048), (0, 33, 13056)])
+def test_token_pass_over_few_keys_and_long_rows(case, context, inter):
+    """Tokens on both sides of the first cut of the keys into ranges (16 keys), and rows that pass through the weight ring in
+    many pieces with one place for the vector (26 048 floats) and with two; tolerance as above."""
+    from emberlm_b200 import engine as E
+    ocfg, ecfg, params = build(dict(CASES[case], intermediate_size=inter), 63)
+    prompt = np.random.default_rng(context).integers(0, ocfg.vocab_size, size=context)
+    dec = E.Decoder(ecfg, max_seq_len=context + 12)
+    dec.load_parameters(params)
+    got = dec.generate(prompt, 10).cpu().numpy()
+    ref = om.forward_logits(params, ocfg, np.concatenate([prompt, got[:-1]])[None, :], acc=np.float64)[0, -10:]
+    limit = 5e-3 * max(np.abs(ref).max(), 1.0)
+    assert np.abs(dec.last_logits().cpu().numpy() - ref[-1]).max() <= limit
+    dec.reset()
+    dec.extend(prompt)
+    for token, want in zip(got[:-1], ref[1:]):
+        assert np.abs(dec.step(int(token)).cpu().numpy() - want).max() <= limit
