@@ -1223,6 +1223,41 @@ int gemm_bf16_tcgen05(const void* A, const void* B, float* Cp, int64_t M, int64_
   }
 }
 
+int gemm_tcgen05_2cta_clamped_glu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tact, int M, int N, int K, float limit, int* status,
+                                  cudaStream_t stream);
+
+// act[M, N] (bfloat16) = clamped GLU of the N gate and N up rows of W against A's rows, where the plain product [M, 2N] would
+// take the paired-CTA kernel in whole ranges of K and a tile's 128 gate columns have their up columns; returns 1 elsewhere (the
+// narrower tiles that fewer rows take have no such epilogue).
+int gemm_bf16_clamped_glu(const void* A, const void* W, __nv_bfloat16* act, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ld_act,
+                          float limit, cudaStream_t stream) {
+  auto a16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (!a16(A) || !a16(W) || !a16(act) || (lda & 7) || (ldw & 7) || (ld_act & 7) || N % 128 != 0 || M < 1 || M > INT32_MAX || 2 * N > INT32_MAX || K < 1 ||
+      K > INT32_MAX)
+    return 1;
+  int bn, splits;
+  bool use_pair;
+  choose_tile(M, 2 * N, (K + BKH - 1) / BKH, &bn, &splits, &use_pair);
+  if (!use_pair || splits != 1) return 1;
+  auto map = [](CUtensorMap* m, const void* base, int64_t inner, int64_t outer, int64_t ld, int rows) {
+    const uint64_t dims[2] = {static_cast<uint64_t>(inner), static_cast<uint64_t>(outer)}, strides[1] = {static_cast<uint64_t>(ld) * 2};
+    const uint32_t box[2] = {64u, static_cast<uint32_t>(rows)};
+    return encode_tensor_map_bf16(m, base, 2, dims, strides, box);
+  };
+  static_assert(BKH == 64, "boxes of 64 columns");
+  CUtensorMap ta, tb, tact;
+  int rc = map(&ta, A, K, M, lda, BM);
+  if (rc == CTDK_OK) rc = map(&tb, W, K, 2 * N, ldw, 128);
+  if (rc == CTDK_OK) rc = map(&tact, act, N, M, ld_act, 32);
+  if (rc != CTDK_OK) return rc;
+  int* st = device_status_word();
+  if (st == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
+  void* const tok = prof_begin(CTDK_PROF_GEMM, 4.0 * static_cast<double>(M) * N * K, stream);
+  rc = gemm_tcgen05_2cta_clamped_glu(ta, tb, tact, static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), limit, st, stream);
+  prof_end(tok, stream);
+  return rc;
+}
+
 namespace {
 
 template <int OUT>

@@ -12,6 +12,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "hybrid_kernels.h"
 
 namespace ctdk {
 namespace {
@@ -48,6 +49,7 @@ struct Gemm2Args {
                   //    output act = silu(gate) * up [M, N]: each tile holds 128 gate and the matching 128 up columns
                   // 2: the product is d(act) [M, N]; the epilogue reads gate|up [M, 2N] through map C and
                   //    writes d(gate)|d(up) [M, 2N] through map D (SwiGLU backward), d(act) is never stored
+                  // 3: as 1 with bfloat16 operands and the clamped GLU, act [M, N] bfloat16 through map D, gate|up is never stored
   int narrow;     // 1: the plain epilogue (store / add of the bare accumulator) is run by the first warp of each lane
                   //    quarter through both staging boxes of its pair, which measured ~1 % faster than eight warps with
                   //    one box each; the epilogues that compute (SwiGLU, +residual) use all eight warps
@@ -55,6 +57,7 @@ struct Gemm2Args {
                   // epilogue also writes delta[(b * dl_H + h) * dl_T + t] = sum over the head's columns of C * O, the row
                   // term of the softmax backward (row = b * dl_T + t); needs swiglu == 0, splits == 1, a plain store
   int dl_T, dl_H, dl_D;
+  float limit;    // of the clamped GLU
   int stages;     // operand ring depth: 6, or 5 when the epilogue needs 64 KB of staging (swiglu == 2)
   int* status;
 };
@@ -187,7 +190,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   const int m_blocks = (args.M + 2 * BM2 - 1) / (2 * BM2);
-  const int n_blocks = args.swiglu == 1 ? args.N / (BN2 / 2) : (args.N + BN2 - 1) / BN2;
+  const int n_blocks = (args.swiglu & 1) != 0 ? args.N / (BN2 / 2) : (args.N + BN2 - 1) / BN2;
   const int num_tiles = m_blocks * n_blocks;
   static_assert(!BF16 || (!A_MN && !B_MN), "bfloat16 operands are K-major");
   constexpr int kElems = BF16 ? BK2H : BK2;   // values of a stage row
@@ -234,7 +237,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
         const int m0 = mb * 2 * BM2 + static_cast<int>(rank) * BM2;
         // B rows of this CTA: its half of the 256 columns, or (fused SwiGLU) 128 gate rows in the
         // even CTA and the matching 128 up rows, N rows further on, in the odd one
-        const int n0 = args.swiglu == 1 ? nb * (BN2 / 2) + static_cast<int>(rank) * args.N
+        const int n0 = (args.swiglu & 1) != 0 ? nb * (BN2 / 2) + static_cast<int>(rank) * args.N
                                    : nb * BN2 + static_cast<int>(rank) * (BN2 / 2);
         const int split = unit / num_tiles;
         const int kb0 = static_cast<int>(static_cast<int64_t>(split) * k_blocks / args.splits);
@@ -470,6 +473,39 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads2, 1)
           fence_async_smem();   // the reads of O's box come before the next fetch into it
           __syncwarp();
         }
+      } else if (BF16 && args.swiglu == 3) {
+        // as below; the warp's 64 columns of act leave as one box of 128-byte rows. Gate and up of 4096 x 3072 in fp32 were
+        // 100 MB written here and read by a kernel of their own: a prefill of 4096 tokens (width 1024, 28 layers) 12.3 -> 11.7 ms,
+        // 1000 tokens of width 2048 and 6144 in the GLU 8.03 -> 7.78.
+        const int r0 = mb * 2 * BM2 + static_cast<int>(rank) * BM2 + q * 32;
+        unsigned char* buf = epi_stage + ew * kEpiBuf;
+        if (lane == 0) bulk_wait_read<0>();   // the box sent before has left
+        __syncwarp();
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          const int ch = half * 2 + h;
+          float g[32], u[32];
+          tmem_ld_32x32(t_row + static_cast<uint32_t>(ch * 32), g);
+          tmem_ld_32x32(t_row + static_cast<uint32_t>(BN2 / 2 + ch * 32), u);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int i = 8 * c + 2 * k;
+              const __nv_bfloat162 p = __floats2bfloat162_rn(hybrid::clamped_glu_f(g[i], u[i], args.limit), hybrid::clamped_glu_f(g[i + 1], u[i + 1], args.limit));
+              w[k] = *reinterpret_cast<const uint32_t*>(&p);
+            }
+            *reinterpret_cast<uint4*>(buf + lane * 128 + (((4 * h + c) ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (r0 < args.M) tma_store_2d(&tmD, buf, nb * (BN2 / 2) + half * 64, r0);
+          bulk_commit();
+          bulk_wait_read<0>();
+        }
       } else if (args.swiglu) {
         // columns 0..127 of the accumulator are gate, 128..255 the matching up columns: three boxes
         // per 32-column chunk (gate and up into the packed buffer, silu(gate)*up into the second
@@ -657,7 +693,7 @@ int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
   auto* kern = gemm_tf32_2cta_kernel<A_MN, B_MN, BF16>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem2);
   if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "gemm(2cta): shared memory opt-in failed: %s", cudaGetErrorString(e));
-  const int tiles = ((args.M + 255) / 256) * (args.swiglu == 1 ? args.N / (BN2 / 2) : (args.N + BN2 - 1) / BN2) * args.splits;
+  const int tiles = ((args.M + 255) / 256) * ((args.swiglu & 1) != 0 ? args.N / (BN2 / 2) : (args.N + BN2 - 1) / BN2) * args.splits;
   int pairs = sm_budget() / 2;
   if (tiles < pairs) pairs = tiles;
   e = launch_pdl(kern, dim3(2 * pairs), dim3(kThreads2), kSmem2, stream, ta, tb, tc, td, args);
@@ -673,7 +709,7 @@ int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
 int gemm_tcgen05_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, bool a_mn, bool b_mn,
                       bool a3d, bool b3d, int tma_out, float* C, const float* aux, int64_t ldc, int M, int N, int K,
                       int epilogue, int vec_ok, int splits, int* status, cudaStream_t stream) {
-  Gemm2Args args{C, aux, ldc, M, N, K, epilogue, vec_ok, splits, a3d ? 1 : 0, b3d ? 1 : 0, tma_out, 0, 1, nullptr, 0, 0, 0, kStages2, status};
+  Gemm2Args args{C, aux, ldc, M, N, K, epilogue, vec_ok, splits, a3d ? 1 : 0, b3d ? 1 : 0, tma_out, 0, 1, nullptr, 0, 0, 0, 0.0f, kStages2, status};
   if (!a_mn && !b_mn) return launch2<false, false>(ta, tb, tc, tc, args, stream);
   if (!a_mn && b_mn) return launch2<false, true>(ta, tb, tc, tc, args, stream);
   if (a_mn && !b_mn) return launch2<true, false>(ta, tb, tc, tc, args, stream);
@@ -684,7 +720,7 @@ int gemm_tcgen05_2cta(const CUtensorMap& ta, const CUtensorMap& tb, const CUtens
 // 1) or split-K partial tiles added into a zeroed C (tma_out 2).
 int gemm_tcgen05_2cta_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, int tma_out, float* C,
                            int64_t ldc, int M, int N, int K, int vec_ok, int splits, int* status, cudaStream_t stream) {
-  Gemm2Args args{C, nullptr, ldc, M, N, K, CTDK_EPI_STORE, vec_ok, splits, 0, 0, tma_out, 0, 1, nullptr, 0, 0, 0, kStages2, status};
+  Gemm2Args args{C, nullptr, ldc, M, N, K, CTDK_EPI_STORE, vec_ok, splits, 0, 0, tma_out, 0, 1, nullptr, 0, 0, 0, 0.0f, kStages2, status};
   return launch2<false, false, true>(ta, tb, tc, tc, args, stream);
 }
 
@@ -693,15 +729,23 @@ int gemm_tcgen05_2cta_bf16(const CUtensorMap& ta, const CUtensorMap& tb, const C
 // outputs, {32, 32} boxes. N must be a multiple of 128.
 int gemm_tcgen05_2cta_swiglu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tgu, const CUtensorMap& tact,
                              int M, int N, int K, int* status, cudaStream_t stream) {
-  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, 0, 1, 1, 0, nullptr, 0, 0, 0, kStages2, status};
+  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, 0, 1, 1, 0, nullptr, 0, 0, 0, 0.0f, kStages2, status};
   return launch2<false, false>(ta, tb, tgu, tact, args, stream);
+}
+
+// act[M, N] (bfloat16) = clamped GLU of A[M, K] * W[2N, K]^T with bfloat16 operands (maps with {64, 128} boxes); tact: act,
+// {64, 32} boxes. N must be a multiple of 128.
+int gemm_tcgen05_2cta_clamped_glu(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tact, int M, int N, int K, float limit, int* status,
+                                  cudaStream_t stream) {
+  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, 0, 1, 3, 0, nullptr, 0, 0, 0, limit, kStages2, status};
+  return launch2<false, false, true>(ta, tb, tact, tact, args, stream);
 }
 
 // Fused SwiGLU backward: d(act)[M, N] = A[M, K] * B[K, N] (B MN-major, 3-D map when b3d) stays in the
 // accumulator; tgu: gate|up [M, 2N] for loading, tdgu: d(gate)|d(up) [M, 2N] for storing, {32, 32} boxes.
 int gemm_tcgen05_2cta_swiglu_bwd(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tgu, const CUtensorMap& tdgu,
                                  bool b3d, int M, int N, int K, int* status, cudaStream_t stream) {
-  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, b3d ? 1 : 0, 1, 2, 0, nullptr, 0, 0, 0, kStages2 - 1, status};
+  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, b3d ? 1 : 0, 1, 2, 0, nullptr, 0, 0, 0, 0.0f, kStages2 - 1, status};
   return launch2<false, true>(ta, tb, tgu, tdgu, args, stream);
 }
 
@@ -710,7 +754,7 @@ int gemm_tcgen05_2cta_swiglu_bwd(const CUtensorMap& ta, const CUtensorMap& tb, c
 int gemm_tcgen05_2cta_dattn_delta(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& to,
                                   bool b3d, float* delta, int M, int N, int K, int T, int H, int D, int* status,
                                   cudaStream_t stream) {
-  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, b3d ? 1 : 0, 1, 0, 0, delta, T, H, D, kStages2 - 1, status};
+  Gemm2Args args{nullptr, nullptr, 0, M, N, K, CTDK_EPI_STORE, 1, 1, 0, b3d ? 1 : 0, 1, 0, 0, delta, T, H, D, 0.0f, kStages2 - 1, status};
   return launch2<false, true>(ta, tb, tc, to, args, stream);
 }
 

@@ -14,7 +14,16 @@
 #include "hybrid_decoder.h"
 
 namespace ctdk {
+
+int gemm_bf16_clamped_glu(const void* A, const void* W, __nv_bfloat16* act, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldw, int64_t ld_act,
+                          float limit, cudaStream_t stream);
+
 namespace hybrid {
+
+int glu_product(const __nv_bfloat16* h, const __nv_bfloat16* w_gu, __nv_bfloat16* act, int64_t M, int64_t ffp, int64_t K, int64_t ld, float limit,
+                cudaStream_t s) {
+  return gemm_bf16_clamped_glu(h, w_gu, act, M, ffp, K, ld, ld, ffp, limit, s);
+}
 
 template <typename T>
 int HybridDecoder<T>::carve(Bump& b) {
@@ -554,8 +563,12 @@ int HybridDecoder<T>::run_rows(const int64_t* ids, int64_t n, int64_t pos, int64
     else pending(vec(L.norm1b), nullptr, nullptr, nullptr);
     if (L.ff > 0) {
       DTRY(sandwich(vec(L.norm2)));
-      DTRY(gemm_rows(h, at<T>(L.w_gu), gu, n, 2 * L.ffp, m.width, m.ldw, m.ldw, 2 * L.ffp, s));
-      DTRY(clamped_glu_rows(gu, act, n, L.ffp, L.limit, s));
+      const int fused = glu_product(h, at<T>(L.w_gu), act, n, L.ffp, m.width, m.ldw, L.limit, s);
+      if (fused < 0) return fused;
+      if (fused > 0) {
+        DTRY(gemm_rows(h, at<T>(L.w_gu), gu, n, 2 * L.ffp, m.width, m.ldw, m.ldw, 2 * L.ffp, s));
+        DTRY(clamped_glu_rows(gu, act, n, L.ffp, L.limit, s));
+      }
       DTRY(gemm_rows(act, at<T>(L.w_down), y1, n, m.width, L.ff, L.ffp, L.ld_down, m.width, s));
       pending(vec(L.norm2b), nullptr, nullptr, nullptr);
     }

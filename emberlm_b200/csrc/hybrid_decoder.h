@@ -23,6 +23,11 @@ inline int gemm_rows(const float* A, const float* W, float* C, int64_t M, int64_
   return ctdk_gemm(A, W, C, M, N, K, lda, ldw, ldc, 0, 1, CTDK_GEMM_FP32_SIMT, CTDK_EPI_STORE, nullptr, s);
 }
 
+// The clamped GLU in the gate|up product's epilogue; 1: not for this type or these sizes.
+int glu_product(const __nv_bfloat16* h, const __nv_bfloat16* w_gu, __nv_bfloat16* act, int64_t M, int64_t ffp, int64_t K, int64_t ld, float limit,
+                cudaStream_t s);
+inline int glu_product(const float*, const float*, float*, int64_t, int64_t, int64_t, int64_t, float, cudaStream_t) { return 1; }
+
 // Device buffers of one branch.
 struct BranchBuffers {
   void* cache = nullptr;        // attention

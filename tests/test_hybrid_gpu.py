@@ -358,3 +358,14 @@ def test_ids_outside_the_vocabulary(family, dtype):
         lib.check(E._L.ctdk_device_status(dec.stream.cuda_stream, words))
         counts.append(words[2])
     assert [b - a for a, b in zip(counts, counts[1:])] == [1, 1, 1, 1]
+
+
+@pytest.mark.parametrize("rows, ff", [(513, 2432), (700, 2560), (700, 2440), (300, 2432)])
+def test_glu_in_the_products_epilogue(rows, ff):
+    """A prompt whose gate|up product takes the paired-CTA kernel with the GLU in its epilogue (ff a multiple of 128, ragged
+    rows), and ones whose ff or rows keep the separate kernel: logits of the last rows against the oracle, limit as above."""
+    cfg = hc.model(40, 64, [hc.delta(1, 1, 8, 8, 2, hc.mlp(ff, 1.0))])
+    w, t = hc.weights(cfg, 81), hc.tokens(cfg, rows, 82)
+    dec = decoder(cfg, w, "bf16", max_seq=rows, max_portion=rows)
+    at = list(range(rows - 40, rows))
+    assert hc.error(dec.extend(t, at).cpu().numpy(), oh.forward(cfg, w, t)[at]) <= LIMIT["bf16"]
