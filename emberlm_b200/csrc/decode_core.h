@@ -62,8 +62,6 @@ struct Bump {
     if (rc_ != CTDK_OK) return rc_;   \
   } while (0)
 
-// ---- grid barrier of the persistent token kernels --------------------------------------------
-// Barrier words: [0] arrivals, [2] abort flag (all zero at launch).
 #ifdef __CUDACC__
 __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
   unsigned int v;
@@ -71,50 +69,6 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
   return v;
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-// All CTAs of a cooperative grid meet here: one release reduction on a counter per CTA (no value
-// comes back, so the arriving thread does not wait for it; the CTA's earlier writes are ordered
-// before it by the bar.sync and the release), then one thread per CTA polls the counter. A flag per
-// CTA watched by every other CTA measured twice as slow (all pollers hit the same few L2 lines).
-// `epoch` counts the barriers this CTA has passed. Bounded: when the wait runs out, the status word
-// gets `where` and the abort flag makes every CTA leave at its next barrier. Returns false once any
-// CTA has given up: the caller unwinds.
-__device__ __forceinline__ bool grid_barrier(unsigned int* sync, int* status, int where, unsigned int& epoch) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ++epoch;
-    const unsigned int target = epoch * gridDim.x;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync[0]) : "memory");
-    int ok = 1;
-    if (ld_acquire_u32(&sync[0]) < target) {
-      const uint64_t t0 = globaltimer_ns();
-      unsigned int spins = 0;
-      while (ld_acquire_u32(&sync[0]) < target) {
-        if ((++spins & 0xffu) == 0u) {
-          if (ld_acquire_u32(&sync[2]) != 0u) {   // someone else gave up
-            ok = 0;
-            break;
-          }
-          if (globaltimer_ns() - t0 > kWaitBudgetNs) {
-            if (atomicCAS(status, 0, CTDK_ETIMEOUT) == 0) {
-              status[1] = where;
-              status[2] = static_cast<int>(blockIdx.x);
-              status[3] = static_cast<int>(epoch);
-            }
-            atomicExch(&sync[2], 1u);
-            ok = 0;
-            break;
-          }
-        }
-      }
-    }
-    if (ok && ld_acquire_u32(&sync[2]) != 0u) ok = 0;
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
 #endif
 
 }  // namespace ctdk

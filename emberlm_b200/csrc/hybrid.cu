@@ -29,7 +29,7 @@ template <typename T>
 int HybridDecoder<T>::carve(Bump& b) {
   if (m.arrangement == Arrangement::kParallel) return carve_parallel(b);
   const int64_t R = max_portion, W = m.width;
-  int64_t n_in = 8, mix = 8, heads_out = 8, packed_n = 0, attn_n = 0, ff = 8, parts = 0, arrives = 0;
+  int64_t n_in = 8, mix = 8, heads_out = 8, packed_n = 0, attn_n = 0, ff = 8, parts = 0;
   int64_t ck_n = 0, cv_n = 0, cs_n = 0, cd_n = 0;
   int64_t chunk_n = 0, qk_tiles = 0, v_tiles = 0;
   int64_t qk = 0, dv_n = 0, dlog_n = 0, db_n = 0, rank = 8, rank_g = 8, gate_n = 0;
@@ -52,7 +52,6 @@ int HybridDecoder<T>::carve(Bump& b) {
         packed_n = std::max(packed_n, rows * (br.heads + 2 * br.kv_heads) * Dp);
         attn_n = std::max(attn_n, rows * br.heads * Dp);
         parts = std::max<int64_t>(parts, static_cast<int64_t>(br.heads) * kAttnSplits * (br.dim + kAttnStats));
-        arrives = std::max<int64_t>(arrives, br.kv_heads);
         for (size_t i = 0; i < ropes.size() && bb.rope < 0; ++i)
           if (ropes[i].spec == br.rope && ropes[i].rows >= bb.chunk) bb.rope = static_cast<int>(i);
         if (bb.rope < 0) {
@@ -143,9 +142,11 @@ int HybridDecoder<T>::carve(Bump& b) {
   ty2 = b.floats(W);
   tgu = b.floats(2 * ff);
   tpart = b.floats(parts);
-  sync_words = kTokenSyncWords + 2 * arrives;
+  sync_words = kTokenSyncWords;
   sync = static_cast<unsigned int*>(b.bytes(sync_words * 4));
   phases_dev = static_cast<TokenPhase*>(b.bytes(static_cast<int64_t>(m.layers.size() * 5 + 1) * sizeof(TokenPhase)));
+  max_products = static_cast<int>(m.layers.size()) * 5 + 1;
+  products_dev = static_cast<RingProduct*>(b.bytes(max_products * static_cast<int64_t>(sizeof(RingProduct))));
   logits = b.floats(vocab);
   cur_token = static_cast<int64_t*>(b.bytes(16));
   counters = static_cast<int*>(b.bytes(64));
@@ -164,7 +165,6 @@ int HybridDecoder<T>::build_phases() {
   auto product = [&](int stage) {
     TokenPhase p{};
     p.stage = stage;
-    p.prefetch = -1;
     return p;
   };
   auto norm_phase = [&](const float* w_pre, bool store) {
@@ -192,7 +192,6 @@ int HybridDecoder<T>::build_phases() {
 
     TokenPhase mx{};
     mx.is_mix = 1;
-    mx.prefetch = -1;
     mx.proj = tproj;
     mx.n_branch = static_cast<int>(L.branches.size());
     TokenPhase o = product(kStageMixed);
@@ -217,7 +216,6 @@ int HybridDecoder<T>::build_phases() {
       const int column_blocks = (br.vdim + 31) / 32;
       if (br.kind == BranchKind::kAttention) {
         t.kind = kTokAttention;
-        t.items = br.kv_heads * kAttnSplits;
         t.b_q = vec(br.b_q);
         t.b_k = vec(br.b_k);
         t.table = ropes[bb.rope].table;
@@ -226,7 +224,12 @@ int HybridDecoder<T>::build_phases() {
         t.scale = br.scale;
         t.cache = bb.cache;
         t.part = tpart;
-        t.arrive = sync + kTokenSyncWords + b * ((sync_words - kTokenSyncWords) / 2);
+        t.elem = static_cast<int>(sizeof(T));
+        // the branch's items and the other one's, if possible, in one turn of the CTAs
+        t.splits = kAttnSplits;
+        const int others = mx.n_branch == 2 ? L.branches[1 - b].heads * ((L.branches[1 - b].vdim + 31) / 32) : 0;
+        if (sm_count() > others) t.splits = std::max(4, std::min(kAttnSplits, (sm_count() - others) / br.kv_heads));
+        t.items = br.kv_heads * t.splits;
       } else if (br.kind == BranchKind::kLightning) {
         t.kind = kTokLightning;
         t.items = br.heads * column_blocks;
@@ -235,6 +238,7 @@ int HybridDecoder<T>::build_phases() {
         t.w_norm = vec(br.w_norm);
       } else {
         t.kind = kTokDelta;
+        t.elem = static_cast<int>(sizeof(T));
         t.items = br.heads * column_blocks;
         t.state = bb.state;
         t.w_norm = vec(br.w_norm);
@@ -251,6 +255,10 @@ int HybridDecoder<T>::build_phases() {
         t.dt_bias = vec(br.dt_bias);
         t.w_a2 = at<T>(br.w_a2);
         t.w_g2 = at<T>(br.w_g2);
+        mx.extra[0] = t.w_a2;
+        mx.extra_bytes[0] = static_cast<int64_t>(br.heads) * br.dim * br.ld_a2 * static_cast<int64_t>(sizeof(T));
+        mx.extra[1] = t.w_g2;
+        mx.extra_bytes[1] = static_cast<int64_t>(br.heads) * br.vdim * br.ld_g2 * static_cast<int64_t>(sizeof(T));
         t.ring = bb.ring;
         t.gate = tgate;
       }
@@ -295,35 +303,28 @@ int HybridDecoder<T>::build_phases() {
   return finish_phases();
 }
 
-// Prefetch order, shared memory, warps per row.
+// Requests, shared memory, the weight ring, warps per row.
 template <typename T>
 int HybridDecoder<T>::finish_phases() {
-  // every phase asks for the weights of one coming product, the mix phases run the queue one ahead
   const int n = static_cast<int>(phases.size());
-  int next = 1;
-  for (int i = 0; i < n; ++i) {
-    next = std::max(next, i + 1);
-    while (next < n && (phases[next].is_mix || (phases[next].n_gemv == 0 && phases[next].extra == nullptr))) ++next;
-    if (next < n && next - i <= 3) phases[i].prefetch = next++;
-  }
-  token_smem = token_smem_bytes(stage_floats, phases.data(), n);
-  CTDK_REQUIRE(token_smem <= 200 * 1024, "hybrid decoder: the token pass needs %zu bytes of shared memory", token_smem);
-  int rc = token_grid<T>(token_smem, m.arrangement == Arrangement::kParallel, &token_ctas);
-  if (rc != CTDK_OK) return rc;
-  for (TokenPhase& p : phases) {
-    if (p.is_mix) continue;
-    int rows = 0, K = 0;
-    for (int i = 0; i < p.n_gemv; ++i) {
-      rows += p.gemv[i].rows;
-      K = std::max(K, p.gemv[i].K);
+  for (int i = 0; i < n; ++i)
+    for (int k = 0; k < kMaxAsks; ++k) {
+      phases[i].ask[k] = phases[(i + 1) % n].extra[k];
+      phases[i].ask_bytes[k] = phases[(i + 1) % n].extra_bytes[k];
     }
-    int wpr = 1;
-    while (wpr < 8 && static_cast<int64_t>(rows) * wpr * 2 <= static_cast<int64_t>(token_ctas) * 8 &&
-           K * static_cast<int>(sizeof(T)) / 16 >= 64 * wpr)
-      wpr *= 2;
-    p.wpr = wpr;
+  token_ctas = sm_count();
+  if (m.arrangement == Arrangement::kParallel) {
+    token_smem = static_cast<size_t>(stage_floats) * 4;
+    CTDK_REQUIRE(token_smem <= 200 * 1024, "hybrid decoder: the token pass needs %zu bytes of shared memory", token_smem);
+    list_plan<T>(phases.data(), n, token_ctas);
+    return list_grid<T>(token_smem, &token_ctas);
   }
-  return CTDK_OK;
+  ring.stage_floats = std::max(stage_floats, token_items(phases.data(), n, &ring.item_at));
+  CTDK_REQUIRE(ring.stage_floats <= 50 * 1024, "hybrid decoder: the token pass needs %d bytes of shared memory", ring.stage_floats * 4);
+  token_smem = token_plan<T>(phases.data(), n, token_ctas, ring, products);
+  CTDK_REQUIRE(token_smem > 0, "hybrid decoder: no room for the weight ring behind %d floats", ring.stage_floats);
+  CTDK_REQUIRE(products.size() <= static_cast<size_t>(max_products), "hybrid decoder: too many products");
+  return token_grid<T>(token_smem, &token_ctas);
 }
 
 // Constant tables: phases, decays, rotations. Synchronises (creation time only).
@@ -331,7 +332,8 @@ template <typename T>
 int HybridDecoder<T>::upload(cudaStream_t s) {
   auto copy = [&](void* dst, const void* src, size_t n) { return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, s) == cudaSuccess; };
   std::vector<std::vector<float>> powers;
-  bool ok = copy(phases_dev, phases.data(), phases.size() * sizeof(TokenPhase));
+  bool ok = copy(phases_dev, phases.data(), phases.size() * sizeof(TokenPhase)) &&
+            copy(products_dev, products.data(), products.size() * sizeof(RingProduct));
   for (size_t l = 0; l < m.layers.size(); ++l)
     for (size_t b = 0; b < bufs[l].size(); ++b)
       if (bufs[l][b].decay != nullptr) {
@@ -634,8 +636,9 @@ int HybridDecoder<T>::portion(const int64_t* ids, int64_t n, int64_t pos, const 
 
 template <typename T>
 TokenArgs HybridDecoder<T>::token_args() const {
-  TokenArgs a{};
+  TokenArgs a = ring;
   a.phases = phases_dev;
+  a.products = products_dev;
   a.n_phases = static_cast<int>(phases.size());
   a.width = m.width;
   a.eps = m.eps;
@@ -657,7 +660,8 @@ template <typename T>
 int HybridDecoder<T>::token_forward(cudaStream_t s) {
   const TokenArgs a = token_args();
   CTDK_REQUIRE(a.status != nullptr, "hybrid decoder: no status word");
-  return launch_token_kernel<T>(a, m.arrangement == Arrangement::kParallel, token_ctas, token_smem, s);
+  return m.arrangement == Arrangement::kParallel ? launch_list_kernel<T>(a, token_ctas, token_smem, s)
+                                                 : launch_token_kernel<T>(a, token_ctas, token_smem, s);
 }
 
 template <typename T>
@@ -667,7 +671,8 @@ int HybridDecoder<T>::burst(int64_t n, int64_t* out_tokens, cudaStream_t s) {
   a.out_tokens = out_tokens;
   a.out_offset = static_cast<int>(generated);
   a.n_tokens = static_cast<int>(n);
-  return launch_token_kernel<T>(a, m.arrangement == Arrangement::kParallel, token_ctas, token_smem, s);
+  return m.arrangement == Arrangement::kParallel ? launch_list_kernel<T>(a, token_ctas, token_smem, s)
+                                                 : launch_token_kernel<T>(a, token_ctas, token_smem, s);
 }
 
 namespace {

@@ -76,6 +76,10 @@ struct HybridDecoder : DecoderBase {
   unsigned int* sync;
   int64_t sync_words = 0;
   TokenPhase* phases_dev;
+  RingProduct* products_dev;   // what passes through the token kernel's weight ring, in order
+  int max_products = 0;
+  std::vector<RingProduct> products;
+  TokenArgs ring{};            // the ring's layout
   std::vector<TokenPhase> phases;
   int stage_floats = 0, token_ctas = 0;
   size_t token_smem = 0;

@@ -43,7 +43,7 @@ int HybridDecoder<T>::carve_parallel(Bump& b) {
       q_up_n = std::max<int64_t>(q_up_n, pad8(static_cast<int64_t>(br.heads) * (br.dim + br.rot_dim)));
       q_rot_n = std::max<int64_t>(q_rot_n, static_cast<int64_t>(br.heads) * latent_q_pitch(br.dim, br.rot_dim));
       kv_n = std::max<int64_t>(kv_n, br.n_ukv);
-      parts = std::max<int64_t>(parts, static_cast<int64_t>(br.heads) * kLatentSplits * (bb.n_latent_rot + kAttnStats4));
+      parts = std::max<int64_t>(parts, static_cast<int64_t>(br.heads) * kLatentSplits * (bb.n_latent_rot + kAttnStats));
       abs_n = std::max<int64_t>(abs_n, br.heads * bb.ld_latent);
       for (size_t i = 0; i < ropes.size() && bb.rope < 0; ++i)
         if (ropes[i].spec == br.rope) bb.rope = static_cast<int>(i);
@@ -136,6 +136,8 @@ int HybridDecoder<T>::carve_parallel(Bump& b) {
   sync_words = kTokenSyncWords;
   sync = static_cast<unsigned int*>(b.bytes(sync_words * 4));
   phases_dev = static_cast<TokenPhase*>(b.bytes((n_layers * 6 + 1) * static_cast<int64_t>(sizeof(TokenPhase))));
+  max_products = static_cast<int>(n_layers) * 10 + 1;   // five mixes, the side product, output and feed-forward
+  products_dev = static_cast<RingProduct*>(b.bytes(max_products * static_cast<int64_t>(sizeof(RingProduct))));
   logits = b.floats(vocab);
   cur_token = static_cast<int64_t*>(b.bytes(16));
   counters = static_cast<int*>(b.bytes(64));
@@ -157,7 +159,6 @@ int HybridDecoder<T>::build_parallel_phases() {
   auto list = [&] {
     TokenPhase p{};
     p.stage = kStageList;
-    p.prefetch = -1;
     return p;
   };
   auto add_op = [&](TokenPhase& p, int kind, int64_t at, int64_t n, int64_t ld, const float* src, const float* src2 = nullptr,
@@ -328,8 +329,8 @@ int HybridDecoder<T>::build_parallel_phases() {
       items(k, kTokLatentKeys, br.heads * ((t.rot_col + key_cols - 1) / key_cols));
       down(k, 0);
       need(kListThreads / 16 * (key_cols + 1));
-      k.extra = at<T>(br.w_ukv);
-      k.extra_bytes = static_cast<int64_t>(br.row_uv) * br.ld_ukv * esize;
+      k.extra[0] = at<T>(br.w_ukv);
+      k.extra_bytes[0] = static_cast<int64_t>(br.row_uv) * br.ld_ukv * esize;
       phases.push_back(k);
 
       TokenPhase sc = list();
@@ -345,8 +346,8 @@ int HybridDecoder<T>::build_parallel_phases() {
       TokenPhase v = list();
       items(v, kTokLatentOut, br.heads * ((br.vdim + kLatentOutRows - 1) / kLatentOutRows));
       need(t.rot_col * (1 + kLatentOutParts) + kLatentSplits);
-      v.extra = at<T>(br.w_ukv) + static_cast<int64_t>(br.row_uv) * br.ld_ukv;
-      v.extra_bytes = static_cast<int64_t>(br.heads) * br.vdim * br.ld_ukv * esize;
+      v.extra[0] = at<T>(br.w_ukv) + static_cast<int64_t>(br.row_uv) * br.ld_ukv;
+      v.extra_bytes[0] = static_cast<int64_t>(br.heads) * br.vdim * br.ld_ukv * esize;
       phases.push_back(v);
 
       TokenPhase o = list();
@@ -356,6 +357,8 @@ int HybridDecoder<T>::build_parallel_phases() {
     } else {
       TokenPhase q = list();
       items(q, kTokWkv, t.items);
+      q.extra[0] = t.w_w2;
+      q.extra_bytes[0] = static_cast<int64_t>(br.heads) * br.dim * br.ld_w2 * static_cast<int64_t>(sizeof(T));
       need(br.ld_w2 + 4 * br.dim + kListThreads);
       if (moe) expert_up(q, 0);
       phases.push_back(q);

@@ -4,14 +4,15 @@
 
 #include <cuda_bf16.h>
 
-#include "common.cuh"
+#include <vector>
+
+#include "token_ring.cuh"
 
 namespace ctdk {
 namespace hybrid {
 
 constexpr int kAttnSplits = 16;   // most key ranges per key/value head
-constexpr int kAttnStats = 2;     // running maximum and sum in front of a partial output
-constexpr int kAttnStats4 = 4;    // the same, with room that keeps the output 16-byte aligned
+constexpr int kAttnStats = 4;     // running maximum and sum in front of a partial output, with room that keeps it 16-byte aligned
 
 constexpr int kListThreads = 512, kListWarps = kListThreads / 32;   // of a CTA that runs kStageList phases, one per SM
 constexpr int kLatentHeads = 16;   // query heads that share one pass over the latent cache (bfloat16)
@@ -36,6 +37,8 @@ struct TokenGemv {
   int mode, per, pitch, top, experts, K2, in2;
   const void* W2;
   const float* h;
+  RingRows ring;   // plain products pass through the weight ring
+  int base;        // first row among the phase's plain rows
 };
 
 // What a kStageList phase puts into the staged vector, in order (`at`: first float; padded with zeros to `ld`).
@@ -54,7 +57,7 @@ struct StageOp {
   int kind, at, n, ld;
   const float *src, *src2, *w;
 };
-constexpr int kMaxGemv = 6, kMaxOps = 4, kTokenMixes = 5;
+constexpr int kMaxGemv = 6, kMaxOps = 4, kTokenMixes = 5, kMaxAsks = 2;
 
 // Residual and norm of the parallel arrangement (see ShiftNormArgs). state: [2 slots][h, m][width], a
 // position reads the slot of the one before and writes its own (slot = position mod 2).
@@ -68,7 +71,7 @@ struct TokenShift {
 // A mixer branch: what the mix phase computes and what the output projection stages from it.
 struct TokenBranch {
   int kind, items;
-  int H, G, dim, vdim;
+  int H, G, dim, vdim, group;   // group: H / G
   int col_q, col_k, col_v, col_g;
   float* out;            // [H * vdim]: attention gated, recurrences raw
   int stage_at;          // offset of this branch in the staged vector
@@ -79,7 +82,7 @@ struct TokenBranch {
   float scale;
   void* cache;
   float* part;           // [H][kAttnSplits][dim + kAttnStats]
-  unsigned int* arrive;  // [G]
+  int elem, tile_keys;   // bytes of a cached value; keys that stand in shared memory at a time
   // recurrences
   const float* decay;
   float* state;
@@ -88,6 +91,7 @@ struct TokenBranch {
   int taps, col_b, col_a1, col_g1, rank_a, rank_g;
   const float *conv_q, *conv_k, *conv_v, *a_log, *dt_bias;
   const void *w_a2, *w_g2;
+  int low_staged;        // whether an item's rows of them fit into shared memory
   float* ring;
   float* gate;           // [H * vdim] output gate before the sigmoid
   // wkv
@@ -95,24 +99,28 @@ struct TokenBranch {
   const void* w_w2;
   const float *w0, *bonus;
   // latent attention
-  int rot_dim, kv_rank, rot_col, ld_cache, ld_ukv, row_uv, splits, blocks, buffers;   // buffers: cache tiles in flight (1 or 2)
+  int rot_dim, kv_rank, rot_col, ld_cache, ld_ukv, row_uv, splits, blocks, buffers;   // splits: most ranges (attention: per key/value head); buffers: cache tiles in flight (1 or 2)
   const void* w_ukv;
   const float *kv_norm, *q_up;   // queries [H][dim + rot_dim]
   void* q_abs;           // [H][ld_cache] queries against the cache rows, scaled: fp32, or two bfloat16 planes
 };
 
-struct TokenPhase {
+struct alignas(16) TokenPhase {
   int is_mix;
   // products
-  int stage, n_gemv, wpr, is_head;
+  int stage, n_gemv, wpr, is_head;   // wpr: warps that share a row (kStageList phases)
   TokenGemv gemv[kMaxGemv];
   // kStageList phases: staging, products and the items of branch 0 in one phase
   int n_ops;
   StageOp op[kMaxOps];
   TokenShift shift;
   int route_groups, route_keep, route_top;
-  const void* extra;     // weights of the items, for the prefetch
-  int64_t extra_bytes;
+  int plain_rows, per;           // rows of all products, how many of them a CTA takes (sandwich layers)
+  int prefetch;                  // kStageList: phase whose weights this one requests into L2, or -1
+  const void* extra[kMaxAsks];   // weights of the items
+  int64_t extra_bytes[kMaxAsks];
+  const void* ask[kMaxAsks];     // those of the next phase: requested into L2 by this one
+  int64_t ask_bytes[kMaxAsks];
   int first_token;       // kStageNorm: x comes from the embedding
   const float *x, *y, *y2, *w_y, *w_y2, *w_post, *w_pre;
   float* x_out;
@@ -120,14 +128,22 @@ struct TokenPhase {
   int ffp;
   float limit;
   // mixing
-  int n_branch;
+  int n_branch, items;   // items: of all branches (sandwich layers)
   TokenBranch br[2];
   const float* proj;
-  int prefetch;          // phase whose weights this one requests into L2, or -1
+};
+
+// A plain product as the requesting warp reads it.
+struct RingProduct {
+  const void* W;
+  int rows, base, per, plain_rows;
+  RingRows ring;
 };
 
 struct TokenArgs {
   const TokenPhase* phases;
+  const RingProduct* products;
+  int n_products, stage_floats, item_at, stages, stage_bytes;   // item_at: first float of what a mix item copies ahead
   int n_phases, width;
   float eps;
   const void* embed;
@@ -137,7 +153,7 @@ struct TokenArgs {
   int vocab;
   int64_t* cur_token;
   int* counters;
-  unsigned int* sync;        // barrier words, the two arg-max words at [128], head arrivals from [256]
+  unsigned int* sync;        // barrier words, the two arg-max words at [128]
   int sync_words;
   int64_t* out_tokens;       // null: one token, logits only
   int out_offset, n_tokens;
@@ -146,12 +162,26 @@ struct TokenArgs {
 
 constexpr int kTokenSyncWords = 256;
 
-// Shared memory the kernel needs for a phase list (bytes), from the largest staged vector (floats).
-size_t token_smem_bytes(int stage_floats, const TokenPhase* phases, int n);
+// Floats that the mix items need in place of the staged vector; tile_at: the first one of what is copied ahead of an item.
+int token_items(TokenPhase* phases, int n, int* tile_at);
+// Deals the rows of all plain products to `grid` CTAs and lays the weight ring out behind the staged vector
+// (a.stage_floats). Returns the kernel's dynamic shared memory (bytes), 0 when there is no room.
 template <typename T>
-int token_grid(size_t smem, bool list, int* grid);   // CTAs of the cooperative launch; list: kStageList phases only
+size_t token_plan(TokenPhase* phases, int n, int grid, TokenArgs& a, std::vector<RingProduct>& products);
 template <typename T>
-int launch_token_kernel(const TokenArgs& a, bool list, int grid, size_t smem, cudaStream_t s);
+int token_grid(size_t smem, int* grid);   // CTAs of the cooperative launch
+template <typename T>
+int launch_token_kernel(const TokenArgs& a, int grid, size_t smem, cudaStream_t s);
+// The same for kStageList phases (hybrid_list.cu).
+template <typename T>
+void list_plan(TokenPhase* phases, int n, int grid);
+template <typename T>
+int list_grid(size_t smem, int* grid);
+template <typename T>
+int launch_list_kernel(const TokenArgs& a, int grid, size_t smem, cudaStream_t s);
+
+int cooperative_grid(const void* kernel, int threads, size_t smem, int* grid);
+int cooperative_launch(const void* kernel, const TokenArgs& a, int grid, int threads, size_t smem, cudaStream_t s);
 
 }  // namespace hybrid
 }  // namespace ctdk

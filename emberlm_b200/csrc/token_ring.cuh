@@ -39,20 +39,66 @@ inline int ring_stage_bytes(const RingRows& r) { return kRingWarps * r.len * 16;
 
 #ifdef __CUDACC__
 
-// Barriers of the compute warps. The instructions want whole warps: lanes that a poll or a store of one lane has
+// Barriers of the compute warps (W of them). The instructions want whole warps: lanes that a poll or a store of one lane has
 // split off come back first.
+template <int W = kRingWarps>
 __device__ __forceinline__ void ring_sync() {
   __syncwarp();
-  asm volatile("bar.sync 1, %0;" ::"n"(kRingThreads) : "memory");
+  asm volatile("bar.sync 1, %0;" ::"n"(32 * W) : "memory");
 }
+template <int W = kRingWarps>
 __device__ __forceinline__ bool ring_or(bool x) {
   unsigned r;
   __syncwarp();
   asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
                : "=r"(r)
-               : "r"(static_cast<unsigned>(x)), "n"(kRingThreads)
+               : "r"(static_cast<unsigned>(x)), "n"(32 * W)
                : "memory");
   return r != 0u;
+}
+
+// Barrier words: [0] arrivals, [kRingAbort] abort flag (all zero at launch).
+// The compute warps of all CTAs of a cooperative grid meet here: one release reduction on a counter per CTA (no value
+// comes back, so the arriving thread does not wait for it; the CTA's earlier writes are ordered
+// before it by the bar.sync and the release), then one thread per CTA polls the counter. A flag per
+// CTA watched by every other CTA measured twice as slow (all pollers hit the same few L2 lines).
+// Arrival and wait are two calls, with whatever does not depend on the others between them. `epoch` counts the barriers this
+// CTA has passed. Bounded: when the wait runs out, the status word gets `where` and the abort flag makes every CTA leave at
+// its next barrier. The wait returns false once any CTA has given up: the caller unwinds.
+template <int W = kRingWarps>
+__device__ __forceinline__ void grid_arrive(unsigned int* sync, unsigned int& epoch) {
+  ring_sync<W>();
+  ++epoch;
+  if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sync[0]) : "memory");
+}
+static __device__ __noinline__ bool grid_wait_longer(unsigned int* sync, int* status, int where, unsigned int target) {
+  const uint64_t t0 = globaltimer_ns();
+  unsigned int spins = 0;
+  while (ld_acquire_u32(&sync[0]) < target) {
+    if ((++spins & 0xffu) != 0u) continue;
+    if (ld_acquire_u32(&sync[kRingAbort]) != 0u) return false;   // someone else gave up
+    if (globaltimer_ns() - t0 > kWaitBudgetNs) {
+      if (atomicCAS(status, 0, CTDK_ETIMEOUT) == 0) {
+        status[1] = where;
+        status[2] = static_cast<int>(blockIdx.x);
+      }
+      atomicExch(&sync[kRingAbort], 1u);
+      return false;
+    }
+  }
+  return true;
+}
+template <int W = kRingWarps>
+__device__ __forceinline__ bool grid_wait(unsigned int* sync, int* status, int where, unsigned int epoch) {
+  bool gone = false;
+  if (threadIdx.x == 0) {
+    const unsigned int target = epoch * gridDim.x;
+    bool there = false;
+#pragma unroll 1
+    for (int i = 0; i < 64 && !there; ++i) there = ld_acquire_u32(&sync[0]) >= target;
+    gone = (!there && !grid_wait_longer(sync, status, where, target)) || ld_acquire_u32(&sync[kRingAbort]) != 0u;
+  }
+  return !ring_or<W>(gone);
 }
 
 // Waits on the ring: the rare part is out of line.

@@ -369,3 +369,29 @@ def test_glu_in_the_products_epilogue(rows, ff):
     dec = decoder(cfg, w, "bf16", max_seq=rows, max_portion=rows)
     at = list(range(rows - 40, rows))
     assert hc.error(dec.extend(t, at).cpu().numpy(), oh.forward(cfg, w, t)[at]) <= LIMIT["bf16"]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [30, 1024, 1028, 2048, 2052])
+def test_widths_of_the_norms(width, dtype):
+    """Widths on both sides of what one and two turns of the token pass's threads take, and one that is no multiple of four;
+    limits as above."""
+    cfg = hc.model(50, width, [hc.parallel(hc.attention(2, 1, 8, 8, 8), hc.lightning(1, 8, 8), hc.mlp(9, 7.0)), hc.delta(1, 1, 8, 8, 2)])
+    w, t = hc.weights(cfg, 71), hc.tokens(cfg, 45, 72)
+    want = oh.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype)
+    for sizes in ([45], [23, 1, 1, 1, 19]):
+        dec.reset()
+        assert hc.error(portions(dec, t, sizes), want) <= LIMIT[dtype], sizes
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("ff", [4104, 33000, 38400, 51000])
+def test_long_rows_of_the_token_pass(ff, dtype):
+    """Staged vectors that leave the weight ring less and less room (rows in several pieces, then shorter pieces), up to nearly
+    the largest that is taken; limits as above."""
+    cfg = hc.model(40, 32, [hc.delta(1, 1, 8, 8, 2, hc.mlp(ff, 1.0)), hc.parallel(hc.attention(2, 1, 8, 8, 8), hc.lightning(1, 8, 8), hc.mlp(24, 1.0))])
+    w, t = hc.weights(cfg, 91), hc.tokens(cfg, 9, 92)
+    want = oh.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype)
+    assert hc.error(portions(dec, t, [4, 1, 1, 1, 1, 1]), want) <= LIMIT[dtype]
