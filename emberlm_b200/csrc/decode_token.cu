@@ -11,8 +11,8 @@
 // each, so the instructions of the chain are what the rest of a phase costs: one body for all products, a row per warp whose
 // sum leaves without another barrier, a RMSNorm factor that is applied to the finished sums, no integer divisions (200
 // cycles each) and nothing in local memory (the ring leaves 28 KB of L1).
-// Qwen3-0.6B, 256 + 128 tokens: 109.3 -> 90.1 ms against sixteen warps with the weights in registers and plain stores of the
-// words; SmolLM2-135M, 37 + 48: 26.2 -> 22.0; SmolLM2-360M, 700 + 16 single steps: 17.6 -> 14.6; Llama-3.2-1B, 200 + 32: 33.7 -> 31.4.
+// Qwen3-0.6B, 256 + 128 tokens: 109.3 -> 88.6 ms against sixteen warps with the weights in registers and plain stores of the
+// words; SmolLM2-135M, 37 + 48: 26.2 -> 22.0; SmolLM2-360M, 700 + 16 single steps: 17.6 -> 14.3.
 //
 // Why a buffer can be overwritten without an acknowledgement: every CTA owns at least one row of each
 // product (token_grid), so a complete vector implies that every CTA has finished the phase that read the
@@ -389,8 +389,7 @@ struct PhaseRows {
 
 template <int DC>
 __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_constant__ TokenKernelArgs a) {
-  // two places for the vector or the attention's scratch, the attention's tile, this CTA's residual rows (eight lanes have a
-  // row, each its own copy), the ring
+  // two places for the vector or the attention's scratch, the attention's tile, this CTA's residual rows, the ring
   extern __shared__ __align__(128) float sm[];
   __shared__ __align__(16) float s_red[kWarps];
   __shared__ Word s_best[kWarps];
@@ -429,7 +428,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
       const bool known = tok >= 0 && tok < a.V;
       const float* row = known ? a.P + a.embed + tok * hid : nullptr;
       if (!known && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.status[2], 1);
-      for (int i = threadIdx.x; i < 8 * s_rows[1].count; i += kThreads) res[i] = known ? row[s_rows[1].first + (i >> 3)] : 0.0f;
+      for (int i = threadIdx.x; i < s_rows[1].count; i += kThreads) res[i] = known ? row[s_rows[1].first + i] : 0.0f;
       const int splits = attn_splits(pos + 1, a.Hk), items = a.Hk * splits;
       const Item mine(blockIdx.x, splits, pos + 1);
       Word best = 0ull;
@@ -494,23 +493,23 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
           sc = rsqrtf((((r0.x + r0.y) + (r0.z + r0.w)) + ((r1.x + r1.y) + (r1.z + r1.w))) * inv_hid + a.eps);
         }
         const int first = s_rows[j].first;
-        const bool ok = ring_multiply<float, kLaneChunks>(ring, s_rows[j].rows, s_rows[j].count, j == 2, xs, [&](int row, float v, float u) {
+        const bool glu = j == 2, added = j == 1 || j == 3;
+        Word* const out = (j == 0 ? a.qkv : (j == 1 ? a.hm : (j == 2 ? a.act : a.x))) + first;
+        const unsigned number = e + (j == 0 ? 1u : 3u + j);
+        const bool ok = ring_multiply<float, kLaneChunks>(ring, s_rows[j].rows, s_rows[j].count, glu, xs, [&](int row, float v, float u) {
           v *= sc;
           if (j == 4) {   // tied LM head and arg-max (first index of the maximum)
-            if ((lane & 7) == 0) a.logits[first + row] = v;
+            a.logits[first + row] = v;
             const Word k = argmax_key(v, first + row);
             best = k > best ? k : best;
             return;
           }
-          if (j == 2) {   // act = silu(gate) * up
-            v = __fdividef(v, 1.0f + __expf(-v)) * (u * sc);
-          } else if (j != 0) {   // the same lanes have a row of O and of the down product
-            float* r = res + 8 * row + (lane & 7);
-            v += *r;
-            *r = v;
+          if (glu) v = __fdividef(v, 1.0f + __expf(-v)) * (u * sc);   // act = silu(gate) * up
+          if (added) {   // the same lane has a row of O and of the down product
+            v += res[row];
+            res[row] = v;
           }
-          if ((lane & 7) == 0)
-            put((j == 0 ? a.qkv : (j == 1 ? a.hm : (j == 2 ? a.act : a.x))) + first + row, v, e + (j == 0 ? 1u : 3u + j));
+          put(out + row, v, number);
         });
         if (!ok) p.gone = true;
         if (a.vector_floats > 0) buffer ^= 1;
@@ -584,7 +583,7 @@ size_t plan(TokenKernelArgs& a, int grid) {
   const int64_t vector = (std::max(std::max(a.hid, a.H * a.D), a.I) + 31) / 32 * 32, G = a.H / a.Hk;
   const int64_t attn = G * (a.D + kTileBytes / (8 * a.D)) + kWarps * 34 + 2 * a.D;
   a.group = static_cast<int>(G);
-  a.residual_floats = (8 * ceil_div(a.hid, grid) + 31) / 32 * 32;
+  a.residual_floats = (ceil_div(a.hid, grid) + 31) / 32 * 32;
   const int K[5] = {a.hid, a.H * a.D, a.hid, a.I, a.hid};
   for (int places = 2; places >= 1; --places) {
     a.vector_floats = places == 2 ? static_cast<int>(vector) : 0;

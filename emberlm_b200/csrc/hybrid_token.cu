@@ -6,7 +6,7 @@
 // fp32 behind grid barriers, and every CTA stages (and norms) its own copy. All waits are bounded.
 // What bounds a phase (10 000 to 16 000 cycles; its weights would take 3000) is its dependent chain: the barrier (3200 cycles),
 // the norms (2500 to 3500) or the merging of the key ranges (7400), the products (800 a turn), the mix items (10 000).
-// zutalix-0.6b, 300 + 64 tokens: 109.4 -> 69.3 ms against sixteen warps that took the rows from L2 and the items' inputs behind
+// zutalix-0.6b, 300 + 64 tokens: 109.4 -> 65.0 ms against sixteen warps that took the rows from L2 and the items' inputs behind
 // the barrier. The items' keys, states and gate rows are on their way before it now, and a phase's description one phase ahead.
 #include <cfloat>
 
@@ -716,7 +716,6 @@ __device__ __forceinline__ unsigned long long plain_products(const TokenPhase& p
     if (hi <= lo) continue;
     // a wait that ran out is seen at the barrier
     ring_multiply<T, kTokenLaneChunks<T>>(ring, g.ring, hi - lo, false, sm + g.in, [&](int r, float y, float) {
-      if ((threadIdx.x & 7) != 0) return;
       y *= f;
       const int row = lo - g.base + r;
       g.y[row] = y;

@@ -232,66 +232,74 @@ struct RingChunk<__nv_bfloat16> {
 };
 
 // This CTA's rows of a product with the staged vector: f(row, sum, 0), or with a pair of matrices f(row, sum of the first,
-// sum of the second), by eight lanes (lane mod 8 = 0 .. 7) for each row. C: 16-byte chunks of a lane in a piece. The sums over the lanes of four turns
-// share shuffles (six instead of twenty). False when a wait ran out.
+// sum of the second), by one lane for each row. C: 16-byte chunks of a lane in a piece. The sums over the lanes of four turns
+// share shuffles (seven instead of twenty), and each sum stands in a lane of its own, so that what f does with it is done once
+// for four turns: against two turns at a time with eight lanes for a row, zutalix-0.6b 300 + 64 tokens 69.3 -> 65.0 ms,
+// Qwen3-0.6B 256 + 128 89.5 -> 88.6, SmolLM2-360M single steps 14.75 -> 14.3. False when a wait ran out.
 template <typename T, int C, class F>
 __device__ __forceinline__ bool ring_multiply(Ring& ring, const RingRows& r, int rows, bool pairs, const float* xs, F f) {
   constexpr int N = RingChunk<T>::kN;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int turns = ((rows + kRingWarps - 1) / kRingWarps) << (pairs ? 1 : 0);
   float x[C][N];
-  float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;   // the last four rows, the latest in a0
   bool ok = true;
-#pragma unroll 1
-  for (int turn = 0; turn < turns; ++turn) {
-    const bool mine = (pairs ? turn >> 1 : turn) * kRingWarps + wid < rows;
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 1
-    for (int piece = 0; piece < r.pieces; ++piece) {
-      const int lo = piece * r.len, len = min(r.len, r.chunks - lo), n = len - lane;   // this lane's chunks: 0, 32, ... below n
-      if (turn == 0 || r.pieces > 1) {
+  int n = 0, len = 0;   // this lane's chunks of the piece: 0, 32, ... below n
+  auto values = [&](int piece) {
+    const int lo = piece * r.len;
+    len = min(r.len, r.chunks - lo);
+    n = len - lane;
 #pragma unroll
-        for (int c = 0; c < C; ++c)
+    for (int c = 0; c < C; ++c)
 #pragma unroll
-          for (int e = 0; e < N; e += 4) {
-            const float4 v = 32 * c < n ? *reinterpret_cast<const float4*>(xs + (lo + lane + 32 * c) * N + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-            x[c][e] = v.x;
-            x[c][e + 1] = v.y;
-            x[c][e + 2] = v.z;
-            x[c][e + 3] = v.w;
-          }
+      for (int e = 0; e < N; e += 4) {
+        const float4 v = 32 * c < n ? *reinterpret_cast<const float4*>(xs + (lo + lane + 32 * c) * N + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[c][e] = v.x;
+        x[c][e + 1] = v.y;
+        x[c][e + 2] = v.z;
+        x[c][e + 3] = v.w;
       }
-      ok = ring_wait(ring.full + ring.stage, ring.parity, ring.sync, ring.status) && ok;
-      if (mine) {
-        const uint4* w4 = reinterpret_cast<const uint4*>(ring.here()) + wid * len + lane;
+  };
+  // a warp without a row multiplies what the stage holds in its place, which goes nowhere
+  auto stage = [&](float (&s)[4]) {
+    ok = ring_wait(ring.full + ring.stage, ring.parity, ring.sync, ring.status) && ok;
+    const uint4* w4 = reinterpret_cast<const uint4*>(ring.here()) + wid * len + lane;
 #pragma unroll
-        for (int c = 0; c < C; ++c)
-          if (32 * c < n) RingChunk<T>::dot(w4[32 * c], x[c], s);
+    for (int c = 0; c < C; ++c)
+      if (32 * c < n) RingChunk<T>::dot(w4[32 * c], x[c], s);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(ring.free + ring.stage);
+    ring.next();
+  };
+  values(0);
+#pragma unroll 1
+  for (int turn = 0; turn < turns; turn += 4) {
+    float a[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      a[b] = 0.0f;
+      if (turn + b >= turns) continue;
+      float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      if (r.pieces == 1) {
+        stage(s);
+      } else {
+#pragma unroll 1
+        for (int piece = 0; piece < r.pieces; ++piece) {
+          values(piece);
+          stage(s);
+        }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(ring.free + ring.stage);
-      ring.next();
+      a[b] = (s[0] + s[2]) + (s[1] + s[3]);
     }
-    a3 = a2;
-    a2 = a1;
-    a1 = a0;
-    a0 = (s[0] + s[2]) + (s[1] + s[3]);
-    if ((turn & 3) != 3 && turn + 1 < turns) continue;
+    // lanes 0 .. 7 have the sum of a[0], 16 .. 23 of a[1], 8 .. 15 of a[2], 24 .. 31 of a[3]
     const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
-    const float v0 = (h16 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h16 ? a0 : a1, 16);
-    const float v1 = (h16 ? a3 : a2) + __shfl_xor_sync(0xffffffffu, h16 ? a2 : a3, 16);
+    const float v0 = (h16 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, h16 ? a[0] : a[1], 16);
+    const float v1 = (h16 ? a[3] : a[2]) + __shfl_xor_sync(0xffffffffu, h16 ? a[2] : a[3], 16);
     float v = (h8 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, h8 ? v0 : v1, 8);
 #pragma unroll
     for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const float before = __shfl_xor_sync(0xffffffffu, v, 16);
-    // lanes 0 .. 7 have the sum of a0, 16 .. 23 of a1, 8 .. 15 of a2, 24 .. 31 of a3
-    const int back = (lane >> 4) + ((lane >> 2) & 2), of = turn - back;
-    if (back > (turn & 3)) continue;
-    if (!pairs) {
-      if (of * kRingWarps + wid < rows) f(of * kRingWarps + wid, v, 0.0f);
-    } else if (lane < 16 && (of >> 1) * kRingWarps + wid < rows) {
-      f((of >> 1) * kRingWarps + wid, before, v);
-    }
+    const float behind = __shfl_xor_sync(0xffffffffu, v, 16);
+    const int of = turn + (lane >> 4) + ((lane >> 2) & 2), row = (pairs ? of >> 1 : of) * kRingWarps + wid;
+    if ((lane & 7) == 0 && row < rows && of < turns && !(pairs && lane >= 16)) f(row, v, behind);
   }
   return ok;
 }
