@@ -308,6 +308,7 @@ __global__ void __launch_bounds__(320, 1)
     tc_fence_after();
     tmem_dealloc(tmem_base, C::kTmemCols);
   }
+  pdl_wait();   // the end of this kernel is the end of both, where it runs beside the dK/dV kernel
 }
 
 int map3(CUtensorMap* m, const float* base, int64_t inner, int64_t T, int64_t B, int rows, bool atom32) {
@@ -318,7 +319,7 @@ int map3(CUtensorMap* m, const float* base, int64_t inner, int64_t T, int64_t B,
 }
 
 template <int D, int TKB, int NB, int STG, bool QT>
-int launch_dq(const float* qkv, const float* dout, const BwdArgs& a, int64_t B, cudaStream_t s) {
+int launch_dq(const float* qkv, const float* dout, const BwdArgs& a, int64_t B, bool beside, cudaStream_t s) {
   using C = DqCfg<D, TKB, NB, STG, QT>;
   const int RS = (a.H + 2 * a.Hk) * D;
   CUtensorMap tq, tdo, tkk, tkm;
@@ -331,7 +332,8 @@ int launch_dq(const float* qkv, const float* dout, const BwdArgs& a, int64_t B, 
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmem);
   if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "attn_bwd dq(tcgen05): shared memory opt-in failed: %s", cudaGetErrorString(e));
   dim3 grid(static_cast<unsigned>(static_cast<int64_t>(a.n_qtiles) * a.H * B));
-  kern<<<grid, 320, C::kSmem, s>>>(tq, tdo, tkk, tkm, a);
+  if (beside) launch_pdl(kern, grid, dim3(320), C::kSmem, s, tq, tdo, tkk, tkm, a);
+  else kern<<<grid, 320, C::kSmem, s>>>(tq, tdo, tkk, tkm, a);
   return check_launch("ctdk_attn_bwd(dq, tcgen05)");
 }
 
@@ -339,7 +341,7 @@ int launch_dq(const float* qkv, const float* dout, const BwdArgs& a, int64_t B, 
 
 // Head size 64: persistent kernels with the left-hand operands in tensor memory (attention_tc_bwd64.cu).
 int attn_bwd_dq_tc64(const float* qkv, const float* dout, const float* lse, const float* delta, float* dqkv,
-                     int64_t B, int64_t T, int H, int Hk, cudaStream_t stream);
+                     int64_t B, int64_t T, int H, int Hk, bool beside, cudaStream_t stream);
 int attn_bwd_dkv_tc64(const float* qkv, const float* dout, const float* lse, const float* delta, float* dqkv,
                       int64_t B, int64_t T, int H, int Hk, cudaStream_t stream);
 static bool bwd64_off() {
@@ -350,13 +352,14 @@ static bool bwd64_off() {
   return off;
 }
 
-// dQ part of the backward. Returns CTDK_OK, a negative status, or 1 when not eligible.
+// dQ part of the backward. Returns CTDK_OK, a negative status, or 1 when not eligible. `beside`: directly behind
+// attn_bwd_dkv_tcgen05 in the stream.
 int attn_bwd_dq_tcgen05(const float* qkv, const float* dout, const float* lse, const float* delta, float* dqkv,
-                        int64_t B, int64_t T, int H, int Hk, int D, cudaStream_t stream) {
+                        int64_t B, int64_t T, int H, int Hk, int D, bool beside, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(qkv) & 15u) || (reinterpret_cast<uintptr_t>(dout) & 15u) ||
       (reinterpret_cast<uintptr_t>(dqkv) & 15u))
     return 1;
-  if (D == 64 && !bwd64_off()) return attn_bwd_dq_tc64(qkv, dout, lse, delta, dqkv, B, T, H, Hk, stream);
+  if (D == 64 && !bwd64_off()) return attn_bwd_dq_tc64(qkv, dout, lse, delta, dqkv, B, T, H, Hk, beside, stream);
   BwdArgs a;
   a.lse = lse;
   a.delta = delta;
@@ -369,7 +372,7 @@ int attn_bwd_dq_tcgen05(const float* qkv, const float* dout, const float* lse, c
   a.scale = 1.0f / sqrtf(static_cast<float>(D));
   a.status = device_status_word();
   if (a.status == nullptr) return fail(CTDK_ELAUNCH, "attn_bwd(tcgen05): no status word");
-  return D == 64 ? launch_dq<64, 64, 2, 2, false>(qkv, dout, a, B, stream) : launch_dq<128, 64, 1, 2, true>(qkv, dout, a, B, stream);
+  return D == 64 ? launch_dq<64, 64, 2, 2, false>(qkv, dout, a, B, beside, stream) : launch_dq<128, 64, 1, 2, true>(qkv, dout, a, B, beside, stream);
 }
 
 // ----------------------------------------------------------------------------------------
@@ -430,6 +433,7 @@ __global__ void __launch_bounds__(DkvCfg<D, TQB, NB, VT>::kThreads, 1)
   uint64_t* v_ready = bars + 15;    // 1    VT: ... and has been copied to tensor memory (NCW arrivals)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
 
+  pdl_launch();   // the dQ kernel, which goes on without another wait: this one is launched the ordinary way
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // One-dimensional grid, longest items first (the first key tile of every kv head and sequence
   // meets the most query tiles).

@@ -60,7 +60,8 @@ struct Bwd64Args {
   int n_items;
   float scale;
   int* status;
-  int* work_counter;   // dK/dV kernel: next unclaimed item (zeroed before the launch)
+  int* work_counter;   // dK/dV kernel: next unclaimed item (zeroed before the launch), or null: item n gridDim.x + blockIdx.x
+  bool beside;         // dQ kernel: launched behind the dK/dV kernel, runs beside it
 };
 
 // Copies this thread's row (64 floats, 256 bytes) of a {2 x [128 rows x 128 bytes]} tile with the
@@ -179,7 +180,7 @@ __global__ void __launch_bounds__(320, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();   // inputs come from earlier kernels in the stream
+  if (!args.beside) pdl_wait();   // inputs come from earlier kernels in the stream, whose end the dK/dV kernel has seen
   const uint32_t tm_qa = tmem_base, tm_doa = tmem_base + 64u;
   // two dQ accumulators (items alternate), so that an item's result is read and stored while the
   // next item's first MMAs are already running
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(320, 1)
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  pdl_wait();   // the end of this kernel is the end of both
 }
 
 // ----------------------------------------------------------------------------------------
@@ -415,7 +417,6 @@ __global__ void __launch_bounds__(320, 1)
                           const __grid_constant__ CUtensorMap tm_kvt,   // qkv  {32, 128, 2, 1} 16-byte swizzle (K, V tiles)
                           const Bwd64Args args) {
   extern __shared__ unsigned char smem_raw[];
-  pdl_launch();
   const uint32_t raw = smem_u32(smem_raw);
   unsigned char* smem = smem_raw + ((1024u - (raw & 1023u)) & 1023u);
   unsigned char* stages = smem;                                   // [3] x {Q, dO K-major, Q, dO MN-major}
@@ -473,6 +474,7 @@ __global__ void __launch_bounds__(320, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();   // inputs come from earlier kernels in the stream
+  pdl_launch();   // the dQ kernel, which goes on without another wait
   const uint32_t tm_ka = tmem_base, tm_va = tmem_base + 64u, tm_dv = tmem_base + 128u, tm_dk = tmem_base + 192u;
   auto tm_s = [&](uint32_t g) { return tmem_base + 256u + (g & 1u) * 128u; };    // S^T, later P^T
   auto tm_dp = [&](uint32_t g) { return tmem_base + 320u + (g & 1u) * 128u; };   // dP^T, later dS^T
@@ -492,7 +494,7 @@ __global__ void __launch_bounds__(320, 1)
       for (uint32_t n = 0; ok; ++n) {
         const uint32_t slot = n & 1u;
         if (!mbar_wait_bounded(&iq_empty[slot], ((n >> 1) & 1u) ^ 1u, args.status, 50)) break;
-        int it = atomicAdd(args.work_counter, 1);
+        int it = args.work_counter != nullptr ? atomicAdd(args.work_counter, 1) : static_cast<int>(blockIdx.x + n * gridDim.x);
         if (it >= args.n_items) it = -1;
         item_q[slot] = it;
         mbar_arrive(&iq_full[slot]);
@@ -759,9 +761,9 @@ int map4(CUtensorMap* m, const float* base, int64_t width, int64_t T, int64_t B,
 
 }  // namespace
 
-// dQ part of the backward for D = 64. Returns CTDK_OK or a negative status.
+// dQ part of the backward for D = 64. Returns CTDK_OK or a negative status. `beside`: directly behind the dK/dV part in the stream.
 int attn_bwd_dq_tc64(const float* qkv, const float* dout, const float* lse, const float* delta, float* dqkv,
-                     int64_t B, int64_t T, int H, int Hk, cudaStream_t stream) {
+                     int64_t B, int64_t T, int H, int Hk, bool beside, cudaStream_t stream) {
   const int64_t RS = static_cast<int64_t>(H + 2 * Hk) * D, HD = static_cast<int64_t>(H) * D;
   Bwd64Args a;
   a.lse = lse;
@@ -778,6 +780,7 @@ int attn_bwd_dq_tc64(const float* qkv, const float* dout, const float* lse, cons
   a.scale = 1.0f / sqrtf(static_cast<float>(D));
   a.status = device_status_word();
   a.work_counter = nullptr;
+  a.beside = beside;
   if (a.status == nullptr) return fail(CTDK_ELAUNCH, "attn_bwd(tcgen05): no status word");
   CUtensorMap tq, tdo, tkv, tkm;
   int rc = map4(&tq, qkv, RS, T, B, TM, D / 32, false);
@@ -828,7 +831,10 @@ int attn_bwd_dkv_tc64(const float* qkv, const float* dout, const float* lse, con
   a.scale = 1.0f / sqrtf(static_cast<float>(D));
   a.status = device_status_word();
   if (a.status == nullptr) return fail(CTDK_ELAUNCH, "attn_bwd(tcgen05): no status word");
-  {
+  a.beside = false;
+  a.work_counter = nullptr;
+  const int sms = sm_budget();
+  if (a.n_items > sms) {
     void* cptr = nullptr;
     if (cudaGetSymbolAddress(&cptr, g_kv_work_counter) != cudaSuccess || cptr == nullptr)
       return fail(CTDK_ELAUNCH, "attn_bwd dkv(tcgen05): no work counter");
@@ -845,7 +851,6 @@ int attn_bwd_dkv_tc64(const float* qkv, const float* dout, const float* lse, con
   if (rc != CTDK_OK) return rc;
   cudaError_t e = cudaFuncSetAttribute(attn_bwd_dkv64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kKvSmem);
   if (e != cudaSuccess) return fail(CTDK_ELAUNCH, "attn_bwd dkv(tcgen05): shared memory opt-in failed: %s", cudaGetErrorString(e));
-  const int sms = sm_budget();
   launch_pdl(attn_bwd_dkv64_kernel, dim3(a.n_items < sms ? a.n_items : sms), dim3(320), kKvSmem, stream, tqk, tdok, tqm, tdom, tkvt, a);
   return check_launch("ctdk_attn_bwd(dkv, tcgen05)");
 }
