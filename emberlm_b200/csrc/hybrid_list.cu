@@ -10,6 +10,9 @@
 // The rows come straight from L2 here and not through the ring of token_ring.cuh as in the sandwich layers: half of a token's
 // weights belong to experts that are only known when they are needed, and the items want the registers and the warps
 // (detatar-0.6b, 1000 + 64 tokens: 106 ms, 116 with the ring and eight warps).
+// What bounds it is registers: 16 warps leave 128 a thread, and what the phases spill comes back from L2. A second row in
+// flight (102 ms against 95), the rows of two experts at once (98 against 97), an expert per warp (97.6 against 95) and items
+// out of line all cost more than they gave.
 #include <cfloat>
 #include <type_traits>
 
@@ -924,10 +927,11 @@ __global__ void __launch_bounds__(kListThreads, 1) hybrid_list_kernel(const __gr
           atomicMax(&words[t & 1], best);
         }
       }
-      if (ph.prefetch >= 0) prefetch_phase<T>(a.phases[ph.prefetch]);
       cp_async_wait<0>();
       if (i + 1 == a.n_phases && a.out_tokens == nullptr) break;   // logits are complete at the end of the kernel
       grid_arrive<kListWarps>(a.sync, epoch);
+      // requests while the others arrive: in front of the arrival they were 1000 to 6000 cycles of every phase
+      if (ph.prefetch >= 0) prefetch_phase<T>(a.phases[ph.prefetch]);
       if (!(alive = grid_wait<kListWarps>(a.sync, a.status, 91, epoch))) break;
     }
     if (!alive || a.out_tokens == nullptr) break;

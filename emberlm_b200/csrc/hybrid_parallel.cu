@@ -316,18 +316,19 @@ int HybridDecoder<T>::build_parallel_phases() {
     const int64_t out_ld = br.ld_o;
     if (latent) {
       const int64_t esize = static_cast<int64_t>(sizeof(T));
-      TokenPhase q = list();   // queries; the position's cache row
+      TokenPhase q = list();   // queries
       items(q, kTokLatentKeys, 0);
       add_gemv(q, at<T>(br.w_uq), tq, static_cast<int64_t>(br.heads) * (br.dim + br.rot_dim), br.ld_uq, 0);
       if (moe) expert_up(q, br.ld_uq);   // one warp chooses while the others go on
       add_op(q, kOpRmsNorm, 0, br.q_rank, br.ld_uq, tproj + br.col_q, nullptr, vec(br.q_norm));
-      add_op(q, kOpLatentStore, 0, 0, 0, nullptr);
       phases.push_back(q);
 
       const int key_cols = 16 * (16 / static_cast<int>(sizeof(T)));
-      TokenPhase k = list();   // queries against the cache rows
+      TokenPhase k = list();   // queries against the cache rows; the position's cache row, by a CTA behind those with rows (next to the
+                                 // choice of the experts it was 5000 cycles longer than any other CTA's phase)
       items(k, kTokLatentKeys, br.heads * ((t.rot_col + key_cols - 1) / key_cols));
       down(k, 0);
+      add_op(k, kOpLatentStore, 0, 0, 0, nullptr);
       need(kListThreads / 16 * (key_cols + 1));
       k.extra[0] = at<T>(br.w_ukv);
       k.extra_bytes[0] = static_cast<int64_t>(br.row_uv) * br.ld_ukv * esize;
