@@ -316,7 +316,7 @@ int HybridDecoder<T>::finish_phases() {
   if (m.arrangement == Arrangement::kParallel) {
     token_smem = static_cast<size_t>(stage_floats) * 4;
     CTDK_REQUIRE(token_smem <= 200 * 1024, "hybrid decoder: the token pass needs %zu bytes of shared memory", token_smem);
-    list_plan<T>(phases.data(), n, token_ctas);
+    list_plan<T>(phases.data(), n, m.width, token_ctas);
     return list_grid<T>(token_smem, &token_ctas);
   }
   ring.stage_floats = std::max(stage_floats, token_items(phases.data(), n, &ring.item_at));

@@ -84,8 +84,8 @@ __device__ __forceinline__ void stage_shift_norm(const TokenArgs& a, const Token
   extern __shared__ __align__(16) float sm[];
   constexpr int U = V == 4 ? 1 : 2;   // turns in flight
   const TokenShift& f = ph.shift;
-  const int W = a.width, gs = W / f.groups, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int g0 = wid / f.wpg, gstep = kListWarps / f.wpg, wj = wid % f.wpg, step = 32 * V * f.wpg;
+  const int W = a.width, gs = f.gs, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int g0 = quotient(wid, f.wpg, f.wpg_inv), gstep = f.gstep, wj = wid - g0 * f.wpg, step = 32 * V * f.wpg;
   const bool active = g0 < gstep, writer = blockIdx.x == 0, shifted = f.shift != nullptr;
   const bool known = known_id(a, tok);
   const T* e = ph.first_token ? static_cast<const T*>(a.embed) + (known ? tok * a.ld_embed : 0) : nullptr;
@@ -265,11 +265,12 @@ __device__ __noinline__ void stage_list(const TokenArgs& a, const TokenPhase& ph
       const int n4 = op.n >> 2;   // ld: number of experts; an identity output's columns are not read
       batched<2>(ph.route_top * n4, threadIdx.x, kListThreads,
                  [&](int c) {
-                   const float* g = op.src + 8 * (c / n4) * n4 + 4 * (c % n4);
+                   const float* g = op.src + 4 * (c + quotient(c, n4, op.quad_inv) * n4);
                    return Pair4{ldg4(g), ldg4(g + 4 * n4)};
                  },
                  [&](int c, const Pair4& v) {
-                   const float w = routed.index[c / n4] < op.ld ? routed.weight[c / n4] : 0.0f;
+                   const int k = quotient(c, n4, op.quad_inv);
+                   const float w = routed.index[k] < op.ld ? routed.weight[k] : 0.0f;
                    store4(xs + 4 * c, make_float4(w * silu_f(v.a.x) * v.b.x, w * silu_f(v.a.y) * v.b.y, w * silu_f(v.a.z) * v.b.z,
                                                   w * silu_f(v.a.w) * v.b.w));
                  });
@@ -335,9 +336,9 @@ __device__ __forceinline__ float gemv_row(const TokenGemv& g, int r, const float
   const T* W = static_cast<const T*>(g.W);
   if (g.mode == kGemvPlain) return row_dot<T>(W + static_cast<int64_t>(r) * g.K, sm + g.in, g.K, part, wpr);
   if (g.mode == kGemvExpertUp) {
-    const int e = routed.index[r / g.per];
+    const int k = quotient(r, g.per, g.per_inv), e = routed.index[k];
     if (e >= g.experts) return 0.0f;
-    return row_dot<T>(W + (static_cast<int64_t>(e) * g.pitch + r % g.per) * g.K, sm + g.in, g.K, part, wpr);
+    return row_dot<T>(W + (static_cast<int64_t>(e) * g.pitch + r - k * g.per) * g.K, sm + g.in, g.K, part, wpr);
   }
   float v = 0.0f;
   for (int k = 0; k < g.top; ++k) {
@@ -356,8 +357,8 @@ __device__ __forceinline__ float gemv_row(const TokenGemv& g, int r, const float
 template <typename T>
 __device__ __forceinline__ void wkv_item(const TokenPhase& ph, const TokenBranch& br, int item, int pos) {
   extern __shared__ __align__(16) float sm[];
-  const int nb = (br.dim + 31) / 32, h = item / nb, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int dim = br.dim, c = (item % nb) * 32 + lane, rw = (br.rank_w + 7) & ~7;
+  const int nb = (br.dim + 31) / 32, h = quotient(item, nb, br.item_inv), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int dim = br.dim, c = (item - h * nb) * 32 + lane, rw = (br.rank_w + 7) & ~7;
   float *low = sm, *q = low + rw, *k = q + dim, *g = k + dim, *b = g + dim, *red = b + dim;
   const bool live = c < dim;
   float* S = br.state + static_cast<int64_t>(h) * dim * dim + c;
@@ -413,7 +414,7 @@ template <typename T>
 __device__ __forceinline__ void latent_keys_item(const TokenBranch& br, int item, int pos) {
   extern __shared__ __align__(16) float sm[];
   constexpr int N = Chunk<T>::kN, COLS = kKeyCols<T>;
-  const int nb = (br.rot_col + COLS - 1) / COLS, h = item / nb, r0 = item % nb * COLS;
+  const int nb = (br.rot_col + COLS - 1) / COLS, h = quotient(item, nb, br.item_inv), r0 = (item - h * nb) * COLS;
   const int cg = threadIdx.x & 15, dg = threadIdx.x >> 4, col = r0 + cg * N;
   const float* q = br.q_up + h * (br.dim + br.rot_dim);
   float acc[N];
@@ -467,9 +468,11 @@ __device__ __forceinline__ void latent_keys_item(const TokenBranch& br, int item
 
 // Position ranges in use for L cached positions, and their length (whole tiles).
 __device__ __forceinline__ int latent_ranges(int L, int splits, int& per) {
-  const int tiles = (L + kLatentKeys - 1) / kLatentKeys, each = (tiles + splits - 1) / splits;
+  // (x + 1/2) / d lies half a d-th or more from every whole number, more than two roundings while x < 2^21
+  auto over = [](int x, int d) { return static_cast<int>(__fdividef(static_cast<float>(x) + 0.5f, static_cast<float>(d))); };
+  const int tiles = (L + kLatentKeys - 1) / kLatentKeys, each = over(tiles + splits - 1, splits);
   per = each * kLatentKeys;
-  return (tiles + each - 1) / each;
+  return over(tiles + each - 1, each);
 }
 
 // kLatentHeadsF32 query heads over one range of cached positions: running maximum, sum and the weighted sum
@@ -478,7 +481,7 @@ __device__ __forceinline__ void latent_scan_f32_item(const TokenBranch& br, int 
   extern __shared__ __align__(16) float sm[];
   using T = float;
   constexpr int N = Chunk<T>::kN, HB = kLatentHeadsF32, KT = kLatentKeys;
-  const int blk = item / br.splits, sp = item % br.splits;
+  const int blk = quotient(item, br.splits, br.item_inv), sp = item - blk * br.splits;
   int per;
   const int n_act = latent_ranges(pos + 1, br.splits, per);
   if (sp >= n_act) return;
@@ -585,7 +588,7 @@ __device__ __forceinline__ void latent_scan_bf16_item(const TokenBranch& br, int
   using bf16 = __nv_bfloat16;
   constexpr int HB = kLatentHeads, KT = kLatentKeys, LP = KT + 8;
   static_assert(HB == kListWarps, "a warp per head");
-  const int blk = item / br.splits, sp = item % br.splits;
+  const int blk = quotient(item, br.splits, br.item_inv), sp = item - blk * br.splits;
   int per;
   const int n_act = latent_ranges(pos + 1, br.splits, per);
   if (sp >= n_act) return;
@@ -731,7 +734,7 @@ constexpr int kOutParts = kLatentOutParts;
 template <typename T>
 __device__ __forceinline__ void latent_out_item(const TokenPhase& ph, const TokenBranch& br, int item, int pos) {
   extern __shared__ __align__(16) float sm[];
-  const int nb = (br.vdim + kLatentOutRows - 1) / kLatentOutRows, h = item / nb, r0 = item % nb * kLatentOutRows;
+  const int nb = (br.vdim + kLatentOutRows - 1) / kLatentOutRows, h = quotient(item, nb, br.item_inv), r0 = (item - h * nb) * kLatentOutRows;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, PS = br.rot_col + kAttnStats;
   int per;
   const int n_act = latent_ranges(pos + 1, br.splits, per);
@@ -769,7 +772,7 @@ __device__ __forceinline__ void latent_out_item(const TokenPhase& ph, const Toke
   {   // four columns per thread; the ranges are dealt to kOutParts groups of threads
     const int quads = br.rot_col / 4, n = quads * kOutParts;
     for (int i = threadIdx.x; i < n; i += kListThreads) {
-      const int c = i % quads * 4, first = i / quads;
+      const int first = quotient(i, quads, br.quad_inv), c = (i - first * quads) * 4;
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
       for (int s = first; s < n_act; s += kOutParts) {
@@ -824,9 +827,9 @@ __device__ unsigned long long list_phase(const TokenArgs& a, const TokenPhase& p
   int total = 0;
   for (int i = 0; i < ph.n_gemv; ++i) total += ph.gemv[i].rows;
   const int items = ph.n_branch > 0 ? ph.br[0].items : 0;
-  int cta = static_cast<int>(blockIdx.x) - items % static_cast<int>(gridDim.x);
-  if (cta < 0) cta += gridDim.x;
-  const int wpr = ph.wpr, groups = kListWarps / (wpr > 0 ? wpr : 1), part = wpr > 0 ? wid % wpr : 0;
+  int cta = static_cast<int>(blockIdx.x) - items;
+  while (cta < 0) cta += gridDim.x;
+  const int wpr = ph.wpr, groups = kListWarps >> (__ffs(wpr) - 1), part = wid & (wpr - 1);   // wpr: a power of two
   auto find = [&](int n, int& r) {
     int i = 0;
     while (n >= ph.gemv[i].rows) n -= ph.gemv[i++].rows;
@@ -849,7 +852,7 @@ __device__ unsigned long long list_phase(const TokenArgs& a, const TokenPhase& p
     }
   } else {
     for (int nb = cta * groups; nb < total; nb += gridDim.x * groups) {
-      const int n = nb + wid / wpr;
+      const int n = nb + (wid >> (__ffs(wpr) - 1));
       int r = 0;
       float v = 0.0f;
       const TokenGemv& g = ph.gemv[n < total ? find(n, r) : 0];
@@ -955,15 +958,25 @@ __global__ void __launch_bounds__(kListThreads, 1) hybrid_list_kernel(const __gr
 // Warps per row (as many as a round of the grid has to spare) and the order of the requests: every phase asks for one coming
 // phase, those with nothing to ask for run the queue one ahead.
 template <typename T>
-void list_plan(TokenPhase* phases, int n, int grid) {
+void list_plan(TokenPhase* phases, int n, int width, int grid) {
   int next = 1;
   for (int i = 0; i < n; ++i) {
     TokenPhase& p = phases[i];
     next = std::max(next, i + 1);
     while (next < n && phases[next].n_gemv == 0 && phases[next].extra[0] == nullptr) ++next;
     p.prefetch = next < n && next - i <= 3 ? next++ : -1;
+    TokenBranch& br = p.br[0];
+    auto blocks = [](int n, int of) { return (n + of - 1) / of; };
+    br.item_inv = division_factor(br.kind == kTokWkv ? blocks(br.dim, 32) : br.kind == kTokLatentKeys ? blocks(br.rot_col, kKeyCols<T>)
+                                  : br.kind == kTokLatentOut ? blocks(br.vdim, kLatentOutRows) : br.splits);
+    br.quad_inv = division_factor(br.rot_col / 4);
+    p.shift.gs = p.shift.groups > 0 ? width / p.shift.groups : 0;
+    p.shift.gstep = p.shift.wpg > 0 ? kListWarps / p.shift.wpg : 0;
+    p.shift.wpg_inv = division_factor(p.shift.wpg);
+    for (int k = 0; k < p.n_ops; ++k) p.op[k].quad_inv = division_factor(p.op[k].n / 4);
     int rows = 0, K = 0;
     for (int k = 0; k < p.n_gemv; ++k) {
+      p.gemv[k].per_inv = division_factor(p.gemv[k].per);
       rows += p.gemv[k].rows;
       K = std::max(K, p.gemv[k].K);
     }
@@ -982,8 +995,8 @@ int launch_list_kernel(const TokenArgs& a, int grid, size_t smem, cudaStream_t s
   return cooperative_launch(reinterpret_cast<const void*>(hybrid_list_kernel<T>), a, grid, kListThreads, smem, s);
 }
 
-template void list_plan<float>(TokenPhase*, int, int);
-template void list_plan<__nv_bfloat16>(TokenPhase*, int, int);
+template void list_plan<float>(TokenPhase*, int, int, int);
+template void list_plan<__nv_bfloat16>(TokenPhase*, int, int, int);
 template int list_grid<float>(size_t, int*);
 template int list_grid<__nv_bfloat16>(size_t, int*);
 template int launch_list_kernel<float>(const TokenArgs&, int, size_t, cudaStream_t);

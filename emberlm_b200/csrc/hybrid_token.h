@@ -39,6 +39,7 @@ struct TokenGemv {
   const float* h;
   RingRows ring;   // plain products pass through the weight ring
   int base;        // first row among the phase's plain rows
+  unsigned per_inv;   // division_factor(per)
 };
 
 // What a kStageList phase puts into the staged vector, in order (`at`: first float; padded with zeros to `ld`).
@@ -56,6 +57,7 @@ enum StageOpKind {
 struct StageOp {
   int kind, at, n, ld;
   const float *src, *src2, *w;
+  unsigned quad_inv;   // division_factor(n / 4)
 };
 constexpr int kMaxGemv = 6, kMaxOps = 4, kTokenMixes = 5, kMaxAsks = 2;
 
@@ -64,6 +66,8 @@ constexpr int kMaxGemv = 6, kMaxOps = 4, kTokenMixes = 5, kMaxAsks = 2;
 struct TokenShift {
   int groups, wpg, n_mix, ld, red;   // red: first float of the reduction scratch
   int vec;                           // columns can be taken four at a time
+  int gs, gstep;                     // columns of a group; groups at a time
+  unsigned wpg_inv;                  // division_factor(wpg)
   const float *x, *y1, *y2, *z1, *z2, *b1, *b2, *w, *shift, *mu[kTokenMixes];
   float *x_out, *h_out, *state;
 };
@@ -102,6 +106,7 @@ struct TokenBranch {
   int rot_dim, kv_rank, rot_col, ld_cache, ld_ukv, row_uv, splits, blocks, buffers;   // splits: most ranges (attention: per key/value head); buffers: cache tiles in flight (1 or 2)
   const void* w_ukv;
   const float *kv_norm, *q_up;   // queries [H][dim + rot_dim]
+  unsigned item_inv, quad_inv;   // division_factor of a head's items (scan: of the splits), of rot_col / 4
   void* q_abs;           // [H][ld_cache] queries against the cache rows, scaled: fp32, or two bfloat16 planes
 };
 
@@ -161,6 +166,7 @@ struct TokenArgs {
 };
 
 constexpr int kTokenSyncWords = 256;
+inline unsigned division_factor(int d) { return 0xffffffffu / static_cast<unsigned>(d > 0 ? d : 1); }   // for quotient()
 
 // Floats that the mix items need in place of the staged vector; tile_at: the first one of what is copied ahead of an item.
 int token_items(TokenPhase* phases, int n, int* tile_at);
@@ -174,7 +180,7 @@ template <typename T>
 int launch_token_kernel(const TokenArgs& a, int grid, size_t smem, cudaStream_t s);
 // The same for kStageList phases (hybrid_list.cu).
 template <typename T>
-void list_plan(TokenPhase* phases, int n, int grid);
+void list_plan(TokenPhase* phases, int n, int width, int grid);
 template <typename T>
 int list_grid(size_t smem, int* grid);
 template <typename T>
