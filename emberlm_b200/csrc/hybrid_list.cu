@@ -14,6 +14,7 @@
 // flight (102 ms against 95), the rows of two experts at once (98 against 97), an expert per warp (97.6 against 95) and items
 // out of line all cost more than they gave.
 #include <cfloat>
+#include <climits>
 #include <type_traits>
 
 #include "decode_core.h"
@@ -874,6 +875,15 @@ __device__ unsigned long long list_phase(const TokenArgs& a, const TokenPhase& p
   return best;
 }
 
+// The chosen experts' rows of the next phase, into L2 (8 MB of detatar-0.6b: 97.0 -> 95.1 ms for 1000 + 64 tokens).
+__device__ void prefetch_experts(const TokenPhase& ph, const Routed& routed) {
+  const int lines = static_cast<int>(ph.ask_bytes[0] / 128);
+  for (int l = static_cast<int>(blockIdx.x) * kListThreads + threadIdx.x; l < ph.route_top * lines; l += gridDim.x * kListThreads) {
+    const int k = quotient(l, lines, ph.ask_inv), e = routed.index[k];
+    if (e < ph.ask_experts) prefetch_l2(static_cast<const char*>(ph.ask[0]) + e * ph.ask_bytes[1] + static_cast<int64_t>(l - k * lines) * 128);
+  }
+}
+
 // Weights of a coming phase, into L2.
 template <typename T>
 __device__ void prefetch_phase(const TokenPhase& ph) {
@@ -934,6 +944,7 @@ __global__ void __launch_bounds__(kListThreads, 1) hybrid_list_kernel(const __gr
       if (i + 1 == a.n_phases && a.out_tokens == nullptr) break;   // logits are complete at the end of the kernel
       grid_arrive<kListWarps>(a.sync, epoch);
       // requests while the others arrive: in front of the arrival they were 1000 to 6000 cycles of every phase
+      if (ph.ask_experts > 0) prefetch_experts(ph, routed);
       if (ph.prefetch >= 0) prefetch_phase<T>(a.phases[ph.prefetch]);
       if (!(alive = grid_wait<kListWarps>(a.sync, a.status, 91, epoch))) break;
     }
@@ -979,6 +990,19 @@ void list_plan(TokenPhase* phases, int n, int width, int grid) {
       p.gemv[k].per_inv = division_factor(p.gemv[k].per);
       rows += p.gemv[k].rows;
       K = std::max(K, p.gemv[k].K);
+    }
+    p.ask_experts = 0;
+    bool chooses = false;
+    for (int k = 0; k < p.n_ops; ++k) chooses |= p.op[k].kind == kOpRoute;
+    for (int k = 0; chooses && i + 1 < n && k < phases[i + 1].n_gemv; ++k) {
+      const TokenGemv& g = phases[i + 1].gemv[k];
+      const int64_t row = g.K * static_cast<int64_t>(sizeof(T)), bytes = g.rows * row / 128 * 128;
+      if (g.mode != kGemvExpertDown || bytes == 0 || bytes * g.top / 128 > INT32_MAX) continue;
+      p.ask[0] = g.W;
+      p.ask_bytes[0] = bytes;
+      p.ask_bytes[1] = g.pitch * row;
+      p.ask_experts = g.experts;
+      p.ask_inv = division_factor(static_cast<int>(bytes / 128));
     }
     p.wpr = 1;
     while (p.wpr < 8 && static_cast<int64_t>(rows) * p.wpr * 2 <= static_cast<int64_t>(grid) * 8 && K * static_cast<int>(sizeof(T)) / 16 >= 64 * p.wpr) p.wpr *= 2;

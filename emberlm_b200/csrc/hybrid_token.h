@@ -126,6 +126,8 @@ struct alignas(16) TokenPhase {
   int64_t extra_bytes[kMaxAsks];
   const void* ask[kMaxAsks];     // those of the next phase: requested into L2 by this one
   int64_t ask_bytes[kMaxAsks];
+  int ask_experts;       // kStageList phases that choose experts: how many there are, those of the next phase's rows lie ask_bytes[1] apart;
+  unsigned ask_inv;      // ask: the first one, ask_bytes[0] bytes long, division_factor(ask_bytes[0] / 128). 0: none
   int first_token;       // kStageNorm: x comes from the embedding
   const float *x, *y, *y2, *w_y, *w_y2, *w_post, *w_pre;
   float* x_out;

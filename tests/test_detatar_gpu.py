@@ -359,3 +359,19 @@ def test_trace_replay(folder, tmp_path, dtype):
     for step, want in ((0, za[[0, 40]]), (2, za[[49, 43]]), (3, zb[[2]]), (4, zb[[19]])):
         got = np.fromfile(tmp_path / f"{step}.f32", np.float32).reshape(-1, V)
         assert hc.error(got, want) <= lim, step
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_ranges_of_the_cache(dtype):
+    """Tokens on both sides of the position where a range of the cache goes from one tile to two (96 ranges of 32 rows), and of
+    whole tiles before it."""
+    cfg = dc.model(40, 24, [dc.latent(2, 8, 4, 8, 16, 8, mlp=dc.moe(5, 3, 20, identity=1))])
+    w = dc.weights(cfg, 131)
+    t = hc.tokens(cfg, 3110, 132)
+    want = od.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype, max_seq=3110, max_portion=3110)
+    for at in (30, 3068, 3100):
+        dec.reset()
+        dec.extend(t[:at])
+        got = portions(dec, t[at:at + 9], [1])
+        assert hc.error(got, want[at:at + 9]) <= LIMIT[dtype], at
