@@ -6,7 +6,7 @@
 // fp32 behind grid barriers, and every CTA stages (and norms) its own copy. All waits are bounded.
 // What bounds a phase (10 000 to 16 000 cycles; its weights would take 3000) is its dependent chain: the barrier (3200 cycles),
 // the norms (2500 to 3500) or the merging of the key ranges (7400), the products (800 a turn), the mix items (10 000).
-// zutalix-0.6b, 300 + 64 tokens: 109.4 -> 65.0 ms against sixteen warps that took the rows from L2 and the items' inputs behind
+// zutalix-0.6b, 300 + 64 tokens: 109.4 -> 64.5 ms against sixteen warps that took the rows from L2 and the items' inputs behind
 // the barrier. The items' keys, states and gate rows are on their way before it now, and a phase's description one phase ahead.
 #include <cfloat>
 
@@ -829,7 +829,6 @@ __global__ void __launch_bounds__(kRingThreads + 32, 1) hybrid_token_kernel(cons
           atomicMax(&words[t & 1], best);
         }
       }
-      ask_items(ph);
       cp_async_wait<0>();
       if (i + 1 == a.n_phases && a.out_tokens == nullptr) break;   // logits are complete at the end of the kernel
       grid_arrive(a.sync, epoch);
@@ -837,6 +836,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 1) hybrid_token_kernel(cons
         const MixItem it = request_item<T>(ph_s[slot], pos, sm + a.item_at);   // the staged vector has been read
         if (threadIdx.x == 0) s_mix = it;
       }
+      ask_items(ph);   // in front of the arrival it was 400 cycles of every phase (65.8 ms against 64.5)
       if (!(alive = grid_wait(a.sync, a.status, 91, epoch))) break;
     }
     if (!alive || a.out_tokens == nullptr) break;
