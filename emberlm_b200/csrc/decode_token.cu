@@ -11,8 +11,8 @@
 // each, so the instructions of the chain are what the rest of a phase costs: one body for all products, a row per warp whose
 // sum leaves without another barrier, a RMSNorm factor that is applied to the finished sums, no integer divisions (200
 // cycles each) and nothing in local memory (the ring leaves 28 KB of L1).
-// Qwen3-0.6B, 256 + 128 tokens: 109.3 -> 88.6 ms against sixteen warps with the weights in registers and plain stores of the
-// words; SmolLM2-135M, 37 + 48: 26.2 -> 22.0; SmolLM2-360M, 700 + 16 single steps: 17.6 -> 14.3.
+// Qwen3-0.6B, 256 + 128 tokens: 109.3 -> 90.2 ms against sixteen warps with the weights in registers and plain stores of the
+// words; SmolLM2-135M, 37 + 48: 26.2 -> 20.4; SmolLM2-360M, 700 + 16 single steps: 17.6 -> 14.0.
 //
 // Why a buffer can be overwritten without an acknowledgement: every CTA owns at least one row of each
 // product (token_grid), so a complete vector implies that every CTA has finished the phase that read the
@@ -159,9 +159,8 @@ __device__ __forceinline__ void request_weights(const TokenKernelArgs& a, const 
     }
 }
 
-// Keys and values of kTileBytes stand in shared memory at a time.
-constexpr int kTileBytes = 32768;
-__device__ __forceinline__ constexpr int tile_keys(int D) { return kTileBytes / (8 * D); }
+// Keys and values of TILE bytes stand in shared memory at a time, in two places: one tile is on its way while the other is read.
+__device__ __forceinline__ constexpr int tile_keys(int D, int TILE) { return TILE / (8 * D); }
 
 // Key ranges per kv head for L keys: of about kRangeKeys, as far as there are CTAs. A range more costs little, a merge is one
 // hand-over, and the scores and sums of 16 keys take a CTA about 1000 cycles: SmolLM2-135M with 37 to 85 keys on one CTA per
@@ -187,26 +186,30 @@ struct Item {
   }
 };
 
-// Cached keys and values of n positions from j0 on into the tile ([tile_keys][D] keys, then values). The row of the new
-// position comes from the QKV product.
-__device__ __forceinline__ void request_tile(const TokenKernelArgs& a, float* tile, int l, int hk, int j0, int n) {
-  const int64_t at = ((static_cast<int64_t>(l) * a.Hk + hk) * a.max_seq + j0) * a.D;
+// Tile number n of an item, into its place ([tile_keys][D] keys, then values): always one group of copies, empty behind the
+// last tile. The row of the new position comes from the QKV product.
+template <int D, int TILE>
+__device__ __forceinline__ void request_tile(const TokenKernelArgs& a, float* tiles, int l, const Item& it, int pos, int n) {
+  constexpr int kKeys = tile_keys(D, TILE);
+  const int j = it.j0 + n * kKeys, floats = min(kKeys, min(it.j1, pos) - j) * D;
+  const int64_t at = ((static_cast<int64_t>(l) * a.Hk + it.hk) * a.max_seq + j) * D;
   const float *k = a.kcache + at, *v = a.vcache + at;
+  float* tile = tiles + (n & 1) * (TILE / 4);
 #pragma unroll 2
-  for (int i = 4 * threadIdx.x; i < n * a.D; i += 4 * kThreads) {
+  for (int i = 4 * threadIdx.x; i < floats; i += 4 * kThreads) {
     cp_async16(tile + i, k + i);
-    cp_async16(tile + kTileBytes / 8 + i, v + i);
+    cp_async16(tile + TILE / 8 + i, v + i);
   }
   cp_async_commit();
 }
 
-// Attention of the new row for one item, whose first tile has been requested: results as words of the attention vector
+// Attention of the new row for one item, whose first two tiles have been requested: results as words of the attention vector
 // (one range) or of the range. Threads: 16 per key for the scores; for the weighted sums a warp per 32 columns of a head
 // and share of the keys.
-template <int DC>
+template <int DC, int TILE>
 __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, const Item it, int splits, int pos, unsigned e, int64_t wqn, int64_t wkn,
-                                            float* sm, float* tile) {
-  constexpr int D = 32 * DC, kKeys = tile_keys(D), kHeadsAtOnce = kWarps / DC;
+                                            float* sm, float* tiles) {
+  constexpr int D = 32 * DC, kKeys = tile_keys(D, TILE), kHeadsAtOnce = kWarps / DC;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = a.group;
   Patience p(a);
   const bool has_new = pos >= it.j0 && pos < it.j1;
@@ -280,16 +283,17 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
     const int h = g0 + blk / DC, col = blk % DC * 32 + lane;
     float m = -FLT_MAX, s = 0.0f, o = 0.0f;
 #pragma unroll 1
-    for (int j = it.j0; j < it.j1; j += kKeys) {
+    for (int j = it.j0, number = 0; j < it.j1; j += kKeys, ++number) {
       const int n = min(kKeys, it.j1 - j);
-      cp_async_wait_all();
+      float* const tile = tiles + (number & 1) * (TILE / 4);
+      cp_async_wait<1>();
       ring_sync();
       if (pos >= j && pos < j + n) {
-        if (threadIdx.x < 2 * D) tile[(threadIdx.x < D ? 0 : kTileBytes / 8) + (pos - j) * D + (threadIdx.x & (D - 1))] = kn[threadIdx.x];
+        if (threadIdx.x < 2 * D) tile[(threadIdx.x < D ? 0 : TILE / 8) + (pos - j) * D + (threadIdx.x & (D - 1))] = kn[threadIdx.x];
         ring_sync();
       }
 #pragma unroll 1
-      for (int key = threadIdx.x >> 4; key < kKeys; key += kThreads / 16) {
+      for (int key = threadIdx.x >> 4; (key & ~1) < n; key += kThreads / 16) {   // whole warps
         const int t = threadIdx.x & 15;
         const float4* k4 = reinterpret_cast<const float4*>(tile + (key < n ? key : 0) * D) + t;
         float4 k[DC / 2];
@@ -320,17 +324,19 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
           m = most;
           s = s * fix + warp_sum(w);
           o *= fix;
-          const float* v = tile + kTileBytes / 8 + first * D + col;
+          const float* v = tile + TILE / 8 + first * D + col;
 #pragma unroll 4
           for (int i = 0; i < count; ++i) o = fmaf(__shfl_sync(0xffffffffu, w, i), v[i * shares * D], o);
         }
       }
-      const bool more = j + kKeys < it.j1;
-      if (more || g0 + kHeadsAtOnce < G) {   // the tile is read again or written anew
-        ring_sync();
-        const int next = more ? j + kKeys : it.j0;
-        request_tile(a, tile, l, it.hk, next, min(kKeys, min(it.j1, pos) - next));
-      }
+      const bool more = j + 2 * kKeys < it.j1;
+      if (more) ring_sync();   // this place has been read
+      request_tile<D, TILE>(a, tiles, l, it, more ? pos : 0, number + 2);
+    }
+    if (g0 + kHeadsAtOnce < G) {
+      ring_sync();
+      request_tile<D, TILE>(a, tiles, l, it, pos, 0);
+      request_tile<D, TILE>(a, tiles, l, it, pos, 1);
     }
     if (shares > 1) {
       scr[wid * 34 + 2 + lane] = o;
@@ -387,7 +393,7 @@ struct PhaseRows {
   int first, count;   // of this CTA
 };
 
-template <int DC>
+template <int DC, int TILE>
 __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_constant__ TokenKernelArgs a) {
   // two places for the vector or the attention's scratch, the attention's tile, this CTA's residual rows, the ring
   extern __shared__ __align__(128) float sm[];
@@ -398,7 +404,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
   __shared__ TokenLayer s_layer[kTokenMaxLayers];
   constexpr int D = 32 * DC;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, hid = a.hid;
-  float *const tile = sm + a.stage_floats, *const res = tile + kTileBytes / 4;
+  float *const tile = sm + a.stage_floats, *const res = tile + 2 * TILE / 4;
   Ring ring(reinterpret_cast<char*>(res + a.residual_floats), s_bar, a.stages, a.stage_bytes, a.sync, a.status);
   if (threadIdx.x == 0) ring.init();
   if (threadIdx.x < 5) {
@@ -438,7 +444,8 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
       for (int step = 0; step <= 4 * a.L; ++step) {
         const int j = step == 4 * a.L ? 4 : step & 3, l = min(step >> 2, a.L - 1);   // QKV, O, gate|up, down; the head
         if (j == 0 && static_cast<int>(blockIdx.x) < items) {   // cached rows, under the QKV product
-          request_tile(a, tile, l, mine.hk, mine.j0, min(tile_keys(D), min(mine.j1, pos) - mine.j0));
+          request_tile<D, TILE>(a, tile, l, mine, pos, 0);
+          request_tile<D, TILE>(a, tile, l, mine, pos, 1);
         }
         if (j == 1) {   // attention of the new row
 #pragma unroll 1
@@ -447,9 +454,10 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
             Item it = mine;
             if (item >= static_cast<int>(gridDim.x)) {
               it = Item(item, splits, pos + 1);
-              request_tile(a, tile, l, it.hk, it.j0, min(tile_keys(D), min(it.j1, pos) - it.j0));
+              request_tile<D, TILE>(a, tile, l, it, pos, 0);
+              request_tile<D, TILE>(a, tile, l, it, pos, 1);
             }
-            if (!attention_item<DC>(a, l, it, splits, pos, e, s_layer[l].wqn, s_layer[l].wkn, sm, tile)) return false;
+            if (!attention_item<DC, TILE>(a, l, it, splits, pos, e, s_layer[l].wqn, s_layer[l].wkn, sm, tile)) return false;
           }
           if (splits > 1) {
             // columns are dealt from the last CTA on (the first ones have the items)
@@ -573,26 +581,29 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
 }
 
 using Kernel = void (*)(TokenKernelArgs);
-Kernel kernel_of(int D) {
-  return D == 64 ? token_kernel<2> : token_kernel<4>;
+constexpr int kTileBytes[2] = {32768, 16384};   // of a place
+Kernel kernel_of(int D, int tile) {
+  if (tile == kTileBytes[0]) return D == 64 ? token_kernel<2, kTileBytes[0]> : token_kernel<4, kTileBytes[0]>;
+  return D == 64 ? token_kernel<2, kTileBytes[1]> : token_kernel<4, kTileBytes[1]>;
 }
 // Lays the shared memory out: two places for the vector where they leave room for the ring, else one; pieces of up to 32
 // kLaneChunks chunks, less where that does not leave room for three stages. Returns its size, 0 when there is no room.
-size_t plan(TokenKernelArgs& a, int grid) {
+size_t plan(TokenKernelArgs& a, int grid, int tile, int* places, int* piece) {
   constexpr int64_t kRoom = 227 * 1024 - 4096;   // the kernel's own arrays take 3.1 KB
   const int64_t vector = (std::max(std::max(a.hid, a.H * a.D), a.I) + 31) / 32 * 32, G = a.H / a.Hk;
-  const int64_t attn = G * (a.D + kTileBytes / (8 * a.D)) + kWarps * 34 + 2 * a.D;
+  const int64_t attn = G * (a.D + tile / (8 * a.D)) + kWarps * 34 + 2 * a.D;
   a.group = static_cast<int>(G);
+  a.tile_bytes = tile;
   a.residual_floats = (ceil_div(a.hid, grid) + 31) / 32 * 32;
   const int K[5] = {a.hid, a.H * a.D, a.hid, a.I, a.hid};
-  for (int places = 2; places >= 1; --places) {
-    a.vector_floats = places == 2 ? static_cast<int>(vector) : 0;
-    a.stage_floats = static_cast<int>((std::max(places * vector, attn) + 31) / 32 * 32);
-    const int64_t front = (a.stage_floats + a.residual_floats) * int64_t{4} + kTileBytes;
-    for (int piece = 32 * kLaneChunks; piece >= 32; piece /= 2) {
+  for (*places = 2; *places >= 1; --*places) {
+    a.vector_floats = *places == 2 ? static_cast<int>(vector) : 0;
+    a.stage_floats = static_cast<int>((std::max(*places * vector, attn) + 31) / 32 * 32);
+    const int64_t front = (a.stage_floats + a.residual_floats) * int64_t{4} + 2 * tile;
+    for (*piece = 32 * kLaneChunks; *piece >= 32; *piece /= 2) {
       a.stage_bytes = 0;
       for (int j = 0; j < 5; ++j) {
-        a.product[j] = ring_rows(K[j] / 4, piece);
+        a.product[j] = ring_rows(K[j] / 4, *piece);
         a.stage_bytes = std::max(a.stage_bytes, ring_stage_bytes(a.product[j]));
       }
       a.stages = static_cast<int>(std::min<int64_t>((kRoom - front) / a.stage_bytes, kRingMaxStages));
@@ -600,6 +611,16 @@ size_t plan(TokenKernelArgs& a, int grid) {
     }
   }
   return 0;
+}
+// Places of 32 KB where they take neither a place of the vector nor a shorter piece nor the fourth stage from the ring, else of
+// 16 KB. Qwen3-0.6B, 4000 + 32 tokens: 46.3 ms with the large ones, 49.7 with the small ones, 49.1 with one place of 32 KB;
+// Llama-3.2-1B, 2000 + 16 tokens (shorter pieces with the large ones): 28.2, 23.7 and 23.7.
+size_t plan(TokenKernelArgs& a, int grid) {
+  int places[2], piece[2];
+  const size_t small = plan(a, grid, kTileBytes[1], &places[1], &piece[1]);
+  const size_t large = plan(a, grid, kTileBytes[0], &places[0], &piece[0]);
+  if (large != 0 && places[0] == places[1] && piece[0] == piece[1] && a.stages >= 4) return large;
+  return small == 0 ? 0 : plan(a, grid, kTileBytes[1], &places[1], &piece[1]);
 }
 int64_t padded(int64_t n) { return (n + 31) / 32 * 32; }
 
@@ -629,7 +650,7 @@ int token_grid(const TokenKernelArgs& args) {
   // every CTA owns at least one row of each product (the protocol needs that)
   const int grid = std::min(std::min(std::min(sm_count(), kTokenMaxGrid), a.hid), std::min(std::min(a.I, a.QKVN), a.V));
   const size_t smem = plan(a, grid);
-  const void* k = reinterpret_cast<const void*>(kernel_of(D));
+  const void* k = reinterpret_cast<const void*>(kernel_of(D, a.tile_bytes));
   if (smem == 0 || cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
       coop == 0 || raise_dynamic_smem(k, smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads + 32, smem) != cudaSuccess || per_sm < 1) {
@@ -650,7 +671,7 @@ int token_launch(TokenKernelArgs& a, Word* words, int grid, cudaStream_t s) {
   if (cudaMemsetAsync(words, 0, bytes, s) != cudaSuccess || cudaMemsetAsync(a.sync, 0, 16 * sizeof(unsigned int), s) != cudaSuccess)
     return fail(CTDK_ELAUNCH, "decode: clearing the exchange words failed");
   void* params[] = {&a};
-  const cudaError_t err = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel_of(a.D)), dim3(grid), dim3(kThreads + 32), params,
+  const cudaError_t err = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel_of(a.D, a.tile_bytes)), dim3(grid), dim3(kThreads + 32), params,
                                                       smem, s);
   if (err != cudaSuccess) return fail(CTDK_ELAUNCH, "decode: cooperative launch failed: %s", cudaGetErrorString(err));
   return check_launch("decode token kernel");

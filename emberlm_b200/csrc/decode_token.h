@@ -31,6 +31,7 @@ struct TokenKernelArgs {
   Word *x, *hm, *qkv, *part, *attn, *act, *best;
   RingRows product[5];         // QKV, O, gate|up, down, head
   int vector_floats, stage_floats, residual_floats, stages, stage_bytes;   // shared memory: a place of the vector (0: there is one only), ...
+  int tile_bytes;   // of a place for cached keys and values, of which there are two
   int64_t* cur_token;
   int* counters;
   unsigned int* sync;          // [2]: abort flag

@@ -320,7 +320,7 @@ int HybridDecoder<T>::finish_phases() {
     return list_grid<T>(token_smem, &token_ctas);
   }
   ring.stage_floats = std::max(stage_floats, token_items(phases.data(), n, &ring.item_at));
-  CTDK_REQUIRE(ring.stage_floats <= 50 * 1024, "hybrid decoder: the token pass needs %d bytes of shared memory", ring.stage_floats * 4);
+  CTDK_REQUIRE(stage_floats <= 50 * 1024, "hybrid decoder: the token pass needs %d bytes of shared memory", stage_floats * 4);
   token_smem = token_plan<T>(phases.data(), n, token_ctas, ring, products);
   CTDK_REQUIRE(token_smem > 0, "hybrid decoder: no room for the weight ring behind %d floats", ring.stage_floats);
   CTDK_REQUIRE(products.size() <= static_cast<size_t>(max_products), "hybrid decoder: too many products");

@@ -233,3 +233,22 @@ def test_token_pass_over_few_keys_and_long_rows(case, context, inter):
     dec.extend(prompt)
     for token, want in zip(got[:-1], ref[1:]):
         assert np.abs(dec.step(int(token)).cpu().numpy() - want).max() <= limit
+
+
+@pytest.mark.parametrize("heads, kv_heads, dim, contexts", [(48, 48, 64, (190, 195, 390)), (96, 16, 64, (570, 640)), (48, 48, 128, (94, 100, 290)),
+                                                            (96, 24, 128, (190, 300))])
+def test_ranges_of_several_tiles(heads, kv_heads, dim, contexts):
+    """Many key/value heads leave few CTAs for each, so that a range of keys is longer than one and two tiles (32 or 64 keys, of
+    128 values half as many), also with more query heads than are taken at once; tolerance as above."""
+    from emberlm_b200 import engine as E
+    kw = dict(CASES[0], num_hidden_layers=1, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=dim)
+    ocfg, ecfg, params = build(kw, 65)
+    prompt = np.random.default_rng(heads).integers(0, ocfg.vocab_size, size=max(contexts) + 3)
+    ref = om.forward_logits(params, ocfg, prompt[None, :], acc=np.float64)[0]
+    dec = E.Decoder(ecfg, max_seq_len=max(contexts) + 8)
+    dec.load_parameters(params)
+    for context in contexts:
+        dec.reset()
+        dec.extend(prompt[:context])
+        for i in range(context, context + 3):
+            assert np.abs(dec.step(int(prompt[i])).cpu().numpy() - ref[i]).max() <= 5e-3 * max(np.abs(ref[i]).max(), 1.0), (context, i)
