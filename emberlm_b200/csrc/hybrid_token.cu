@@ -325,6 +325,9 @@ struct KeyTile {
   }
 };
 
+// Floats of partial sums: of the warps' shares of the keys, or of the blocks of 32 columns beyond the warps' first ones.
+inline int attention_scratch(int dim) { return std::max(kRingWarps * 34, (dim + 32 * kRingWarps - 1) / (32 * kRingWarps) * kRingThreads); }
+
 // The new token against the keys [j0, j1) of key/value head g, all query heads of the group, into the partial results of
 // the range. Keys are the values. 16 threads per key for the scores, a warp per 32 columns of a head and share of the keys
 // for the sums.
@@ -338,7 +341,7 @@ __device__ __forceinline__ void attention_item(const TokenPhase& ph, const Token
   float* qs = sm;                    // [hq][2 P] rotated, scaled
   float* kn = qs + hq * 2 * P;       // [2 P] this token's key
   float* sc = kn + 2 * P;            // [hq][32] scores
-  float* scr = sc + hq * 32;         // [kRingWarps][34]
+  float* scr = sc + hq * 32;         // [kRingWarps][34], or a float of every thread and turn (attention_scratch)
   const int slot = it.part == it.ranges - 1 ? j1 - 1 : -1;   // the last range holds the new position
 #pragma unroll 1
   for (int r = wid; r < hq + (slot >= 0 ? 1 : 0); r += kRingWarps) {
@@ -365,103 +368,111 @@ __device__ __forceinline__ void attention_item(const TokenPhase& ph, const Token
   const int nb = (dim + 31) >> 5, at_once = nb == 1 ? 8 : (nb == 2 ? 4 : (nb <= 4 ? 2 : 1));   // kRingWarps / nb
 #pragma unroll 1
   for (int g0 = 0; g0 < hq; g0 += at_once) {
-    // blocks of 32 columns; with more of them than warps a warp takes them one after the other
+    // blocks of 32 columns, a warp each, with shares of the keys where there are more warps; of a head with more blocks than
+    // warps every warp takes several, whose sums stand in `scr` between two tiles
     const int heads = min(at_once, hq - g0), blocks = heads * nb, turns = (blocks + kRingWarps - 1) / kRingWarps;
     const int sh = blocks * 8 <= kRingWarps ? 3 : (blocks * 4 <= kRingWarps ? 2 : (blocks * 2 <= kRingWarps ? 1 : 0)), shares = 1 << sh;
+    int blk = wid, share = 0, h = g0;
+    if (turns == 1) {
 #pragma unroll 1
-    for (int turn = 0; turn < turns; ++turn) {
-      int blk = turn * kRingWarps + wid, share = 0, h = g0;
-      if (turns == 1) {
+      for (; blk >= blocks; blk -= blocks) ++share;
 #pragma unroll 1
-        for (; blk >= blocks; blk -= blocks) ++share;
+      for (; blk >= nb; blk -= nb) ++h;   // blk: block of the head's columns
+    }
+    const bool takes_part = share < shares;
+    float m = -FLT_MAX, l = 0.0f, o = 0.0f;
+#pragma unroll 1
+    for (int jb = j0; jb < j1; jb += KT) {
+      const int n = min(KT, j1 - jb);
+      if (jb != j0 || g0 > 0) {
+        ring_sync();   // the tile has been read
+        if (j1 - j0 > KT) tile.request(br, g, jb, n);
       }
-      const bool mine_any = blk < blocks && share < shares;
+      cp_async_wait<0>();
+      ring_sync();
+      const int t = threadIdx.x & 15;
 #pragma unroll 1
-      for (int c = blk; mine_any && c >= nb; c -= nb, blk = c) ++h;   // blk: block of the head's columns
-      const int col = (mine_any ? blk * 32 : 0) + lane;
-      float m = -FLT_MAX, l = 0.0f, o = 0.0f;
+      for (int key = threadIdx.x >> 4; key < 32; key += kRingThreads / 16) {
+        const bool fresh = jb + key == slot;
 #pragma unroll 1
-      for (int jb = j0; jb < j1; jb += KT) {
-        const int n = min(KT, j1 - jb);
-        if (jb != j0 || g0 > 0 || turn > 0) {
-          ring_sync();   // the tile has been read
-          if (j1 - j0 > KT) tile.request(br, g, jb, n);
-        }
-        cp_async_wait<0>();
-        ring_sync();
-        if (turn == 0) {
-          const int t = threadIdx.x & 15;
+        for (int h0 = g0; h0 < g0 + heads; h0 += 4) {
+          float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+          if (key < n) {
 #pragma unroll 1
-          for (int key = threadIdx.x >> 4; key < 32; key += kRingThreads / 16) {
-          const bool fresh = jb + key == slot;
-#pragma unroll 1
-          for (int h0 = g0; h0 < g0 + heads; h0 += 4) {
-            float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (key < n) {
-#pragma unroll 1
-              for (int p = t; p < P; p += 16) {
-                const int d = 2 * p;
-                const T* row = tile.keys + key * dim + d;
-                const float u = fresh ? kn[d] : to_f(row[0]), v = fresh ? kn[d + 1] : (d + 1 < dim ? to_f(row[1]) : 0.0f);
-                const float2 rot = p < br.rot_pairs ? tile.angles[key * br.rot_pairs + p] : make_float2(1.0f, 0.0f);
-                const float x = u * rot.x - v * rot.y, y = v * rot.x + u * rot.y;
+            for (int p = t; p < P; p += 16) {
+              const int d = 2 * p;
+              const T* row = tile.keys + key * dim + d;
+              const float u = fresh ? kn[d] : to_f(row[0]), v = fresh ? kn[d + 1] : (d + 1 < dim ? to_f(row[1]) : 0.0f);
+              const float2 rot = p < br.rot_pairs ? tile.angles[key * br.rot_pairs + p] : make_float2(1.0f, 0.0f);
+              const float x = u * rot.x - v * rot.y, y = v * rot.x + u * rot.y;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                  const float2 q = *reinterpret_cast<const float2*>(qs + min(h0 + k, hq - 1) * 2 * P + d);
-                  acc[k] = fmaf(q.x, x, fmaf(q.y, y, acc[k]));
-                }
+              for (int k = 0; k < 4; ++k) {
+                const float2 q = *reinterpret_cast<const float2*>(qs + min(h0 + k, hq - 1) * 2 * P + d);
+                acc[k] = fmaf(q.x, x, fmaf(q.y, y, acc[k]));
               }
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-#pragma unroll
-              for (int x = 8; x > 0; x >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], x);
-              if (t == 0 && h0 + k < g0 + heads) sc[(h0 + k) * 32 + key] = acc[k];
-            }
           }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+#pragma unroll
+            for (int x = 8; x > 0; x >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], x);
+            if (t == 0 && h0 + k < g0 + heads) sc[(h0 + k) * 32 + key] = acc[k];
           }
-          ring_sync();
         }
-        if (mine_any) {
-          const int mine = (n - share + shares - 1) >> sh;   // keys share, share + shares, ... of the tile
-          const float d = lane < mine ? sc[h * 32 + share + lane * shares] : -FLT_MAX;
-          const float most = fmaxf(m, warp_max(d)), w = lane < mine ? expf(d - most) : 0.0f, fix = expf(m - most);
-          m = most;
-          l = l * fix + warp_sum(w);
+      }
+      ring_sync();
+      if (takes_part) {
+        const int mine = (n - share + shares - 1) >> sh;   // keys share, share + shares, ... of the tile
+        const float d = lane < mine ? sc[h * 32 + share + lane * shares] : -FLT_MAX;
+        const float most = fmaxf(m, warp_max(d)), w = lane < mine ? expf(d - most) : 0.0f, fix = expf(m - most);
+        m = most;
+        l = l * fix + warp_sum(w);
+#pragma unroll 1
+        for (int turn = 0; turn < turns; ++turn) {
+          const int col = (blk + turn * kRingWarps) * 32 + lane, c = col < dim ? col : 0;
+          if (turns > 1 && jb != j0) o = scr[turn * kRingThreads + threadIdx.x];
           o *= fix;
-          const int c = col < dim ? col : 0;
 #pragma unroll 4
           for (int i = 0; i < mine; ++i) {
             const int key = share + i * shares;
             const float v = jb + key == slot ? kn[c] : to_f(tile.keys[key * dim + c]);
             o = fmaf(__shfl_sync(0xffffffffu, w, i), v, o);
           }
-        }
-      }
-      if (shares > 1) {
-        if (mine_any) {
-          scr[wid * 34 + 2 + lane] = o;
-          if (lane == 0) *reinterpret_cast<float2*>(scr + wid * 34) = make_float2(m, l);
-        }
-        ring_sync();
-        if (mine_any && share == 0) {
-#pragma unroll 1
-          for (int k = 1; k < shares; ++k) {
-            const float* other = scr + (wid + k * blocks) * 34;
-            const float most = fmaxf(m, other[0]), f = expf(m - most), fo = expf(other[0] - most);
-            l = l * f + other[1] * fo;
-            o = o * f + other[2 + lane] * fo;
-            m = most;
+          if (turns > 1) {
+            scr[turn * kRingThreads + threadIdx.x] = o;
+            o = 0.0f;
           }
         }
       }
-      if (mine_any && share == 0 && col < dim) {
-        float* dst = br.part + (static_cast<int64_t>(g * hq + h) * kAttnSplits + it.part) * stride;
-        dst[kAttnStats + col] = o;
-        if (col == 0) {
-          dst[0] = m;
-          dst[1] = l;
+    }
+    if (shares > 1) {
+      if (takes_part) {
+        scr[wid * 34 + 2 + lane] = o;
+        if (lane == 0) *reinterpret_cast<float2*>(scr + wid * 34) = make_float2(m, l);
+      }
+      ring_sync();
+      if (takes_part && share == 0) {
+#pragma unroll 1
+        for (int k = 1; k < shares; ++k) {
+          const float* other = scr + (wid + k * blocks) * 34;
+          const float most = fmaxf(m, other[0]), f = expf(m - most), fo = expf(other[0] - most);
+          l = l * f + other[1] * fo;
+          o = o * f + other[2 + lane] * fo;
+          m = most;
         }
+      }
+    }
+    if (takes_part && share == 0) {
+      float* dst = br.part + (static_cast<int64_t>(g * hq + h) * kAttnSplits + it.part) * stride;
+#pragma unroll 1
+      for (int turn = 0; turn < turns; ++turn) {
+        const int col = (blk + turn * kRingWarps) * 32 + lane;
+        if (turns > 1) o = scr[turn * kRingThreads + threadIdx.x];   // of this thread
+        if (col < dim) dst[kAttnStats + col] = o;
+      }
+      if (blk == 0 && lane == 0) {
+        dst[0] = m;
+        dst[1] = l;
       }
     }
   }
@@ -873,7 +884,7 @@ int token_items(TokenPhase* phases, int n, int* tile_at) {
         const int64_t hq = br.H / br.G, key = br.dim * size + br.rot_pairs * 8;
         for (br.tile_keys = 32; br.tile_keys > 1 && br.tile_keys * key > kTile; br.tile_keys /= 2) {
         }
-        f = (hq + 1) * (br.dim + 1) + hq * 32 + kRingWarps * 34 + 2;
+        f = (hq + 1) * (br.dim + 1) + hq * 32 + attention_scratch(br.dim) + 2;
         t = br.tile_keys * key + 32;
       } else if (br.kind == kTokLightning) {
         f = 2 * br.dim + kRingWarps * 32;

@@ -395,3 +395,20 @@ def test_long_rows_of_the_token_pass(ff, dtype):
     want = oh.forward(cfg, w, t)
     dec = decoder(cfg, w, dtype)
     assert hc.error(portions(dec, t, [4, 1, 1, 1, 1, 1]), want) <= LIMIT[dtype]
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim, rot", [(264, 24), (264, 264), (512, 512), (512, 64), (1024, 1024), (1024, 32)])
+def test_wide_attention_heads_over_several_tiles(dim, rot, dtype):
+    """Heads with more blocks of 32 columns than the token pass has warps, single tokens on both sides of one and two tiles of
+    keys a range (8, 16 or 32 keys) with one, several and the most ranges in use (four: the lightning heads fill the other CTAs);
+    limits as above."""
+    cfg = hc.model(50, 72, [hc.parallel(hc.attention(4, 2, dim, 1000, rot), hc.lightning(140, 4, 4))])
+    w = muted(cfg, hc.weights(cfg, 101), "attention")
+    t = hc.tokens(cfg, 280, 102)
+    want = oh.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype, max_seq=280, max_portion=280)
+    for at in (7, 15, 31, 62, 127, 254, 276):
+        dec.reset()
+        dec.extend(t[:at])
+        assert hc.error(portions(dec, t[at:at + 4], [1]), want[at:at + 4]) <= LIMIT[dtype], at
