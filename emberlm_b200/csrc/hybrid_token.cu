@@ -224,7 +224,7 @@ __device__ __forceinline__ void stage_mixed(const TokenArgs& a, const TokenPhase
     } else {
       const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
       for (int h = wid; h < br.H; h += kRingWarps) {
-        constexpr int kHeld = 8;   // vdim <= 256
+        constexpr int kHeld = 8;   // 256 columns in registers, the others are read twice
         float v[kHeld], f[kHeld], t = 0.0f;
 #pragma unroll
         for (int u = 0; u < kHeld; ++u) {
@@ -233,11 +233,11 @@ __device__ __forceinline__ void stage_mixed(const TokenArgs& a, const TokenPhase
           f[u] = d < br.vdim ? br.w_norm[d] * sigmoid_f(ldg_f(br.gate + h * br.vdim + d)) : 0.0f;
           t += v[u] * v[u];
         }
-        t = warp_sum(t);
         for (int d = lane + 32 * kHeld; d < br.vdim; d += 32) {
           const float w = ldg_f(br.out + h * br.vdim + d);
-          t += warp_sum(w * w);
+          t += w * w;
         }
+        t = warp_sum(t);   // behind the loop: its trips differ between the lanes
         const float sc = rsqrtf(t / static_cast<float>(br.vdim) + a.eps);
 #pragma unroll
         for (int u = 0; u < kHeld; ++u)

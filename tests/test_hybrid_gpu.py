@@ -412,3 +412,17 @@ def test_wide_attention_heads_over_several_tiles(dim, rot, dtype):
         dec.reset()
         dec.extend(t[:at])
         assert hc.error(portions(dec, t[at:at + 4], [1]), want[at:at + 4]) <= LIMIT[dtype], at
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("vdim", [256, 257, 288, 300, 320, 520])
+def test_wide_values_of_the_delta_rule(vdim, dtype):
+    """Value heads on both sides of the 256 columns that the token pass's norm holds in registers, in whole and in broken warps;
+    limits as above."""
+    cfg = hc.model(50, 72, [hc.delta(9, 3, 16, vdim, 3)])
+    w, t = hc.weights(cfg, 111), hc.tokens(cfg, 24, 112)
+    want = oh.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype)
+    for sizes in ([24], [9, 1, 1, 1]):
+        dec.reset()
+        assert hc.error(portions(dec, t, sizes), want) <= LIMIT[dtype], sizes
