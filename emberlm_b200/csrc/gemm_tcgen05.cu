@@ -1315,7 +1315,7 @@ int gemm_3xtf32(const float*, const float*, float*, int64_t, int64_t, int64_t, i
 // where it did with three products (K > 1024, or K > 512 with accumulation; in several rounds the
 // cluster kernel does not overlap its exchange: 903 rows of SmolLM2-135M 38.4 -> 40.2 ms a step). Returns 1 from about two
 // rounds of tiles on: the paired-CTA kernel's large tiles, three times, are then faster.
-// The operands are split here, in the launch that also zeroes C where the product adds to it. Nothing is enqueued when it returns 1.
+// The operands are split here, in the launch that as a rule also zeroes C where the product adds to it. Nothing is enqueued when it returns 1.
 int gemm_split_tcgen05(const SplitOperands& ops, float* Cp, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, int transa,
                        int transb, int epilogue, const float* aux, int run, cudaStream_t stream) {
   const float *A = ops.a_hi, *A2 = ops.a_lo, *B = ops.b_hi, *B2 = ops.b_lo;
@@ -1386,7 +1386,12 @@ int gemm_split_tcgen05(const SplitOperands& ops, float* Cp, int64_t M, int64_t N
   if (rc == CTDK_OK) rc = map_a(&ta2, A2);
   if (rc == CTDK_OK) rc = map_b(&tb, B);
   if (rc == CTDK_OK) rc = map_b(&tb2, B2);
-  if (rc == CTDK_OK) rc = split_operands(ops, splits > 1 && epilogue != CTDK_EPI_ACCUMULATE ? Cp : nullptr, M, N, ldc, stream);
+  // The product reads the parts only, so C may be one of the operands: it is then zeroed behind the launch that splits them.
+  const float* c_end = Cp + (M - 1) * ldc + N;
+  const bool zero = splits > 1 && epilogue != CTDK_EPI_ACCUMULATE;
+  const bool in_place = (Cp < ops.a + ops.na && ops.a < c_end) || (Cp < ops.b + ops.nb && ops.b < c_end);
+  if (rc == CTDK_OK) rc = split_operands(ops, zero && !in_place ? Cp : nullptr, M, N, ldc, stream);
+  if (rc == CTDK_OK && zero && in_place) rc = zero_rows(Cp, M, N, ldc, stream);
   if (rc != CTDK_OK) return rc;
   // the work of the three products, as where they are launched one by one
   void* const tok = prof_begin(CTDK_PROF_GEMM, 6.0 * static_cast<double>(M) * N * K, stream);

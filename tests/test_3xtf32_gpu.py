@@ -35,6 +35,20 @@ def test_gemm_3xtf32_is_near_fp32(ta, tb, M, N, K):
     assert relmax(c.cpu().numpy(), ref + base.cpu().numpy()) < 5e-6
 
 
+@pytest.mark.parametrize("M,N,K,operand", [(1024, 1024, 1024, 0), (1024, 1024, 1024, 1), (903, 576, 576, 0), (96, 64, 64, 0)])
+def test_gemm_3xtf32_into_an_operand(M, N, K, operand):
+    """The result in the place of an operand (with two ranges of K that add to zeroes, in one range, on a cluster): the bits of a
+    product with a place of its own."""
+    from emberlm_b200 import lib, ops
+    gen = torch.Generator("cuda").manual_seed(4)
+    ab = [torch.empty(s, device="cuda").uniform_(-1, 1, generator=gen) for s in ((M, K), (K, N))]
+    want = ops.matmul(*ab, precision=lib.GEMM_3XTF32)
+    for _ in range(3):
+        mine = [t.clone() for t in ab]
+        ops.matmul(*mine, precision=lib.GEMM_3XTF32, out=mine[operand])
+        assert torch.equal(mine[operand], want)
+
+
 @pytest.mark.parametrize("B,T,H,Hk,D", [(2, 130, 4, 2, 64), (1, 200, 2, 1, 128)])
 def test_attention_3xtf32_is_near_fp32(B, T, H, Hk, D):
     from emberlm_b200 import lib, ops
