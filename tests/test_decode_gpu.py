@@ -252,3 +252,28 @@ def test_ranges_of_several_tiles(heads, kv_heads, dim, contexts):
         dec.extend(prompt[:context])
         for i in range(context, context + 3):
             assert np.abs(dec.step(int(prompt[i])).cpu().numpy() - ref[i]).max() <= 5e-3 * max(np.abs(ref[i]).max(), 1.0), (context, i)
+
+
+@pytest.mark.parametrize("gate", [-87.5, -88.0, -88.5, -40.0])
+def test_gates_at_the_edge_of_the_range(gate):
+    """Gates whose 1 + exp(-gate) lies between 2^126 and 2^128, where an approximate division gives zero, against up values that
+    make a product of ordinary size of it; tolerance as above."""
+    from emberlm_b200 import engine as E
+    ocfg, ecfg, params = build(dict(CASES[0], num_hidden_layers=1), 67)
+    hid, inter, p = ocfg.hidden_size, 256, "model.layers.0."
+    rng = np.random.default_rng(68)
+    params["model.embed_tokens.weight"][7] = 1.0   # the token's row, which reaches the gate as it is
+    params[p + "post_attention_layernorm.weight"][:] = 1.0
+    params[p + "self_attn.o_proj.weight"][:] = 0.0
+    params[p + "mlp.gate_proj.weight"][:] = gate / hid
+    params[p + "mlp.up_proj.weight"][:] = (rng.uniform(-1.0, 1.0, (inter, 1)) * (1.0 + np.exp(-gate)) / -gate / hid).astype(F32)
+    dec = E.Decoder(ecfg, max_seq_len=8)
+    dec.load_parameters(params)
+    dec.extend([7])
+    got = dec.step(7).cpu().numpy()
+    ref = om.forward_logits(params, ocfg, np.array([[7, 7]]), acc=np.float64)[0, 1]
+    silent = dict(params, **{p + "mlp.down_proj.weight": 0.0 * params[p + "mlp.down_proj.weight"]})
+    quiet = om.forward_logits(silent, ocfg, np.array([[7, 7]]), acc=np.float64)[0, 1]
+    limit = 5e-3 * max(np.abs(ref).max(), 1.0)
+    assert np.abs(quiet - ref).max() > 20 * limit
+    assert np.abs(got - ref).max() <= limit
