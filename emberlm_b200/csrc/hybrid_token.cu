@@ -589,8 +589,11 @@ struct DeltaTile {
     a2_from = static_cast<const T*>(br.w_a2) + static_cast<int64_t>(h) * br.dim * ra;
     g2_from = static_cast<const T*>(br.w_g2) + (static_cast<int64_t>(h) * br.vdim + c0) * rg;
   }
-  __device__ __forceinline__ void request(const TokenBranch& br, const MixItem& it, int pos) {
+  __device__ __forceinline__ void request_rows(const TokenBranch& br, const MixItem& it, int pos) {
     if (pos > 0) request_state(state, br.state + static_cast<int64_t>(it.head) * br.dim * br.vdim, br.dim, br.vdim, it.part * 32);
+  }
+  __device__ __forceinline__ void request(const TokenBranch& br, const MixItem& it, int pos) {
+    if (!br.state_late) request_rows(br, it, pos);
     if (br.low_staged) {
       copy16(a2, a2_from, a2_bytes >> 4);
       copy16(g2, g2_from, g2_bytes >> 4);
@@ -655,6 +658,13 @@ __device__ __forceinline__ void delta_item(const TokenPhase& ph, const TokenBran
     if ((threadIdx.x & 15) == 0 && vb * 32 + e < br.vdim) br.gate[h * br.vdim + vb * 32 + e] = z;
   }
   ring_sync();
+  if (br.state_late) {   // a1 and g1 have been read
+    tile.state = a1;
+    tile.request_rows(br, it, pos);
+    cp_async_commit();
+    cp_async_wait<0>();
+    ring_sync();
+  }
   float nq = 0.0f, nk = 0.0f;
 #pragma unroll
   for (int i = 0; i < kRingWarps; ++i) {
@@ -871,6 +881,7 @@ __global__ void __launch_bounds__(kRingThreads + 32, 1) hybrid_token_kernel(cons
 
 int token_items(TokenPhase* phases, int n, int* tile_at) {
   constexpr int64_t kTile = 64 * 1024;   // of the low-rank rows or of a tile of keys, where they are large
+  constexpr int64_t kLateFloats = 52 * 1024;   // with the shortest ring behind it 222 KB; the ranks are then 40 000 and more, a state 8192 floats
   int64_t scratch = 0, tile = 0;
   for (int i = 0; i < n; ++i) {
     phases[i].items = 0;
@@ -893,7 +904,9 @@ int token_items(TokenPhase* phases, int n, int* tile_at) {
         f = ra + rg + 3 * br.dim + 32 + 2 * kRingWarps * 32 + 2 * kRingWarps;
         const int64_t low = (br.dim * ra + 32 * rg) * size;
         br.low_staged = low <= kTile ? 1 : 0;
-        t = br.dim * 128 + (br.low_staged ? low : 0);
+        // the largest ranks leave the state no room of its own and are larger than it
+        br.state_late = f + br.dim * 32 > kLateFloats ? 1 : 0;
+        t = (br.state_late ? 0 : br.dim * 128) + (br.low_staged ? low : 0);
       }
       scratch = std::max(scratch, f);
       tile = std::max(tile, (t + 127) / 128 * 32);

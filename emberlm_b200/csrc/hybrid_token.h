@@ -96,6 +96,7 @@ struct TokenBranch {
   const float *conv_q, *conv_k, *conv_v, *a_log, *dt_bias;
   const void *w_a2, *w_g2;
   int low_staged;        // whether an item's rows of them fit into shared memory
+  int state_late;        // whether its state has no room of its own there, but takes that of the low-rank vectors behind them
   float* ring;
   float* gate;           // [H * vdim] output gate before the sigmoid
   // wkv

@@ -426,3 +426,17 @@ def test_wide_values_of_the_delta_rule(vdim, dtype):
     for sizes in ([24], [9, 1, 1, 1]):
         dec.reset()
         assert hc.error(portions(dec, t, sizes), want) <= LIMIT[dtype], sizes
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim, vdim, rank", [(256, 40, (49000, 40)), (200, 33, (8, 49900)), (256, 36, (43900, 8))])
+def test_the_largest_low_ranks(dim, vdim, rank, dtype):
+    """Low-rank vectors that leave the state of the delta rule no room of its own in the token pass, and nearly so; limits as
+    above."""
+    cfg = hc.model(50, 24, [hc.delta(2, 1, dim, vdim, 3)])
+    w, t = hc.weights(cfg, 121, rank=rank), hc.tokens(cfg, 12, 122)
+    want = oh.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype, max_seq=16, max_portion=16)
+    for sizes in ([12], [5, 1, 1, 1], [1]):
+        dec.reset()
+        assert hc.error(portions(dec, t, sizes), want) <= LIMIT[dtype], sizes
