@@ -395,7 +395,7 @@ struct PhaseRows {
 
 template <int DC, int TILE>
 __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_constant__ TokenKernelArgs a) {
-  // two places for the vector or the attention's scratch, the attention's tile, this CTA's residual rows, the ring
+  // two places for the vector, under them the attention's scratch and tiles (plan), this CTA's residual rows, the ring
   extern __shared__ __align__(128) float sm[];
   __shared__ __align__(16) float s_red[kWarps];
   __shared__ Word s_best[kWarps];
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
   __shared__ TokenLayer s_layer[kTokenMaxLayers];
   constexpr int D = 32 * DC;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, hid = a.hid;
-  float *const tile = sm + a.stage_floats, *const res = tile + 2 * TILE / 4;
+  float *const tile = sm + a.tile_at, *const res = sm + a.front_floats;
   Ring ring(reinterpret_cast<char*>(res + a.residual_floats), s_bar, a.stages, a.stage_bytes, a.sync, a.status);
   if (threadIdx.x == 0) ring.init();
   if (threadIdx.x < 5) {
@@ -422,7 +422,6 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
   int pos = a.counters[0];
   int64_t tok = *a.cur_token;
   unsigned e = 0;   // number of the last exchange
-  int buffer = 0;
   const float inv_hid = 1.0f / static_cast<float>(hid);
 
   // False: a wait ran out, here or in another CTA.
@@ -444,6 +443,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
       for (int step = 0; step <= 4 * a.L; ++step) {
         const int j = step == 4 * a.L ? 4 : step & 3, l = min(step >> 2, a.L - 1);   // QKV, O, gate|up, down; the head
         if (j == 0 && static_cast<int>(blockIdx.x) < items) {   // cached rows, under the QKV product
+          if (a.tiles_over != 0) ring_sync();   // the second place of the vector has been read
           request_tile<D, TILE>(a, tile, l, mine, pos, 0);
           request_tile<D, TILE>(a, tile, l, mine, pos, 1);
         }
@@ -469,9 +469,9 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
           ask(a.P + s_layer[l + 1].w_in, hid * 4);
           ask(a.P + s_layer[l + 1].w_post, hid * 4);
         }
-        // ---- the vector, in one of two places: the other one may still be read. xs = v (times the norm weights; s_red collects the sum of squares of v) ----
+        // ---- the vector, in one of two places in turn: the other one may still be read. xs = v (times the norm weights; s_red collects the sum of squares of v) ----
         const bool normed = j != 1 && j != 3;
-        float* const xs = sm + buffer * a.vector_floats;
+        float* const xs = sm + (normed ? 0 : a.second_at);
         {
           const float* nw = a.P + (j == 0 ? s_layer[l].w_in : (j == 2 ? s_layer[l].w_post : a.norm));
           float ss = 0.0f;
@@ -521,8 +521,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
           put(out + row, v, number);
         });
         if (!ok) p.gone = true;
-        if (a.vector_floats > 0) buffer ^= 1;
-        else ring_sync();   // one place only: the vector has been read
+        if (a.second_at == 0) ring_sync();   // one place only: the vector has been read
         if (j == 3) e += 6;
       }
       if (a.out_tokens == nullptr) return true;
@@ -587,41 +586,51 @@ Kernel kernel_of(int D, int tile) {
   if (tile == kTileBytes[0]) return D == 64 ? token_kernel<2, kTileBytes[0]> : token_kernel<4, kTileBytes[0]>;
   return D == 64 ? token_kernel<2, kTileBytes[1]> : token_kernel<4, kTileBytes[1]>;
 }
-// Lays the shared memory out: two places for the vector where they leave room for the ring, else one; pieces of up to 32
-// kLaneChunks chunks, less where that does not leave room for three stages. Returns its size, 0 when there is no room.
-size_t plan(TokenKernelArgs& a, int grid, int tile, int* places, int* piece) {
+// Lays the shared memory out and returns its size (0: no room). The vectors of width hid stand in the first place and the
+// other two, attention and act, in the second one, so that the places of a phase and the next differ; with one place a phase
+// waits until the one before has read it. The attention's scratch lies over both places, its tiles behind them or (`over`, a
+// block barrier more) over the second one: they are asked for while the QKV product reads the first, and have been read when the
+// attention vector comes. The ring gets what is left, in pieces of up to `piece` chunks.
+size_t lay_out(TokenKernelArgs& a, int grid, int tile, int places, bool over, int piece) {
   constexpr int64_t kRoom = 227 * 1024 - 4096;   // the kernel's own arrays take 3.1 KB
-  const int64_t vector = (std::max(std::max(a.hid, a.H * a.D), a.I) + 31) / 32 * 32, G = a.H / a.Hk;
-  const int64_t attn = G * (a.D + tile / (8 * a.D)) + kWarps * 34 + 2 * a.D;
+  auto up = [](int64_t n) { return (n + 31) / 32 * 32; };
+  const int64_t first = up(a.hid), second = up(std::max(a.H * a.D, a.I)), G = a.H / a.Hk;
+  const int64_t scratch = up(G * (a.D + tile / (8 * a.D)) + kWarps * 34 + 2 * a.D);
   a.group = static_cast<int>(G);
   a.tile_bytes = tile;
-  a.residual_floats = (ceil_div(a.hid, grid) + 31) / 32 * 32;
+  a.residual_floats = static_cast<int>(up(ceil_div(a.hid, grid)));
+  a.second_at = places == 2 ? static_cast<int>(first) : 0;
+  const int64_t vectors = std::max(first, a.second_at + second), tiles = int64_t{2} * tile / 4;
+  a.tile_at = static_cast<int>(std::max(over ? first : vectors, scratch));
+  a.tiles_over = a.tile_at < vectors ? 1 : 0;
+  a.front_floats = static_cast<int>(std::max(vectors, a.tile_at + tiles));
+  const int64_t front = (a.front_floats + a.residual_floats) * int64_t{4};
   const int K[5] = {a.hid, a.H * a.D, a.hid, a.I, a.hid};
-  for (*places = 2; *places >= 1; --*places) {
-    a.vector_floats = *places == 2 ? static_cast<int>(vector) : 0;
-    a.stage_floats = static_cast<int>((std::max(*places * vector, attn) + 31) / 32 * 32);
-    const int64_t front = (a.stage_floats + a.residual_floats) * int64_t{4} + 2 * tile;
-    for (*piece = 32 * kLaneChunks; *piece >= 32; *piece /= 2) {
-      a.stage_bytes = 0;
-      for (int j = 0; j < 5; ++j) {
-        a.product[j] = ring_rows(K[j] / 4, *piece);
-        a.stage_bytes = std::max(a.stage_bytes, ring_stage_bytes(a.product[j]));
-      }
-      a.stages = static_cast<int>(std::min<int64_t>((kRoom - front) / a.stage_bytes, kRingMaxStages));
-      if (a.stages >= 3) return front + static_cast<size_t>(a.stages) * a.stage_bytes;
-    }
+  a.stage_bytes = 0;
+  for (int j = 0; j < 5; ++j) {
+    a.product[j] = ring_rows(K[j] / 4, piece);
+    a.stage_bytes = std::max(a.stage_bytes, ring_stage_bytes(a.product[j]));
   }
-  return 0;
+  a.stages = static_cast<int>(std::min<int64_t>((kRoom - front) / a.stage_bytes, kRingMaxStages));
+  return a.stages >= 3 ? static_cast<size_t>(front + static_cast<int64_t>(a.stages) * a.stage_bytes) : 0;
 }
-// Places of 32 KB where they take neither a place of the vector nor a shorter piece nor the fourth stage from the ring, else of
-// 16 KB. Qwen3-0.6B, 4000 + 32 tokens: 46.3 ms with the large ones, 49.7 with the small ones, 49.1 with one place of 32 KB;
-// Llama-3.2-1B, 2000 + 16 tokens (shorter pieces with the large ones): 28.2, 23.7 and 23.7.
+// The longest pieces of which three stages fit, in two places rather than one, four stages rather than three, tiles of their own
+// rather than over the second place, and of 32 KB where that leaves four stages. A stage costs the warps about the same whatever
+// it holds, and what is on its way has to cover the memory's latency: four layers of Llama-3-8B's sizes (4096, 14336) took 833 us
+// a token with four stages of 16 KB behind two places for any vector and tiles of their own, and take 567 with four of 32 KB; two
+// layers of 8192 and 28672 1436 with four of 16 KB, 1007 with three of 32 KB and one place. Rows of 32768 leave five of 16 KB (four
+// layers of width 1024: 437 us, 751 with eleven of 8 KB). Llama-3.2-1B, 16000 + 8 tokens, with tiles of 32 KB over the second place
+// 1984 and 2060 us, of 16 KB beside it 1946 and 1997.
 size_t plan(TokenKernelArgs& a, int grid) {
-  int places[2], piece[2];
-  const size_t small = plan(a, grid, kTileBytes[1], &places[1], &piece[1]);
-  const size_t large = plan(a, grid, kTileBytes[0], &places[0], &piece[0]);
-  if (large != 0 && places[0] == places[1] && piece[0] == piece[1] && a.stages >= 4) return large;
-  return small == 0 ? 0 : plan(a, grid, kTileBytes[1], &places[1], &piece[1]);
+  for (int piece = 32 * kLaneChunks; piece >= 32; piece /= 2)
+    for (int places = 2; places >= 1; --places)
+      for (int stages = 4; stages >= 3; --stages)
+        for (int over = 0; over <= 1; ++over)
+          for (int tile : kTileBytes) {
+            const size_t size = lay_out(a, grid, tile, places, over != 0, piece);
+            if (size != 0 && a.stages >= (tile == kTileBytes[0] ? 4 : stages)) return size;
+          }
+  return 0;
 }
 int64_t padded(int64_t n) { return (n + 31) / 32 * 32; }
 

@@ -30,7 +30,7 @@ struct TokenKernelArgs {
   float* logits;
   Word *x, *hm, *qkv, *part, *attn, *act, *best;
   RingRows product[5];         // QKV, O, gate|up, down, head
-  int vector_floats, stage_floats, residual_floats, stages, stage_bytes;   // shared memory: a place of the vector (0: there is one only), ...
+  int second_at, tile_at, tiles_over, front_floats, residual_floats, stages, stage_bytes;   // shared memory (decode_token.cu): the second place of the vector (0: there is one only), ...
   int tile_bytes;   // of a place for cached keys and values, of which there are two
   int64_t* cur_token;
   int* counters;

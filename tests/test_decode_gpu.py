@@ -277,3 +277,23 @@ def test_gates_at_the_edge_of_the_range(gate):
     limit = 5e-3 * max(np.abs(ref).max(), 1.0)
     assert np.abs(quiet - ref).max() > 20 * limit
     assert np.abs(got - ref).max() <= limit
+
+
+@pytest.mark.parametrize("hid, inter, heads, kv_heads, dim, contexts", [(128, 26048, 48, 48, 64, (10, 190, 390)), (128, 20480, 96, 24, 128, (190, 300)),
+                                                                       (1024, 31616, 16, 2, 128, (9, 600))])
+def test_tiles_over_the_place_of_the_vector(hid, inter, heads, kv_heads, dim, contexts):
+    """Rows so long that the attention's tiles lie over the second place of the vector, or that there is one place only, with
+    ranges of one and several tiles; tolerance as above (weights are drawn so that a layer keeps the size of what passes through it)."""
+    from emberlm_b200 import engine as E
+    kw = dict(CASES[0], hidden_size=hid, intermediate_size=inter, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=dim)
+    ocfg, ecfg = om.LlamaConfig(**kw), E.make_config(**kw)
+    params = om.init_params(ocfg, seed=69, std=0.5 * hid ** -0.5)
+    prompt = np.random.default_rng(heads).integers(0, ocfg.vocab_size, size=max(contexts) + 3)
+    ref = om.forward_logits(params, ocfg, prompt[None, :], acc=np.float64)[0]
+    dec = E.Decoder(ecfg, max_seq_len=max(contexts) + 8)
+    dec.load_parameters(params)
+    for context in contexts:
+        dec.reset()
+        dec.extend(prompt[:context])
+        for i in range(context, context + 3):
+            assert np.abs(dec.step(int(prompt[i])).cpu().numpy() - ref[i]).max() <= 5e-3 * max(np.abs(ref[i]).max(), 1.0), (context, i)
