@@ -203,20 +203,66 @@ __device__ __forceinline__ void request_tile(const TokenKernelArgs& a, float* ti
   cp_async_commit();
 }
 
+inline __host__ __device__ int attention_scratch(int blocks) { return (blocks > kWarps ? blocks : kWarps) * 34; }
+
+// Scores of n keys of a tile with all query heads, sc[head][key]: 16 threads per key, four sums of NH heads and 4 / NH keys at a
+// time, whose reductions share shuffles (five in a chain of four instead of sixteen in a row). With that, eight keys' products in
+// flight and one walk over the keys for all heads of a group, us a token behind 4000, 8000 and 16 000 positions: four layers of
+// Llama-3-8B's sizes 690 -> 644, Qwen3-0.6B 1475 -> 1265, Llama-3.2-1B 1984 -> 1651.
+template <int DC, int NH, int KEYS>
+__device__ __forceinline__ void tile_scores(const float* tile, const float* qs, float* sc, int G, int n) {
+  constexpr int D = 32 * DC, NK = 4 / NH;
+  const int t = threadIdx.x & 15;
+  const bool h8 = (t & 8) != 0, h4 = (t & 4) != 0;
+  const int which = (h4 ? 2 : 0) + (h8 ? 1 : 0), my_key = kThreads / 16 * (which / NH), my_head = which % NH;   // of this thread's sum
+#pragma unroll 1
+  for (int key = threadIdx.x >> 4; (key & ~1) < n; key += kThreads / 16 * NK) {   // whole warps
+    float4 k[NK][DC / 2];
+#pragma unroll
+    for (int x = 0; x < NK; ++x) {
+      const int at = key + kThreads / 16 * x;
+      const float4* k4 = reinterpret_cast<const float4*>(tile + (at < n ? at : 0) * D) + t;
+#pragma unroll
+      for (int c = 0; c < DC / 2; ++c) k[x][c] = k4[16 * c];
+    }
+#pragma unroll 1
+    for (int g = 0; g < G; g += NH) {
+      float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int h = 0; h < NH; ++h) {
+        const float4* q4 = reinterpret_cast<const float4*>(qs + min(g + h, G - 1) * D) + t;
+#pragma unroll
+        for (int c = 0; c < DC / 2; ++c) {
+          const float4 q = q4[16 * c];
+#pragma unroll
+          for (int x = 0; x < NK; ++x)
+            d[x * NH + h] = fmaf(q.x, k[x][c].x, fmaf(q.y, k[x][c].y, fmaf(q.z, k[x][c].z, fmaf(q.w, k[x][c].w, d[x * NH + h]))));
+        }
+      }
+      const float d0 = (h8 ? d[1] : d[0]) + __shfl_xor_sync(0xffffffffu, h8 ? d[0] : d[1], 8);
+      const float d1 = (h8 ? d[3] : d[2]) + __shfl_xor_sync(0xffffffffu, h8 ? d[2] : d[3], 8);
+      float v = (h4 ? d1 : d0) + __shfl_xor_sync(0xffffffffu, h4 ? d0 : d1, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      if ((t & 3) == 0 && key + my_key < n && g + my_head < G) sc[(g + my_head) * KEYS + key + my_key] = v;
+    }
+  }
+}
+
 // Attention of the new row for one item, whose first two tiles have been requested: results as words of the attention vector
 // (one range) or of the range. Threads: 16 per key for the scores; for the weighted sums a warp per 32 columns of a head
 // and share of the keys.
 template <int DC, int TILE>
 __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, const Item it, int splits, int pos, unsigned e, int64_t wqn, int64_t wkn,
                                             float* sm, float* tiles) {
-  constexpr int D = 32 * DC, kKeys = tile_keys(D, TILE), kHeadsAtOnce = kWarps / DC;
+  constexpr int D = 32 * DC, kKeys = tile_keys(D, TILE);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = a.group;
   Patience p(a);
   const bool has_new = pos >= it.j0 && pos < it.j1;
   float* qs = sm;                  // [G][D] rotated, scaled
   float* sc = qs + G * D;          // [G][kKeys] scores
-  float* scr = sc + G * kKeys;     // [kWarps][34] partial results of the shares of the keys
-  float* kn = scr + kWarps * 34;   // [2][D] the new row
+  float* scr = sc + G * kKeys;     // [kWarps or blocks][34] partial results of the shares of the keys, or of the blocks
+  float* kn = scr + attention_scratch(G * DC);   // [2][D] the new row
   // new rows: a warp per head; queries 0 .. G-1, then key and value where the range holds the new position
 #pragma unroll 1
   for (int r = wid; r < G + (has_new ? 2 : 0); r += kWarps) {
@@ -272,50 +318,41 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
   }
   if (p.left()) return false;
 
+  // blocks of 32 columns of a head, a warp each, with shares of the keys (the largest power of two that the warps allow); where
+  // there are more blocks than warps, a warp takes several, whose sums stand in its places of `scr` between two tiles
+  const int blocks = G * DC, turns = (blocks + kWarps - 1) / kWarps;
+  const int sh = blocks * 8 <= kWarps ? 3 : (blocks * 4 <= kWarps ? 2 : (blocks * 2 <= kWarps ? 1 : 0)), shares = 1 << sh;
+  int mine_first = wid, share = 0;   // this warp's first block
+  if (turns == 1) {
 #pragma unroll 1
-  for (int g0 = 0; g0 < G; g0 += kHeadsAtOnce) {
-    const int heads = min(kHeadsAtOnce, G - g0), blocks = heads * DC;
-    // shares of the keys: the largest power of two that the warps allow
-    const int sh = blocks * 8 <= kWarps ? 3 : (blocks * 4 <= kWarps ? 2 : (blocks * 2 <= kWarps ? 1 : 0)), shares = 1 << sh;
-    int blk = wid, share = 0;
+    for (; mine_first >= blocks; mine_first -= blocks) ++share;
+  }
+  float m = -FLT_MAX, s = 0.0f, o = 0.0f;
 #pragma unroll 1
-    for (; blk >= blocks; blk -= blocks) ++share;
-    const int h = g0 + blk / DC, col = blk % DC * 32 + lane;
-    float m = -FLT_MAX, s = 0.0f, o = 0.0f;
-#pragma unroll 1
-    for (int j = it.j0, number = 0; j < it.j1; j += kKeys, ++number) {
-      const int n = min(kKeys, it.j1 - j);
-      float* const tile = tiles + (number & 1) * (TILE / 4);
-      cp_async_wait<1>();
+  for (int j = it.j0, number = 0; j < it.j1; j += kKeys, ++number) {
+    const int n = min(kKeys, it.j1 - j);
+    float* const tile = tiles + (number & 1) * (TILE / 4);
+    cp_async_wait<1>();
+    ring_sync();
+    if (pos >= j && pos < j + n) {
+      if (threadIdx.x < 2 * D) tile[(threadIdx.x < D ? 0 : TILE / 8) + (pos - j) * D + (threadIdx.x & (D - 1))] = kn[threadIdx.x];
       ring_sync();
-      if (pos >= j && pos < j + n) {
-        if (threadIdx.x < 2 * D) tile[(threadIdx.x < D ? 0 : TILE / 8) + (pos - j) * D + (threadIdx.x & (D - 1))] = kn[threadIdx.x];
-        ring_sync();
-      }
+    }
+    if (G == 1) tile_scores<DC, 1, kKeys>(tile, qs, sc, 1, n);
+    else if (G == 2) tile_scores<DC, 2, kKeys>(tile, qs, sc, 2, n);
+    else tile_scores<DC, 4, kKeys>(tile, qs, sc, G, n);
+    ring_sync();
+    if (share < shares) {
+      const int mine = (n - share + shares - 1) >> sh;   // keys share, share + shares, ... of the tile
 #pragma unroll 1
-      for (int key = threadIdx.x >> 4; (key & ~1) < n; key += kThreads / 16) {   // whole warps
-        const int t = threadIdx.x & 15;
-        const float4* k4 = reinterpret_cast<const float4*>(tile + (key < n ? key : 0) * D) + t;
-        float4 k[DC / 2];
-#pragma unroll
-        for (int c = 0; c < DC / 2; ++c) k[c] = k4[16 * c];
-#pragma unroll 1
-        for (int g = g0; g < g0 + heads; ++g) {
-          const float4* q4 = reinterpret_cast<const float4*>(qs + g * D) + t;
-          float d = 0.0f;
-#pragma unroll
-          for (int c = 0; c < DC / 2; ++c) {
-            const float4 q = q4[16 * c];
-            d = fmaf(q.x, k[c].x, fmaf(q.y, k[c].y, fmaf(q.z, k[c].z, fmaf(q.w, k[c].w, d))));
-          }
-#pragma unroll
-          for (int x = 8; x > 0; x >>= 1) d += __shfl_xor_sync(0xffffffffu, d, x);
-          if (t == 0) sc[g * kKeys + key] = d;
+      for (int blk = mine_first; blk < blocks; blk += kWarps) {
+        const int h = blk / DC, col = blk % DC * 32 + lane;
+        float* const held = scr + blk * 34;
+        if (turns > 1 && j != it.j0) {
+          m = held[0];
+          s = held[1];
+          o = held[2 + lane];
         }
-      }
-      ring_sync();
-      if (share < shares) {
-        const int mine = (n - share + shares - 1) >> sh;   // keys share, share + shares, ... of the tile
 #pragma unroll 1
         for (int i0 = 0; i0 < mine; i0 += 32) {
           const int count = min(32, mine - i0), first = share + i0 * shares;
@@ -325,36 +362,48 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
           s = s * fix + warp_sum(w);
           o *= fix;
           const float* v = tile + TILE / 8 + first * D + col;
-#pragma unroll 4
+#pragma unroll 8
           for (int i = 0; i < count; ++i) o = fmaf(__shfl_sync(0xffffffffu, w, i), v[i * shares * D], o);
         }
-      }
-      const bool more = j + 2 * kKeys < it.j1;
-      if (more) ring_sync();   // this place has been read
-      request_tile<D, TILE>(a, tiles, l, it, more ? pos : 0, number + 2);
-    }
-    if (g0 + kHeadsAtOnce < G) {
-      ring_sync();
-      request_tile<D, TILE>(a, tiles, l, it, pos, 0);
-      request_tile<D, TILE>(a, tiles, l, it, pos, 1);
-    }
-    if (shares > 1) {
-      scr[wid * 34 + 2 + lane] = o;
-      if (lane == 0) *reinterpret_cast<float2*>(scr + wid * 34) = make_float2(m, s);
-      ring_sync();
-      if (share == 0) {
-#pragma unroll 1
-        for (int k = 1; k < shares; ++k) {
-          const float* other = scr + (wid + k * blocks) * 34;
-          const float most = fmaxf(m, other[0]), f = __expf(m - most), fo = __expf(other[0] - most);
-          s = s * f + other[1] * fo;
-          o = o * f + other[2 + lane] * fo;
-          m = most;
+        if (turns > 1) {
+          __syncwarp();   // all lanes have read the maximum and the sum
+          held[2 + lane] = o;
+          if (lane == 0) *reinterpret_cast<float2*>(held) = make_float2(m, s);
+          __syncwarp();
+          m = -FLT_MAX;
+          s = o = 0.0f;
         }
       }
     }
+    const bool more = j + 2 * kKeys < it.j1;
+    if (more) ring_sync();   // this place has been read
+    request_tile<D, TILE>(a, tiles, l, it, more ? pos : 0, number + 2);
+  }
+  if (shares > 1) {
+    scr[wid * 34 + 2 + lane] = o;
+    if (lane == 0) *reinterpret_cast<float2*>(scr + wid * 34) = make_float2(m, s);
+    ring_sync();
     if (share == 0) {
-      const int head = it.hk * G + h;
+#pragma unroll 1
+      for (int k = 1; k < shares; ++k) {
+        const float* other = scr + (wid + k * blocks) * 34;
+        const float most = fmaxf(m, other[0]), f = __expf(m - most), fo = __expf(other[0] - most);
+        s = s * f + other[1] * fo;
+        o = o * f + other[2 + lane] * fo;
+        m = most;
+      }
+    }
+  }
+  if (share == 0) {
+#pragma unroll 1
+    for (int blk = mine_first; blk < blocks; blk += kWarps) {
+      const int head = it.hk * G + blk / DC, col = blk % DC * 32 + lane;
+      if (turns > 1 && it.j0 < it.j1) {
+        const float* held = scr + blk * 34;
+        m = held[0];
+        s = held[1];
+        o = held[2 + lane];
+      }
       if (splits == 1) {
         put(a.attn + head * D + col, o / s, e + 3);
       } else {   // [column][range]: the ranges of a column side by side
@@ -366,8 +415,8 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
         }
       }
     }
-    ring_sync();   // the scratch is written again
   }
+  ring_sync();   // the scratch is written again
   return !p.gone;
 }
 
@@ -595,7 +644,7 @@ size_t lay_out(TokenKernelArgs& a, int grid, int tile, int places, bool over, in
   constexpr int64_t kRoom = 227 * 1024 - 4096;   // the kernel's own arrays take 3.1 KB
   auto up = [](int64_t n) { return (n + 31) / 32 * 32; };
   const int64_t first = up(a.hid), second = up(std::max(a.H * a.D, a.I)), G = a.H / a.Hk;
-  const int64_t scratch = up(G * (a.D + tile / (8 * a.D)) + kWarps * 34 + 2 * a.D);
+  const int64_t scratch = up(G * (a.D + tile / (8 * a.D)) + attention_scratch(static_cast<int>(G) * a.D / 32) + 2 * a.D);
   a.group = static_cast<int>(G);
   a.tile_bytes = tile;
   a.residual_floats = static_cast<int>(up(ceil_div(a.hid, grid)));
@@ -614,19 +663,19 @@ size_t lay_out(TokenKernelArgs& a, int grid, int tile, int places, bool over, in
   a.stages = static_cast<int>(std::min<int64_t>((kRoom - front) / a.stage_bytes, kRingMaxStages));
   return a.stages >= 3 ? static_cast<size_t>(front + static_cast<int64_t>(a.stages) * a.stage_bytes) : 0;
 }
-// The longest pieces of which three stages fit, in two places rather than one, four stages rather than three, tiles of their own
-// rather than over the second place, and of 32 KB where that leaves four stages. A stage costs the warps about the same whatever
-// it holds, and what is on its way has to cover the memory's latency: four layers of Llama-3-8B's sizes (4096, 14336) took 833 us
-// a token with four stages of 16 KB behind two places for any vector and tiles of their own, and take 567 with four of 32 KB; two
+// The longest pieces of which three stages fit, in two places rather than one, four stages rather than three, tiles of 32 KB where
+// that leaves four stages, and of their own rather than over the second place. A stage costs the warps about the same whatever it
+// holds, and what is on its way has to cover the memory's latency: four layers of Llama-3-8B's sizes (4096, 14336) took 833 us a
+// token with four stages of 16 KB behind two places for any vector and tiles of their own, and take 567 with four of 32 KB; two
 // layers of 8192 and 28672 1436 with four of 16 KB, 1007 with three of 32 KB and one place. Rows of 32768 leave five of 16 KB (four
-// layers of width 1024: 437 us, 751 with eleven of 8 KB). Llama-3.2-1B, 16000 + 8 tokens, with tiles of 32 KB over the second place
-// 1984 and 2060 us, of 16 KB beside it 1946 and 1997.
+// layers of width 1024: 437 us, 751 with eleven of 8 KB). Tiles of 32 KB over the second place against tiles of 16 KB beside it, us a
+// token: Qwen3-1.7B behind 10, 300 and 4000 positions 1275, 1304, 1667 and 1272, 1335, 1833; Llama-3.2-1B behind 16 000 1651 and 1765.
 size_t plan(TokenKernelArgs& a, int grid) {
   for (int piece = 32 * kLaneChunks; piece >= 32; piece /= 2)
     for (int places = 2; places >= 1; --places)
       for (int stages = 4; stages >= 3; --stages)
-        for (int over = 0; over <= 1; ++over)
-          for (int tile : kTileBytes) {
+        for (int tile : kTileBytes)
+          for (int over = 0; over <= 1; ++over) {
             const size_t size = lay_out(a, grid, tile, places, over != 0, piece);
             if (size != 0 && a.stages >= (tile == kTileBytes[0] ? 4 : stages)) return size;
           }

@@ -297,3 +297,21 @@ def test_tiles_over_the_place_of_the_vector(hid, inter, heads, kv_heads, dim, co
         dec.extend(prompt[:context])
         for i in range(context, context + 3):
             assert np.abs(dec.step(int(prompt[i])).cpu().numpy() - ref[i]).max() <= 5e-3 * max(np.abs(ref[i]).max(), 1.0), (context, i)
+
+
+@pytest.mark.parametrize("heads, kv_heads, dim", [(32, 1, 128), (5, 1, 64), (9, 3, 64), (2, 2, 128), (17, 1, 64)])
+def test_groups_of_query_heads(heads, kv_heads, dim):
+    """Groups of one, two, three and more query heads, which share the walk over the keys, with as many blocks of 32 columns as a
+    range's warps, fewer and more; tolerance as above."""
+    from emberlm_b200 import engine as E
+    kw = dict(CASES[0], num_hidden_layers=1, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=dim)
+    ocfg, ecfg, params = build(kw, 71)
+    prompt = np.random.default_rng(heads).integers(0, ocfg.vocab_size, size=1400)
+    ref = om.forward_logits(params, ocfg, prompt[None, :], acc=np.float64)[0]
+    dec = E.Decoder(ecfg, max_seq_len=1408)
+    dec.load_parameters(params)
+    for context in (1, 15, 70, 700, 1397):
+        dec.reset()
+        dec.extend(prompt[:context])
+        for i in range(context, context + 3):
+            assert np.abs(dec.step(int(prompt[i])).cpu().numpy() - ref[i]).max() <= 5e-3 * max(np.abs(ref[i]).max(), 1.0), (context, i)
