@@ -229,7 +229,6 @@ int HybridDecoder<T>::build_phases() {
         t.splits = kAttnSplits;
         const int others = mx.n_branch == 2 ? L.branches[1 - b].heads * ((L.branches[1 - b].vdim + 31) / 32) : 0;
         if (sm_count() > others) t.splits = std::max(4, std::min(kAttnSplits, (sm_count() - others) / br.kv_heads));
-        t.items = br.kv_heads * t.splits;
       } else if (br.kind == BranchKind::kLightning) {
         t.kind = kTokLightning;
         t.items = br.heads * column_blocks;

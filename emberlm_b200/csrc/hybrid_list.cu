@@ -467,13 +467,11 @@ __device__ __forceinline__ void latent_keys_item(const TokenBranch& br, int item
   }
 }
 
-// Position ranges in use for L cached positions, and their length (whole tiles).
+// Position ranges in use for L cached positions (less than 2^25), and their length (whole tiles).
 __device__ __forceinline__ int latent_ranges(int L, int splits, int& per) {
-  // (x + 1/2) / d lies half a d-th or more from every whole number, more than two roundings while x < 2^21
-  auto over = [](int x, int d) { return static_cast<int>(__fdividef(static_cast<float>(x) + 0.5f, static_cast<float>(d))); };
-  const int tiles = (L + kLatentKeys - 1) / kLatentKeys, each = over(tiles + splits - 1, splits);
+  const int tiles = (L + kLatentKeys - 1) / kLatentKeys, each = small_quotient(tiles + splits - 1, splits);
   per = each * kLatentKeys;
-  return over(tiles + each - 1, each);
+  return small_quotient(tiles + each - 1, each);
 }
 
 // kLatentHeadsF32 query heads over one range of cached positions: running maximum, sum and the weighted sum

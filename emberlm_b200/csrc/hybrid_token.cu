@@ -143,11 +143,15 @@ __device__ __forceinline__ float stage_norm(const TokenArgs& a, const TokenPhase
   return rsqrtf(sum[0] * inv + a.eps);
 }
 
-// Key ranges in use at position pos, and their length.
-__device__ __forceinline__ int attention_ranges(const TokenBranch& br, int pos, int& per) {
-  const int L = pos % br.chunk + 1, n = min(br.splits, (L + 15) / 16);
-  per = (L + n - 1) / n;
-  return (L + per - 1) / per;
+// Key ranges in use at a slot of the chunk, and their length: of 16 keys, as many as leave all of the phase's items one turn of the CTAs
+// (br.splits), more of them where the ranges would be longer than kRangeMost: a second item, a recurrent one, costs a CTA as much as
+// about 60 keys. Eight layers of width 2048 with 8 key/value heads, chunks of 8192, us a token behind 1000 and 8000 positions: with
+// 32 recurrent heads (4 ranges at least) 827 -> 711 and 2457 -> 1095, with 16 (10 ranges) 588 -> 585 and 1256 -> 991.
+constexpr int kRangeMost = 128;
+__device__ __forceinline__ int attention_ranges(const TokenBranch& br, int slot, int& per) {
+  const int L = slot + 1, n = max(min(br.splits, (L + 15) / 16), min(kAttnSplits, (L + kRangeMost - 1) / kRangeMost));
+  per = quotient(L + n - 1, n);
+  return quotient(L + per - 1, per);
 }
 
 // Outputs of the mix phase as inputs of the output projections; scale: what the rows of a branch's product are
@@ -256,41 +260,45 @@ __device__ __forceinline__ void stage_mixed(const TokenArgs& a, const TokenPhase
 // ---- items of the mix phase ----
 // What an item reads that does not depend on the token (cached keys and their angles, states, low-rank rows) is copied to
 // shared memory while the CTA waits for the projections, request_item(), for the CTA's first item. Which item that is takes
-// a dozen integer divisions (about 200 cycles each), which are made there too.
+// half a dozen divisions, which are made there too.
 struct MixItem {
   int branch;      // -1: none
   int head, part;  // attention: key/value head and range; recurrences: head and block of 32 columns
-  int slot, j0, j1; // attention: slot of this position, slots of the range (none: j0 == j1)
-  int ranges;      // of the phase's attention branch, set for every CTA
+  int slot, j0, j1; // attention: slot of this position, slots of the range
+  int ranges;      // of the phase's attention branch, set for every CTA, as is the number of
+  int items;       // all items of the phase
   int group;       // delta: head of the queries and keys
   int tap;         // delta: place of this position in the ring of the convolutions
 };
 __device__ __forceinline__ MixItem mix_item(const TokenPhase& ph, int it, int pos) {
-  MixItem m{-1, 0, 0, 0, 0, 0, 0, 0, 0};
+  MixItem m{-1, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int b = 0; b < ph.n_branch; ++b) {
     const TokenBranch& br = ph.br[b];
-    const bool here = m.branch < 0 && it < br.items;
+    int n = br.items;
     if (br.kind == kTokAttention) {
       int per;
-      m.ranges = attention_ranges(br, pos, per);
-      if (here) {
-        m.part = it / br.G;
+      m.slot = pos < br.chunk ? pos : pos % br.chunk;
+      m.ranges = attention_ranges(br, m.slot, per);
+      n = br.G * m.ranges;
+      if (it >= 0 && it < n) {
+        m.branch = b;
+        m.part = quotient(it, br.G);
         m.head = it - m.part * br.G;
         m.j0 = m.part * per;
-        m.slot = pos % br.chunk;
-        m.j1 = m.part < m.ranges ? min(m.slot + 1, m.j0 + per) : m.j0;
+        m.j1 = min(m.slot + 1, m.j0 + per);
       }
-    } else if (here) {
+    } else if (it >= 0 && it < n) {
       const int nb = (br.vdim + 31) / 32;
-      m.head = it / nb;
+      m.branch = b;
+      m.head = quotient(it, nb);
       m.part = it - m.head * nb;
       if (br.kind == kTokDelta) {
-        m.group = m.head / br.group;
-        m.tap = pos % br.taps;
+        m.group = quotient(m.head, br.group);
+        m.tap = pos - quotient(pos, br.taps) * br.taps;
       }
     }
-    if (here) m.branch = b;
-    it -= br.items;
+    it -= n;
+    m.items += n;
   }
   return m;
 }
@@ -335,7 +343,6 @@ template <typename T>
 __device__ __forceinline__ void attention_item(const TokenPhase& ph, const TokenBranch& br, const MixItem it, int pos, float* sm, float* tile_at, bool requested) {
   const int g = it.head, dim = br.dim, P = (dim + 1) >> 1, hq = br.group, KT = br.tile_keys, j0 = it.j0, j1 = it.j1;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, stride = dim + kAttnStats;
-  if (j0 == j1) return;
   KeyTile<T> tile(br, tile_at);
   if (!requested) tile.request(br, g, j0, min(KT, j1 - j0));
   float* qs = sm;                    // [hq][2 P] rotated, scaled
@@ -698,7 +705,7 @@ __device__ __forceinline__ MixItem request_item(const TokenPhase& ph, int pos, f
   if (it.branch < 0) return it;
   const TokenBranch& br = ph.br[it.branch];
   if (br.kind == kTokAttention) {
-    if (it.j0 < it.j1) KeyTile<T>(br, tile_at).request(br, it.head, it.j0, min(br.tile_keys, it.j1 - it.j0));
+    KeyTile<T>(br, tile_at).request(br, it.head, it.j0, min(br.tile_keys, it.j1 - it.j0));
   } else if (br.kind == kTokLightning) {
     if (pos > 0) request_state(tile_at, br.state + static_cast<int64_t>(it.head) * br.dim * br.vdim, br.dim, br.vdim, it.part * 32);
     cp_async_commit();
@@ -717,7 +724,7 @@ __device__ __forceinline__ void mix_phase(const TokenPhase& ph, MixItem it, int 
     else if (br.kind == kTokLightning) lightning_item(ph, br, it, pos, sm, tile_at, first);
     else delta_item<T>(ph, br, it, pos, sm, tile_at, first);
     n += gridDim.x;
-    if (n >= ph.items) return;
+    if (n >= it.items) return;
     it = mix_item(ph, n, pos);
     ring_sync();
   }
@@ -884,10 +891,8 @@ int token_items(TokenPhase* phases, int n, int* tile_at) {
   constexpr int64_t kLateFloats = 52 * 1024;   // with the shortest ring behind it 222 KB; the ranks are then 40 000 and more, a state 8192 floats
   int64_t scratch = 0, tile = 0;
   for (int i = 0; i < n; ++i) {
-    phases[i].items = 0;
     for (int b = 0; b < phases[i].n_branch; ++b) {
       TokenBranch& br = phases[i].br[b];
-      phases[i].items += br.items;
       br.group = br.G > 0 ? br.H / br.G : 1;
       const int64_t ra = (br.rank_a + 7) & ~7, rg = (br.rank_g + 7) & ~7, size = br.elem;
       int64_t f, t;   // floats, bytes

@@ -136,7 +136,7 @@ struct alignas(16) TokenPhase {
   int ffp;
   float limit;
   // mixing
-  int n_branch, items;   // items: of all branches (sandwich layers)
+  int n_branch;
   TokenBranch br[2];
   const float* proj;
 };

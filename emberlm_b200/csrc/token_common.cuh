@@ -83,6 +83,13 @@ __device__ __forceinline__ int quotient(int n, int d, unsigned inv) {
   return static_cast<int>(q + (static_cast<unsigned>(n) - q * static_cast<unsigned>(d) >= static_cast<unsigned>(d) ? 1u : 0u));
 }
 
+// The same for a divisor that only the device knows, x < 2^20, d < 2^24: (x + 1/2) / d lies half a d-th or more from every whole
+// number, more than the approximate division's two ulp and a rounding.
+__device__ __forceinline__ int small_quotient(int x, int d) {
+  return static_cast<int>(__fdividef(static_cast<float>(x) + 0.5f, static_cast<float>(d)));
+}
+__device__ __forceinline__ int quotient(int x, int d) { return x < (1 << 20) ? small_quotient(x, d) : x / d; }
+
 // V neighbouring columns.
 template <int V>
 struct Cols {

@@ -440,3 +440,18 @@ def test_the_largest_low_ranks(dim, vdim, rank, dtype):
     for sizes in ([12], [5, 1, 1, 1], [1]):
         dec.reset()
         assert hc.error(portions(dec, t, sizes), want) <= LIMIT[dtype], sizes
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("kv_heads, recurrent, dim", [(2, 140, 64), (37, 1, 8), (1, 1, 32)])
+def test_ranges_of_long_chunks(kv_heads, recurrent, dim, dtype):
+    """Positions where the number of key ranges goes from what leaves the phase one turn of the CTAs (4, 4 and 16) to ranges of 128
+    keys, from one chunk into the next, with the recurrent heads behind them; limits as above."""
+    cfg = hc.model(50, 40, [hc.parallel(hc.attention(kv_heads, kv_heads, dim, 2100, dim), hc.lightning(recurrent, 4, 4))])
+    w, t = hc.weights(cfg, 131), hc.tokens(cfg, 2124, 132)
+    want = oh.forward(cfg, w, t)
+    dec = decoder(cfg, w, dtype, max_seq=2124, max_portion=2124)
+    for at in (58, 510, 638, 2045, 2098):
+        dec.reset()
+        dec.extend(t[:at])
+        assert hc.error(portions(dec, t[at:at + 6], [1]), want[at:at + 6]) <= LIMIT[dtype], at
