@@ -580,6 +580,7 @@ int run_bwd_legacy(const float* qkv, const float* dout, const float* lse, const 
   const int smem_q = (2 * BQ + 2 * BKV) * (D + 4) * static_cast<int>(sizeof(float));
   const int smem_k = ((2 * BKV + 2 * QT) * (D + 4) + 2 * QT) * static_cast<int>(sizeof(float));
   int rc = CTDK_OK;
+  bool beside = do_dq && do_dkv;
   if (do_dkv) {
     rc = set_smem(attn_bwd_dkv_kernel<D, QT, X3>, smem_k, "ctdk_attn_bwd");
     if (rc != CTDK_OK) return rc;
@@ -587,6 +588,13 @@ int run_bwd_legacy(const float* qkv, const float* dout, const float* lse, const 
     const int64_t tiles = static_cast<int64_t>(gk.x) * gk.y * gk.z, chain = static_cast<int64_t>(H / Hk) * ((T + QT - 1) / QT);
     int R = 1;
     while (R < 8 && tiles * R * 2 <= 2 * sm_count() && R * 2 <= chain) R *= 2;
+    // The dQ kernel runs beside the dK/dV kernel where the SMs hold both at once; elsewhere the two take each other's SMs in
+    // mid-chain. us with 9 heads of 64 on 3: 3 x 301 positions 131 -> 114, 1 x 127 69 -> 55, but 4 x 1023 1040 -> 1319 (a step of
+    // SmolLM2-135M 74.4 -> 83.1 ms), 3 x 1000 629 -> 685; 16 heads of 128 on 8, 1 x 600 648 -> 746. Clusters of eight that share SMs
+    // wait for each other's: 1 x 600 181 -> 187.
+    constexpr int kSmem = 227 * 1024;
+    const int64_t per_k = kSmem / (smem_k + 1024), per_q = kSmem / (smem_q + 1024), all_q = static_cast<int64_t>(gq.x) * gq.y * gq.z;
+    beside = beside && (tiles * R + per_k - 1) / per_k + (all_q + per_q - 1) / per_q <= sm_count() && (R < 8 || tiles * R <= sm_count());
     gk.x *= R;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = gk;
@@ -607,8 +615,7 @@ int run_bwd_legacy(const float* qkv, const float* dout, const float* lse, const 
   if (do_dq) {
     rc = set_smem(attn_bwd_dq_kernel<D, X3>, smem_q, "ctdk_attn_bwd");
     if (rc != CTDK_OK) return rc;
-    // beside the dK/dV kernel (launched first): SmolLM2-135M 3 x 301 positions 19.2 -> 18.7 ms
-    if (do_dkv) launch_pdl(attn_bwd_dq_kernel<D, X3>, gq, dim3(128), smem_q, s, qkv, dout, lse, delta, dqkv, Ti, H, Hk, scale);
+    if (beside) launch_pdl(attn_bwd_dq_kernel<D, X3>, gq, dim3(128), smem_q, s, qkv, dout, lse, delta, dqkv, Ti, H, Hk, scale);
     else attn_bwd_dq_kernel<D, X3><<<gq, 128, smem_q, s>>>(qkv, dout, lse, delta, dqkv, Ti, H, Hk, scale);
     rc = check_launch("ctdk_attn_bwd(dq)");
   }
