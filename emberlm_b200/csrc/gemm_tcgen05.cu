@@ -1037,6 +1037,16 @@ double plain_us(double units, int splits, bool bf16) { return 0.39 * units + (bf
 
 }  // namespace
 
+// Zeroes in front of a product whose ranges of K add to C. Weight gradients (A transposed) run beside the chain of the backward pass,
+// where a product that starts earlier takes the SMs of the chain's next kernel: a memset node, behind which it starts later
+// (SmolLM2-135M, 64 x 63 positions, 30 gate|up gradients a step: 12.97 -> 12.65 ms; 4 x 511 unchanged). Elsewhere the product is a
+// link of the chain: the kernel that overlaps it (SmolLM2-360M, 2 x 700 positions, 97 a step: 14.57 ms, 14.92 with memset nodes).
+static int zero_result(float* C, int64_t M, int64_t N, int64_t ldc, bool gradient, cudaStream_t s) {
+  if (!gradient) return zero_rows(C, M, N, ldc, s);
+  const cudaError_t e = cudaMemset2DAsync(C, static_cast<size_t>(ldc) * sizeof(float), 0, static_cast<size_t>(N) * sizeof(float), static_cast<size_t>(M), s);
+  return e == cudaSuccess ? CTDK_OK : fail(CTDK_ELAUNCH, "gemm: memset failed: %s", cudaGetErrorString(e));
+}
+
 // Returns CTDK_OK after enqueueing, or 1 when the shape/alignment is not eligible for the
 // tensor-core path (the caller then uses the SIMT kernel).
 int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N, int64_t K,
@@ -1104,7 +1114,7 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
     if (st == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
     const int vec = (a16(Cp) && (ldc & 3) == 0 && (aux == nullptr || a16(aux))) ? 1 : 0;
     if (splits > 1 && epilogue != CTDK_EPI_ACCUMULATE) {
-      rc = zero_rows(Cp, M, N, ldc, stream);
+      rc = zero_result(Cp, M, N, ldc, transa != 0, stream);
       if (rc != CTDK_OK) return rc;
     }
     // Output through TMA (coalesced, off the load/store pipe): plain store, or an fp32 add at L2
@@ -1134,7 +1144,7 @@ int gemm_tcgen05(const float* A, const float* B, float* Cp, int64_t M, int64_t N
   args.status = device_status_word();
   if (args.status == nullptr) return fail(CTDK_ELAUNCH, "gemm: no status word");
   if (splits > 1 && epilogue != CTDK_EPI_ACCUMULATE) {
-    rc = zero_rows(Cp, M, N, ldc, stream);
+    rc = zero_result(Cp, M, N, ldc, transa != 0, stream);
     if (rc != CTDK_OK) return rc;
   }
 
