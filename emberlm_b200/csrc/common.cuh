@@ -474,8 +474,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
 // until the predecessor has completed and its writes are visible. Every kernel launched this way
 // calls pdl_wait() before it touches global memory and before any thread exits, so completion
 // stays ordered along the stream. In a kernel launched the ordinary way both calls return at once.
-// A kernel that reads nothing of its predecessor's may wait at its end instead and run beside it, if the predecessor passes
-// pdl_launch() only behind its own pdl_wait() (the attention backward's dQ kernels behind the dK/dV kernels).
+// A kernel that reads nothing of its predecessor's may wait at its end instead and run beside it, if the predecessor either passes
+// pdl_launch() only behind its own pdl_wait() or is launched the ordinary way, without the attribute: what lies before both has
+// then ended (the attention backward's dQ kernels behind the dK/dV kernels, of which the one for head size 64 is the first kind).
 // CTDK_PDL=0 in the environment turns the attribute off.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -211,7 +211,6 @@ int HybridDecoder<T>::build_phases() {
       t.col_k = br.col_k;
       t.col_v = br.col_v;
       t.col_g = br.col_g;
-      t.out = tout[b];
       t.stage_at = offset;
       const int column_blocks = (br.vdim + 31) / 32;
       if (br.kind == BranchKind::kAttention) {
@@ -231,12 +230,14 @@ int HybridDecoder<T>::build_phases() {
         if (sm_count() > others) t.splits = std::max(4, std::min(kAttnSplits, (sm_count() - others) / br.kv_heads));
       } else if (br.kind == BranchKind::kLightning) {
         t.kind = kTokLightning;
+        t.out = tout[b];
         t.items = br.heads * column_blocks;
         t.decay = bb.decay;
         t.state = bb.state;
         t.w_norm = vec(br.w_norm);
       } else {
         t.kind = kTokDelta;
+        t.out = tout[b];
         t.elem = static_cast<int>(sizeof(T));
         t.items = br.heads * column_blocks;
         t.state = bb.state;
@@ -332,7 +333,7 @@ int HybridDecoder<T>::upload(cudaStream_t s) {
   auto copy = [&](void* dst, const void* src, size_t n) { return cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, s) == cudaSuccess; };
   std::vector<std::vector<float>> powers;
   bool ok = copy(phases_dev, phases.data(), phases.size() * sizeof(TokenPhase)) &&
-            copy(products_dev, products.data(), products.size() * sizeof(RingProduct));
+            (products.empty() || copy(products_dev, products.data(), products.size() * sizeof(RingProduct)));
   for (size_t l = 0; l < m.layers.size(); ++l)
     for (size_t b = 0; b < bufs[l].size(); ++b)
       if (bufs[l][b].decay != nullptr) {

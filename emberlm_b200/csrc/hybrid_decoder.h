@@ -76,7 +76,7 @@ struct HybridDecoder : DecoderBase {
   unsigned int* sync;
   int64_t sync_words = 0;
   TokenPhase* phases_dev;
-  RingProduct* products_dev;   // what passes through the token kernel's weight ring, in order
+  RingProduct* products_dev = nullptr;   // what passes through the weight ring of the sandwich layers' token kernel, in order
   int max_products = 0;
   std::vector<RingProduct> products;
   TokenArgs ring{};            // the ring's layout

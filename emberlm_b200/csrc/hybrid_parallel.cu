@@ -136,8 +136,7 @@ int HybridDecoder<T>::carve_parallel(Bump& b) {
   sync_words = kTokenSyncWords;
   sync = static_cast<unsigned int*>(b.bytes(sync_words * 4));
   phases_dev = static_cast<TokenPhase*>(b.bytes((n_layers * 6 + 1) * static_cast<int64_t>(sizeof(TokenPhase))));
-  max_products = static_cast<int>(n_layers) * 10 + 1;   // five mixes, the side product, output and feed-forward
-  products_dev = static_cast<RingProduct*>(b.bytes(max_products * static_cast<int64_t>(sizeof(RingProduct))));
+  products_dev = nullptr;   // its token kernel has no weight ring
   logits = b.floats(vocab);
   cur_token = static_cast<int64_t*>(b.bytes(16));
   counters = static_cast<int*>(b.bytes(64));

@@ -5,7 +5,8 @@
 // launch. Weights pass through the ring of token_ring.cuh while the compute warps wait and stage; vectors between phases are
 // fp32 behind grid barriers, and every CTA stages (and norms) its own copy. All waits are bounded.
 // What bounds a phase (10 000 to 16 000 cycles; its weights would take 3000) is its dependent chain: the barrier (3200 cycles),
-// the norms (2500 to 3500) or the merging of the key ranges (7400), the products (800 a turn), the mix items (10 000).
+// the norms (2500 to 3500 at widths up to 2048; wider ones walk the columns several times) or the merging of the key ranges
+// (7400), the products (800 a turn), the mix items (10 000).
 // zutalix-0.6b, 300 + 64 tokens: 109.4 -> 64.5 ms against sixteen warps that took the rows from L2 and the items' inputs behind
 // the barrier. The items' keys, states and gate rows are on their way before it now, and a phase's description one phase ahead.
 #include <cfloat>

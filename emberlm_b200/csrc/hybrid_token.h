@@ -1,5 +1,5 @@
-// One-token pass of the layer-list family: a list of phases that one persistent cooperative kernel
-// walks, separated by grid barriers (hybrid_token.cu). The list is built once per decoder.
+// One-token pass of the layer-list family: a list of phases that a persistent cooperative kernel walks, separated by grid
+// barriers: hybrid_token.cu for sandwich layers, hybrid_list.cu for the parallel arrangement. The list is built once per decoder.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -77,7 +77,7 @@ struct TokenBranch {
   int kind, items;
   int H, G, dim, vdim, group;   // group: H / G
   int col_q, col_k, col_v, col_g;
-  float* out;            // [H * vdim]: attention gated, recurrences raw
+  float* out;            // [H * vdim]: recurrences raw, latent attention gated; the attention of sandwich layers leaves `part`
   int stage_at;          // offset of this branch in the staged vector
   // attention
   const float *b_q, *b_k;
@@ -104,7 +104,7 @@ struct TokenBranch {
   const void* w_w2;
   const float *w0, *bonus;
   // latent attention
-  int rot_dim, kv_rank, rot_col, ld_cache, ld_ukv, row_uv, splits, blocks, buffers;   // splits: most ranges (attention: per key/value head); buffers: cache tiles in flight (1 or 2)
+  int rot_dim, kv_rank, rot_col, ld_cache, ld_ukv, row_uv, splits, blocks, buffers;   // splits: most ranges (attention: per key/value head in one turn of the CTAs); buffers: cache tiles in flight (1 or 2)
   const void* w_ukv;
   const float *kv_norm, *q_up;   // queries [H][dim + rot_dim]
   unsigned item_inv, quad_inv;   // division_factor of a head's items (scan: of the splits), of rot_col / 4

@@ -9,7 +9,8 @@ namespace hybrid {
 
 __device__ __forceinline__ float ldg_f(const float* p) { return __ldcg(p); }
 
-// Eight (bfloat16) or four (fp32) weights against the staged vector.
+// Eight (bfloat16) or four (fp32) weights, from memory, against the vector in shared memory (RingChunk of token_ring.cuh: from
+// shared memory against values that a lane holds).
 template <typename T>
 struct Chunk;
 template <>
