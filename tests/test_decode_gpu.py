@@ -280,10 +280,11 @@ def test_gates_at_the_edge_of_the_range(gate):
 
 
 @pytest.mark.parametrize("hid, inter, heads, kv_heads, dim, contexts", [(128, 26048, 48, 48, 64, (10, 190, 390)), (128, 20480, 96, 24, 128, (190, 300)),
-                                                                       (1024, 31616, 16, 2, 128, (9, 600))])
+                                                                       (1024, 31616, 16, 2, 128, (9, 600)), (128, 33024, 4, 2, 64, (9, 190)),
+                                                                       (128, 45056, 4, 2, 64, (9, 190))])
 def test_tiles_over_the_place_of_the_vector(hid, inter, heads, kv_heads, dim, contexts):
-    """Rows so long that the attention's tiles lie over the second place of the vector, or that there is one place only, with
-    ranges of one and several tiles; tolerance as above (weights are drawn so that a layer keeps the size of what passes through it)."""
+    """Rows so long that the attention's tiles lie over the second place of the vector, that there is one place only, or that the ring
+    takes pieces of 128 and 64 chunks, with ranges of one and several tiles; tolerance as above (weights are drawn so that a layer keeps the size of what passes through it)."""
     from emberlm_b200 import engine as E
     kw = dict(CASES[0], hidden_size=hid, intermediate_size=inter, num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=dim)
     ocfg, ecfg = om.LlamaConfig(**kw), E.make_config(**kw)
