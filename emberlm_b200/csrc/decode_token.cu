@@ -166,21 +166,26 @@ __device__ __forceinline__ constexpr int tile_keys(int D, int TILE) { return TIL
 // hand-over, and the scores and sums of 16 keys take a CTA about 1000 cycles: SmolLM2-135M with 37 to 85 keys on one CTA per
 // kv head took 13 200 cycles a layer.
 constexpr int kRangeKeys = 16;
-__device__ __forceinline__ int attn_splits(int L, int Hk) {   // called once a token
-  int most = gridDim.x / Hk;
+__device__ __forceinline__ int attn_splits(int L, int parts) {   // called once a token; parts: of all query heads
+  int most = gridDim.x / parts;
   if (most > kTokenMaxSplits) most = kTokenMaxSplits;
   if (L <= kRangeKeys || most < 2) return 1;
   return min(most, (L + kRangeKeys - 1) / kRangeKeys);
 }
 
-// An item: the query heads of kv head hk against keys [j0, j1), range sp. Made once a token: a phase has no time for the
-// divisions (about 200 cycles each).
+// An item: query heads [head, head + heads) of kv head hk against keys [j0, j1), range sp; the first ones of a kv head write its new
+// row. Made once a token: a phase has no time for the divisions (about 200 cycles each).
 struct Item {
-  int hk, sp, j0, j1;
-  __device__ __forceinline__ Item(int item, int splits, int L) {
-    const int per = (L + splits - 1) / splits;
-    hk = item / splits;
-    sp = item - hk * splits;
+  int hk, head, heads, sp, j0, j1;
+  bool writes;
+  __device__ __forceinline__ Item(const TokenKernelArgs& a, int item, int splits, int L) {
+    const int per = (L + splits - 1) / splits, of = item / splits;
+    hk = of / a.head_groups;
+    const int part = of - hk * a.head_groups, first = a.group * part / a.head_groups;
+    head = hk * a.group + first;
+    heads = a.group * (part + 1) / a.head_groups - first;
+    writes = part == 0;
+    sp = item - of * splits;
     j0 = min(L, sp * per);
     j1 = min(L, j0 + per);
   }
@@ -256,7 +261,7 @@ template <int DC, int TILE>
 __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, const Item it, int splits, int pos, unsigned e, int64_t wqn, int64_t wkn,
                                             float* sm, float* tiles) {
   constexpr int D = 32 * DC, kKeys = tile_keys(D, TILE);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = a.group;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, G = it.heads;
   Patience p(a);
   const bool has_new = pos >= it.j0 && pos < it.j1;
   float* qs = sm;                  // [G][D] rotated, scaled
@@ -266,7 +271,7 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
   // new rows: a warp per head; queries 0 .. G-1, then key and value where the range holds the new position
 #pragma unroll 1
   for (int r = wid; r < G + (has_new ? 2 : 0); r += kWarps) {
-    const int head = r < G ? it.hk * G + r : (r == G ? a.H + it.hk : a.H + a.Hk + it.hk);
+    const int head = r < G ? it.head + r : (r == G ? a.H + it.hk : a.H + a.Hk + it.hk);
     const Word* src = a.qkv + static_cast<int64_t>(head) * D + lane;
     // angles and norm weights are requested before the wait
     float2 cs[DC / 2];
@@ -310,7 +315,7 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
     float* dst = (r < G ? qs + r * D : kn + (r - G) * D) + lane;
 #pragma unroll
     for (int c = 0; c < DC; ++c) dst[32 * c] = x[c];
-    if (r >= G) {
+    if (r >= G && it.writes) {
       float* cache = (r == G ? a.kcache : a.vcache) + ((static_cast<int64_t>(l) * a.Hk + it.hk) * a.max_seq + pos) * D + lane;
 #pragma unroll
       for (int c = 0; c < DC; ++c) cache[32 * c] = x[c];
@@ -397,7 +402,7 @@ __device__ __noinline__ bool attention_item(const TokenKernelArgs& a, int l, con
   if (share == 0) {
 #pragma unroll 1
     for (int blk = mine_first; blk < blocks; blk += kWarps) {
-      const int head = it.hk * G + blk / DC, col = blk % DC * 32 + lane;
+      const int head = it.head + blk / DC, col = blk % DC * 32 + lane;
       if (turns > 1 && it.j0 < it.j1) {
         const float* held = scr + blk * 34;
         m = held[0];
@@ -483,8 +488,8 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
       const float* row = known ? a.P + a.embed + tok * hid : nullptr;
       if (!known && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.status[2], 1);
       for (int i = threadIdx.x; i < s_rows[1].count; i += kThreads) res[i] = known ? row[s_rows[1].first + i] : 0.0f;
-      const int splits = attn_splits(pos + 1, a.Hk), items = a.Hk * splits;
-      const Item mine(blockIdx.x, splits, pos + 1);
+      const int parts = a.Hk * a.head_groups, splits = attn_splits(pos + 1, parts), items = parts * splits;
+      const Item mine(a, blockIdx.x, splits, pos + 1);
       Word best = 0ull;
       // Exchanges of layer l: e + 1 qkv, e + 2 ranges, e + 3 attention, e + 4 hm, e + 5 act, e + 6 x. One body for all
       // products keeps the code that a token runs through small.
@@ -502,7 +507,7 @@ __global__ void __launch_bounds__(kThreads + 32, 1) token_kernel(const __grid_co
             ring_sync();   // the scratch lies over both places of the vector
             Item it = mine;
             if (item >= static_cast<int>(gridDim.x)) {
-              it = Item(item, splits, pos + 1);
+              it = Item(a, item, splits, pos + 1);
               request_tile<D, TILE>(a, tile, l, it, pos, 0);
               request_tile<D, TILE>(a, tile, l, it, pos, 1);
             }
@@ -643,9 +648,12 @@ Kernel kernel_of(int D, int tile) {
 size_t lay_out(TokenKernelArgs& a, int grid, int tile, int places, bool over, int piece) {
   constexpr int64_t kRoom = 227 * 1024 - 4096;   // the kernel's own arrays take 3.1 KB
   auto up = [](int64_t n) { return (n + 31) / 32 * 32; };
-  const int64_t first = up(a.hid), second = up(std::max(a.H * a.D, a.I)), G = a.H / a.Hk;
+  // With one or two key/value heads the ranges leave most CTAs without an item: their query heads are dealt to several. Four layers
+  // behind 3000 positions, us a token: 32 heads of 128 on one key/value head (width 4096) 893 -> 674, 96 on one (2048) 1207 -> 418.
+  a.group = a.H / a.Hk;
+  a.head_groups = std::min(a.group, std::max(1, grid / (a.Hk * kTokenMaxSplits)));
+  const int64_t first = up(a.hid), second = up(std::max(a.H * a.D, a.I)), G = ceil_div(a.group, a.head_groups);
   const int64_t scratch = up(G * (a.D + tile / (8 * a.D)) + attention_scratch(static_cast<int>(G) * a.D / 32) + 2 * a.D);
-  a.group = static_cast<int>(G);
   a.tile_bytes = tile;
   a.residual_floats = static_cast<int>(up(ceil_div(a.hid, grid)));
   a.second_at = places == 2 ? static_cast<int>(first) : 0;

@@ -22,7 +22,7 @@ struct TokenKernelArgs {
   const float* P;
   TokenLayer lw[kTokenMaxLayers];
   int64_t embed, norm;
-  int L, hid, I, D, H, Hk, group, V, QKVN, max_seq;   // group: H / Hk
+  int L, hid, I, D, H, Hk, group, head_groups, V, QKVN, max_seq;   // group: H / Hk, attended to in head_groups parts
   int qk_norm;
   float eps, scale;
   const float2* table;      // [max_seq][D/2] (cos, sin)

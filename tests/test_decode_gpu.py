@@ -300,7 +300,7 @@ def test_tiles_over_the_place_of_the_vector(hid, inter, heads, kv_heads, dim, co
             assert np.abs(dec.step(int(prompt[i])).cpu().numpy() - ref[i]).max() <= 5e-3 * max(np.abs(ref[i]).max(), 1.0), (context, i)
 
 
-@pytest.mark.parametrize("heads, kv_heads, dim", [(32, 1, 128), (5, 1, 64), (9, 3, 64), (2, 2, 128), (17, 1, 64)])
+@pytest.mark.parametrize("heads, kv_heads, dim", [(32, 1, 128), (5, 1, 64), (9, 3, 64), (2, 2, 128), (17, 1, 64), (96, 1, 128), (10, 2, 64)])
 def test_groups_of_query_heads(heads, kv_heads, dim):
     """Groups of one, two, three and more query heads, which share the walk over the keys, with as many blocks of 32 columns as a
     range's warps, fewer and more; tolerance as above."""
