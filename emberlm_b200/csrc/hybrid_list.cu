@@ -467,7 +467,7 @@ __device__ __forceinline__ void latent_keys_item(const TokenBranch& br, int item
   }
 }
 
-// Position ranges in use for L cached positions (less than 2^25), and their length (whole tiles).
+// Position ranges in use for L cached positions, and their length (whole tiles).
 __device__ __forceinline__ int latent_ranges(int L, int splits, int& per) {
   const int tiles = (L + kLatentKeys - 1) / kLatentKeys, each = small_quotient(tiles + splits - 1, splits);
   per = each * kLatentKeys;

@@ -84,10 +84,11 @@ __device__ __forceinline__ int quotient(int n, int d, unsigned inv) {
   return static_cast<int>(q + (static_cast<unsigned>(n) - q * static_cast<unsigned>(d) >= static_cast<unsigned>(d) ? 1u : 0u));
 }
 
-// The same for a divisor that only the device knows, x < 2^20, d < 2^24: (x + 1/2) / d lies half a d-th or more from every whole
-// number, more than the approximate division's two ulp and a rounding.
+// The same for a divisor that only the device knows, d < 2^24, and a quotient below 2^20: the approximate division's two ulp and the
+// roundings of its operands are less than one half there, so the quotient is at most one off.
 __device__ __forceinline__ int small_quotient(int x, int d) {
-  return static_cast<int>(__fdividef(static_cast<float>(x) + 0.5f, static_cast<float>(d)));
+  const int q = static_cast<int>(__fdividef(static_cast<float>(x), static_cast<float>(d))), r = x - q * d;
+  return q + (r >= d ? 1 : 0) - (r < 0 ? 1 : 0);
 }
 __device__ __forceinline__ int quotient(int x, int d) { return x < (1 << 20) ? small_quotient(x, d) : x / d; }
 
